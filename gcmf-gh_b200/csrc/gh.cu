@@ -1411,13 +1411,15 @@ __device__ bool seq_step4(PairCtx& c) {
   return true;
 }
 
-// step 5: split vertex pairs (polyclip.h:661-714)
+// step 5: split vertex pairs (polyclip.h:661-714).  n >= 0: the candidates of P are the n
+// slots listed in P.ls, in order
 template <int EX>
-__device__ bool seq_step5(PairCtx& c) {
+__device__ bool seq_step5(PairCtx& c, int n = -1) {
   Ring& P = c.R[0];
   Ring& Q = c.R[1];
-  const int pm0 = P.used;
-  for (int ip = 0; ip < pm0; ++ip) {
+  const int pm0 = n < 0 ? P.used : n;
+  for (int i = 0; i < pm0; ++i) {
+    const int ip = n < 0 ? i : P.ls(i);
     if (!(P.fl(ip) & 1)) continue;
     int iq = P.nb(ip);
     if (iq < 0 || !(Q.fl(iq) & 1)) continue;
@@ -1459,6 +1461,19 @@ __device__ void seq_step6(PairCtx& c) {
   }
 }
 
+// A walk that never closes repeats itself: the piece that starts at V of a ring is the same
+// each time within one component.  Brent's cycle detection (1980) over the pieces' starts
+// ends such a pair after a few rounds of its cycle instead of the whole step budget; the
+// pair's status is the same (3, no output).
+struct WalkRepeat {
+  int v = -1, side = -1, steps = 0, power = 1;
+  __device__ __forceinline__ bool seen(int V, int s) {
+    if (V == v && s == side) return true;
+    if (++steps == power) { v = V; side = s; steps = 0; power <<= 1; }
+    return false;
+  }
+};
+
 // tracing (polyclip.h:743-783): starts at unvisited CROSSING vertices of P in ring order
 // from slot 0; visited vertices are marked by clearing their intersection flag.
 __device__ bool seq_trace(PairCtx& c) {
@@ -1476,11 +1491,14 @@ __device__ bool seq_trace(PairCtx& c) {
     O.begin();
     int side = 0, V = I;
     P.it(V) = 0;
+    WalkRepeat again;
     do {
       Ring& C = c.R[side];
       int8_t st = toggled(C.ee(V));
+      int left = C.used + 1;                           // once round the ring finds every stop
+      if (again.seen(V, side)) { fail(c, DEV_TRACE); return false; }
       do {
-        if (--budget < 0) { fail(c, DEV_TRACE); return false; }
+        if (--budget < 0 || --left < 0) { fail(c, DEV_TRACE); return false; }
         V = ((st == E_EXIT) ^ c.uni) ? C.nx(V) : C.pv(V);
         C.it(V) = 0;
         O.push(C.x(V), C.y(V));
@@ -1600,50 +1618,23 @@ struct WarpGroup {
     total = __shfl_sync(kFull, x, 31);
     return x;
   }
-};
-
-// A tile of W lanes (a power of two below 32) of one warp: the tiles work on different pairs
-// side by side, each with its own lane mask.
-template <int W>
-struct TileGroup {
-  static constexpr bool kBlock = false;
-  static constexpr bool kSolo = false;
-  unsigned mask;
-  int base;
-  __device__ __forceinline__ TileGroup() {
-    base = (int)(lane_id() & ~(unsigned)(W - 1));
-    mask = ((1u << W) - 1u) << base;
-  }
-  __device__ __forceinline__ int rank() const { return (int)lane_id() - base; }
-  __device__ __forceinline__ int size() const { return W; }
-  __device__ __forceinline__ void sync() const { __syncwarp(mask); }
-  __device__ __forceinline__ bool all(bool v) const { return (__ballot_sync(mask, v) & mask) == mask; }
-  __device__ __forceinline__ bool any(bool v) const { return (__ballot_sync(mask, v) & mask) != 0u; }
-  __device__ __forceinline__ int sum(int v) const {
-#pragma unroll
-    for (int o = W / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o, W);
-    return v;
-  }
-  template <class T>
-  __device__ __forceinline__ T bcast0(T v) const { return __shfl_sync(mask, v, 0, W); }
-  __device__ __forceinline__ int first(bool hit) const {
-    const unsigned m = (__ballot_sync(mask, hit) & mask) >> base;
-    return m ? __ffs(m) - 1 : -1;
-  }
-  __device__ __forceinline__ int incl_scan(int v, int& total) const {
-#pragma unroll
-    for (int o = 1; o < W; o <<= 1) {
-      const int w = __shfl_up_sync(mask, v, o, W);
-      if (rank() >= o) v += w;
+  // f(s, hit, hits before s) for every s in [0, n); returns the number of hits
+  template <class P, class F>
+  __device__ __forceinline__ int list(int n, P pred, F f) const {
+    int carry = 0;
+    for (int b = 0; b < n; b += 32) {
+      const int s = b + rank();
+      const bool hit = s < n && pred(s);
+      const unsigned m = __ballot_sync(kFull, hit);
+      if (s < n) f(s, hit, carry + __popc(m & lanemask_lt()));
+      carry += __popc(m);
     }
-    total = __shfl_sync(mask, v, W - 1, W);
-    return v;
+    return carry;
   }
 };
 
 // One thread per pair: every collective is the identity, nothing synchronises.
 struct SoloGroup {
-  static constexpr bool kBlock = false;
   static constexpr bool kSolo = true;
   __device__ __forceinline__ int rank() const { return 0; }
   __device__ __forceinline__ int size() const { return 1; }
@@ -1657,21 +1648,21 @@ struct SoloGroup {
   __device__ __forceinline__ int incl_scan(int v, int& total) const { total = v; return v; }
 };
 
-template <int W> struct TileOf { using type = TileGroup<W>; };
-template <> struct TileOf<1> { using type = SoloGroup; };
-
 // Block-wide versions over shared scratch (kBlockLabelThreads / 32 warps); each call
 // begins with a barrier so the scratch of the previous call is free.
 constexpr int kBlockLabelThreads = 512;
-// Dynamic shared memory of the block labelling kernel: the trace's run table of pairs with
-// up to 8,192 runs (two blocks per SM at its register budget).
-constexpr int kBlockRunTableBytes = 96 * 1024;
+constexpr int kBlockLabelWarps = kBlockLabelThreads / 32;
+// Dynamic shared memory of the block labelling kernel: the trace's loop table of pairs with
+// up to 8,192 segments of P, 12 bytes each (two blocks per SM).
+constexpr int kBlockLoopTableBytes = 96 * 1024;
+constexpr int kBlockListRounds = 8;   // elements per thread between two barriers of list()
+constexpr int kBlockScratch = kBlockLabelWarps + 1 + (kBlockListRounds * kBlockLabelWarps + 2) / 2;
 struct BlockGroup {
   static constexpr bool kBlock = true;
   static constexpr bool kSolo = false;
-  long long* sm;        // kBlockLabelThreads / 32 + 1 entries
-  int32_t* runs;        // shared memory for the trace's run table (3 words per run)
-  int runsCap;          // runs that fit
+  long long* sm;        // kBlockScratch entries
+  uint32_t* loops;      // shared memory for the trace's loop table
+  int loopsCap;         // segments that fit
   __device__ __forceinline__ int rank() const { return (int)threadIdx.x; }
   __device__ __forceinline__ int size() const { return kBlockLabelThreads; }
   __device__ __forceinline__ void sync() const { __syncthreads(); }
@@ -1716,6 +1707,47 @@ struct BlockGroup {
     for (int w = 0; w < kBlockLabelThreads / 32; ++w) { if (w < me) before += sm[w]; all += sm[w]; }
     total = (int)all;
     return (int)(before + x);
+  }
+  // As WarpGroup's: each thread takes kBlockListRounds elements per step, so that the
+  // barriers and the scan of the warps' counts are paid once per 4,096 elements.
+  template <class P, class F>
+  __device__ __forceinline__ int list(int n, P pred, F f) const {
+    int* cnt = reinterpret_cast<int*>(sm + kBlockLabelWarps + 1);   // [round][warp], then the total
+    const int warp = (int)(threadIdx.x >> 5), lane = (int)lane_id();
+    constexpr int kCounts = kBlockListRounds * kBlockLabelWarps, kPer = kCounts / 32;
+    int carry = 0;
+    for (int b = 0; b < n; b += kBlockListRounds * kBlockLabelThreads) {
+      unsigned m[kBlockListRounds];
+#pragma unroll
+      for (int r = 0; r < kBlockListRounds; ++r) {
+        const int s = b + r * kBlockLabelThreads + (int)threadIdx.x;
+        m[r] = __ballot_sync(kFull, s < n && pred(s));
+      }
+      __syncthreads();
+      if (lane == 0) {
+#pragma unroll
+        for (int r = 0; r < kBlockListRounds; ++r) cnt[r * kBlockLabelWarps + warp] = __popc(m[r]);
+      }
+      __syncthreads();
+      if (warp == 0) {
+        int v[kPer], t = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) { v[j] = cnt[lane * kPer + j]; t += v[j]; }
+        const int incl = warp_incl_scan(t);
+        int run = incl - t;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) { cnt[lane * kPer + j] = run; run += v[j]; }
+        if (lane == 31) cnt[kCounts] = incl;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kBlockListRounds; ++r) {
+        const int s = b + r * kBlockLabelThreads + (int)threadIdx.x;
+        if (s < n) f(s, ((m[r] >> lane) & 1u) != 0, carry + cnt[r * kBlockLabelWarps + warp] + __popc(m[r] & lanemask_lt()));
+      }
+      carry += cnt[kCounts];
+    }
+    return carry;
   }
 };
 
@@ -1971,9 +2003,15 @@ __device__ void grp_step6(const G& g, PairCtx& c) {
   g.sync();
 }
 
-// Run-table tracing for warp-sized pairs: the table is kept per ring slot (tl, tn, to),
-// which saves the slot-to-index translation of the indexed variant below; the walk marks
-// visited vertices in the rings' intersection flags.  Same phases and results.
+// Run-table tracing for one-thread pairs.  With entry/exit flags alternating along both
+// rings (checked here), every run of the sequential walk goes from a flagged vertex to the
+// adjacent flagged vertex in its direction, and the next run starts at that vertex's
+// neighbour.  Phase 1 gives each flagged vertex, by its slot, its run (tl: the length, signed
+// by direction; tn: the next run's start); phase 2 follows the runs in the order of the
+// sequential walk and assigns each its output offset (to), marking visited vertices in the
+// rings' intersection flags; phase 3 copies the runs.  Returns 0 when done, 1 when the
+// flags do not alternate (the caller then runs the general walk), -1 on a capacity or trace
+// error.
 template <class G>
 __device__ int grp_trace_runs_slots(const G& g, PairCtx& c) {
   int nF[2];
@@ -2108,176 +2146,329 @@ __device__ int grp_trace_runs_slots(const G& g, PairCtx& c) {
   return 0;
 }
 
-// Tracing from a run table.  With entry/exit flags alternating along both rings (checked
-// here), every run of the sequential walk goes from a flagged vertex to the adjacent
-// flagged vertex in its direction, and the next run starts at that vertex's neighbour.
-// Phase 1 (parallel) lists the flagged slots of each ring and gives each flagged vertex
-// (by its index in that list) its run: the length, signed by direction, and the index of
-// the next run's start on the other ring.  Phase 2 (one member) follows the runs in the
-// order of the sequential walk -- components from the first unvisited crossing of P, in
-// P's slot order -- and assigns each run its output offset.  Phase 3 (parallel) copies
-// the runs.  Indexing the table by flagged vertex keeps the walk's visited marks in the
-// table itself, so the walk touches no ring array.  Returns 0 when done, 1
-// when the flags do not alternate (the caller then runs the general walk), -1 on a
-// capacity or trace error.
+// Copies one run per lane (L vertices of ring A from slot s0 on, exclusive, in direction
+// dir) to dst: short runs by their lane, long ones by the whole warp one after another.
+// Every lane of the warp calls it; lanes without a run pass L = 0.
+__device__ __forceinline__ void warp_copy_runs(const Ring& A, int s0, int L, int dir, double2* dst) {
+  constexpr int kShortRun = 16;
+  const int m = A.m;
+  if (L <= kShortRun) {
+    int w = s0;
+    for (int j = 0; j < L; ++j) {
+      w += dir;
+      if (w >= m) w -= m;
+      if (w < 0) w += m;
+      dst[j] = A.xy(w);
+    }
+  }
+  unsigned longs = __ballot_sync(kFull, L > kShortRun);
+  while (longs) {
+    const int src = __ffs(longs) - 1;
+    longs &= longs - 1;
+    const int bs = __shfl_sync(kFull, s0, src), bL = __shfl_sync(kFull, L, src), bd = __shfl_sync(kFull, dir, src);
+    double2* d = reinterpret_cast<double2*>(__shfl_sync(kFull, (unsigned long long)dst, src));
+    for (int j = (int)lane_id(); j < bL; j += 32) {
+      int w = bs + bd * (j + 1);                       // |j + 1| <= m: one wrap at most
+      if (w >= m) w -= m;
+      if (w < 0) w += m;
+      d[j] = A.xy(w);
+    }
+  }
+}
+
+// The loop table of one pair.  A P segment t has two ends, 0 its first and 1 its last vertex.
+// link(t, e): the P segment and the end of it that a walk leaving t at end e gets to over the
+// Q segment there, as 2 * segment + end; w(t, e): the vertices of t and of that Q segment.
+// Bit 31 of w(t, 1) is set when neither end is a crossing.
+constexpr unsigned kNoCrossing = 0x80000000u;
+struct LoopsGlobal {
+  const int32_t *l0, *l1, *w0, *w1;
+  __device__ __forceinline__ int link(int t, int e) const { return (e ? l1 : l0)[t]; }
+  __device__ __forceinline__ unsigned raw(int t) const { return (unsigned)w1[t]; }
+  __device__ __forceinline__ int w(int t, int e) const { return e ? (int)(raw(t) & ~kNoCrossing) : w0[t]; }
+};
+struct LoopsShared {                                     // 12 bytes per segment, fewer than 2^15 segments
+  uint32_t* p;
+  int n;
+  __device__ __forceinline__ int link(int t, int e) const { return (int)((p[t] >> (16 * e)) & 0xffffu); }
+  __device__ __forceinline__ unsigned raw(int t) const { return p[2 * n + t]; }
+  __device__ __forceinline__ int w(int t, int e) const { return e ? (int)(raw(t) & ~kNoCrossing) : (int)p[n + t]; }
+};
+
+// The size of t's loop when t is its smallest segment with a crossing, else 0 (-1: the walk
+// did not close within guard steps).  The walk goes both ways at once and stops at the
+// first smaller segment: over a loop of L segments the searches take O(L log L) steps in
+// all, whatever its order, and the smallest segment's own takes L / 2.
+template <class T>
+__device__ __forceinline__ int loop_size(const T& tab, int t, int guard) {
+  if (tab.raw(t) & kNoCrossing) return 0;
+  int f = tab.link(t, 1), b = tab.link(t, 0);            // where the two walks arrive
+  int sz = tab.w(t, 1);
+  while ((f >> 1) != t) {
+    const int ft = f >> 1, bt = b >> 1, fo = 1 - (f & 1), bi = b & 1;
+    if ((ft < t && !(tab.raw(ft) & kNoCrossing)) || (bt < t && !(tab.raw(bt) & kNoCrossing))) return 0;
+    sz += tab.w(ft, fo);
+    if (ft == bt) break;
+    sz += tab.w(bt, bi);
+    f = tab.link(ft, fo);
+    if ((f >> 1) == bt) break;
+    b = tab.link(bt, 1 - bi);
+    if ((guard -= 2) < 0) return -1;
+  }
+  return sz;
+}
+
+// Output offsets of the segments of t's loop (size vertices from base on), walked from t
+// entered at end `in`; from both ends of the range.  A segment entered at its last vertex
+// has ~offset.
+template <class T>
+__device__ __forceinline__ void loop_offsets(const T& tab, int t, int in, int base, int size, int32_t* off) {
+  off[t] = in ? ~base : base;
+  int of = base + tab.w(t, 1 - in), ob = base + size;
+  int f = tab.link(t, 1 - in), b = tab.link(t, in);
+  while (of < ob) {
+    const int ft = f >> 1, fi = f & 1;
+    off[ft] = fi ? ~of : of;
+    of += tab.w(ft, 1 - fi);
+    if (of >= ob) break;
+    const int bt = b >> 1, be = b & 1;                   // the walk leaves bt at end be
+    ob -= tab.w(bt, be);
+    off[bt] = be ? ob : ~ob;
+    f = tab.link(ft, 1 - fi);
+    b = tab.link(bt, 1 - be);
+  }
+}
+
+// Tracing by loops.  The walk of polyclip.h:743-783 starts at crossings of P, leaves a vertex
+// that starts a piece (a forward vertex: entry, or exit for a union) in ring order and stops
+// at the next flagged vertex of the other kind, leaves one of the other kind against ring
+// order, and goes on at a stop's neighbour.  Wherever a ring's flags change from forward to
+// backward there is a segment: forward walks stop at its last vertex, backward walks at
+// its first, and no other flagged vertex is ever stopped at.  The neighbours link the segments of
+// P and Q into loops.  Where every stop has a flagged neighbour, the links are the same in
+// both directions, and every crossing of P ends a segment (all checked here), the loops
+// are disjoint and the walk emits them in the order of their smallest crossing of P, each
+// from that crossing on.  So instead of walking them one after another (a chain of dependent
+// loads over all pieces of the pair, with the rest of the group waiting), every segment finds
+// out whether it is its loop's smallest, the loops' sizes are scanned, and all loops are
+// walked at once for the offsets of their segments.
+// Returns 0 when done, 1 when the conditions do not hold (the caller then runs the general
+// walk), -1 on a capacity error.
 template <class G>
-__device__ int grp_trace_runs(const G& g, PairCtx& c) {
-  int nF[2];
-  bool mismatch = false;     // a flagged vertex that is not a crossing, or the reverse
+__device__ int grp_trace_loops(const G& g, PairCtx& c) {
+  Ring& P = c.R[0];
+  Ring& Q = c.R[1];
+  const bool uni = c.uni;
+  const int mP = P.m, mQ = Q.m;
+  auto fwd_at = [uni](const Ring& A, int s) { return (A.ee(s) == E_ENTRY) != uni; };
+  auto cross_at = [](const Ring& A, int s) { return A.it(s) && A.lb(s) == L_CROSSING; };
+  bool bad = false, crossing = false, beside = false;
+  int nF[2], nS[2];
+  bool wrapFirst = false;
   for (int sd = 0; sd < 2; ++sd) {
     Ring& A = c.R[sd];
-    int carry = 0;
-    for (int b = 0; b < A.m; b += g.size()) {
-      const int s = b + g.rank();
-      const int f = (s < A.m && (A.ee(s) == E_ENTRY || A.ee(s) == E_EXIT)) ? 1 : 0;
-      if (s < A.m && (f != 0) != (A.it(s) && A.lb(s) == L_CROSSING)) mismatch = true;
-      int tot;
-      const int incl = g.incl_scan(f, tot);
-      if (f) { A.ls(carry + incl - 1) = s; A.to(s) = carry + incl - 1; }   // slot -> index
-      carry += tot;
-    }
-    nF[sd] = carry;
-  }
-  if (g.any(mismatch)) return 1;
-  if (nF[0] == 0 && nF[1] == 0) return 0;
-  // run table by list index, in the rings' scratch arrays: length RL, next start RN (sign
-  // bit = visited), output offset RO.  The slot -> index map in `to` is read until phase 1
-  // ends; the offsets take its place then.  (Pointers are selected per side in registers.)
-  int32_t* RL0 = &c.R[0].tl(0); int32_t* RL1 = &c.R[1].tl(0);
-  int32_t* RN0 = &c.R[0].tn(0); int32_t* RN1 = &c.R[1].tn(0);
-  int32_t* RO0 = &c.R[0].to(0); int32_t* RO1 = &c.R[1].to(0);
-#define RL_(sd) ((sd) ? RL1 : RL0)
-#define RN_(sd) ((sd) ? RN1 : RN0)
-#define RO_(sd) ((sd) ? RO1 : RO0)
-  bool bad = nF[0] < 2 || nF[1] < 2;
-  bool longRun = false;
-  for (int sd = 0; sd < 2 && !bad; ++sd) {
-    Ring& A = c.R[sd];
-    const Ring& B = c.R[1 - sd];
-    const int n = nF[sd], m = A.m;
-    for (int i = g.rank(); i < n; i += g.size()) {
-      const int s = A.ls(i);
-      const int8_t e = A.ee(s);
-      if (A.ee(A.ls((i + 1 < n) ? i + 1 : 0)) == e) { bad = true; continue; }   // alternation
-      const int nb = A.nb(s);
-      if (nb < 0 || nb >= B.m || B.ee(nb) != toggled(e)) { bad = true; continue; }
-      const int8_t st = toggled(e);
-      const int dir = ((st == E_EXIT) ^ c.uni) ? 1 : -1;
-      const int W = A.ls((i + dir + n) % n);
-      int L = dir > 0 ? W - s : s - W;
-      if (L <= 0) L += m;
-      const int nbW = A.nb(W);
-      if (nbW < 0 || nbW >= B.m) { bad = true; continue; }
-      RL_(sd)[i] = dir * L;
-      RN_(sd)[i] = B.to(nbW);          // a flagged twin (checked): its index in B's list
-      if (L > 32) longRun = true;
-    }
+    // ls: the flagged slots in ring order
+    nF[sd] = g.list(
+        A.m,
+        [&](int s) {
+          const bool flagged = A.ee(s) != E_NEITHER;
+          if (sd == 0 && cross_at(A, s)) { crossing = true; if (!flagged) bad = true; }
+          return flagged;
+        },
+        [&](int s, bool hit, int before) { if (hit) A.ls(before) = s; });
+    g.sync();
+    const int n = nF[sd];
+    // Segment numbers by the place of the first vertex, except that P's segment around
+    // slot 0 is the first one when its smaller end is a crossing (the walk starts there).
+    // tn: segment -> place of its first vertex in ls; to: flagged slot -> its segment
+    if (sd == 0) wrapFirst = n > 1 && !fwd_at(A, A.ls(0)) && fwd_at(A, A.ls(n - 1)) && cross_at(A, A.ls(0));
+    nS[sd] = g.list(n, [&](int f) { return fwd_at(A, A.ls(f)) && !fwd_at(A, A.ls(f + 1 < n ? f + 1 : 0)); },
+                    [&](int f, bool hit, int before) {
+                      const int s = A.ls(f);
+                      const bool fw = fwd_at(A, s);
+                      if (hit) A.tn(before) = f;
+                      else if (sd == 0 && cross_at(A, s) && (fw || !fwd_at(A, A.ls(f > 0 ? f - 1 : n - 1)))) beside = true;
+                      A.to(s) = (hit || fw) ? before : before - 1;   // -1 and the count stand for the wrapped one
+                    });
+    g.sync();
   }
   if (g.any(bad)) return 1;
-  if constexpr (G::kBlock) {
-    // The walk below is one long chain of dependent loads: with the table in shared
-    // memory each step costs tens of cycles instead of an L2 round trip.
-    if (nF[0] + nF[1] <= g.runsCap) {
-      int32_t* sh = g.runs;
-      int32_t* dst[6] = {sh, sh + nF[0], sh + 2 * nF[0], sh + 3 * nF[0], sh + 3 * nF[0] + nF[1],
-                         sh + 3 * nF[0] + 2 * nF[1]};
-      for (int sd = 0; sd < 2; ++sd)
-        for (int i = g.rank(); i < nF[sd]; i += g.size()) {
-          dst[3 * sd][i] = RL_(sd)[i];
-          dst[3 * sd + 1][i] = RN_(sd)[i];
-        }
-      RL0 = dst[0]; RN0 = dst[1]; RO0 = dst[2];
-      RL1 = dst[3]; RN1 = dst[4]; RO1 = dst[5];
+  if (!g.any(crossing)) return 0;                        // nothing to start from
+  const int n = nS[0], nQ = nS[1], nFP = nF[0], nFQ = nF[1];
+  if (n == 0 || n > nQ) return 1;
+  // scratch: at most half of a ring's vertices start segments, so a column holds two arrays
+  int32_t* bP = &P.tn(0);
+  int32_t* lead = &P.tn(mP >> 1);
+  int32_t* bQ = &Q.tn(0);
+  int32_t* eV = &Q.tn(mQ >> 1);                          // where a segment is entered, if not at its end
+  int32_t* off = &P.to(0);                               // (when the slot map is done with)
+  const LoopsGlobal glob{&P.tl(0), &P.tl(mP >> 1), &Q.tl(0), &Q.tl(mQ >> 1)};
+  bool shared = false;
+  LoopsShared shrd{nullptr, n};
+  if constexpr (G::kBlock) { shared = n <= g.loopsCap; shrd.p = g.loops; }
+  auto link = [&](int t, int e) { return shared ? shrd.link(t, e) : glob.link(t, e); };
+  auto place = [&](int t) { return bP[wrapFirst ? (t > 0 ? t - 1 : n - 1) : t]; };
+  auto end_p = [&](int t, int e) { const int f = place(t) + e; return P.ls(f < nFP ? f : 0); };
+  auto end_q = [&](int j, int e) { const int f = bQ[j] + e; return Q.ls(f < nFQ ? f : 0); };
+  auto seg_p = [&](int p) {
+    int t = P.to(p);
+    t = t < 0 ? n - 1 : (t >= n ? 0 : t);
+    return wrapFirst ? (t + 1 < n ? t + 1 : 0) : t;
+  };
+  auto seg_q = [&](int q) { const int j = Q.to(q); return j < 0 ? nQ - 1 : (j >= nQ ? 0 : j); };
+  auto dist = [](int from, int to, int m) { const int d = to - from; return d > 0 ? d : d + m; };
+  bool odd = false;                                      // some segment is entered beside its end
+  for (int t = g.rank(); t < n; t += g.size()) {
+    const int v0 = end_p(t, 0), v1 = end_p(t, 1);
+    const int lp = dist(v0, v1, mP);
+    int lk[2] = {0, 0};
+    unsigned w[2] = {0, 0};
+    for (int e = 0; e < 2; ++e) {
+      const int q = P.nb(e ? v1 : v0);
+      if (q < 0 || q >= mQ || Q.ee(q) == E_NEITHER) { bad = true; break; }
+      const int qe = fwd_at(Q, q) ? 0 : 1, j = seg_q(q); // entered at end qe, left at the other
+      const int W = end_q(j, 1 - qe), p2 = Q.nb(W);
+      if (p2 < 0 || p2 >= mP || P.ee(p2) == E_NEITHER) { bad = true; break; }
+      const int t2 = seg_p(p2), pe = fwd_at(P, p2) ? 0 : 1;
+      if (q != end_q(j, qe) || p2 != end_p(t2, pe)) odd = true;
+      lk[e] = 2 * t2 + pe;
+      w[e] = (unsigned)(lp + (qe ? dist(W, q, mQ) : dist(q, W, mQ)));
     }
-  }
-  for (int sd = 0; sd < 2; ++sd)
-    for (int i = g.rank(); i < nF[sd]; i += g.size()) RO_(sd)[i] = -1;
-  const bool anyLong = g.any(longRun);
-  // ---- phase 2: the walk over the run table, one member
-  constexpr int32_t kSeen = (int32_t)0x80000000u;
-  OutRegion& O = c.O;
-  int status = 0;
-  int64_t nv = O.nv;
-  int nc = O.nc;
-  if (g.rank() == 0) {
-    const int64_t nv0 = O.nv;
-    const int nFP = nF[0], nFQ = nF[1];
-    long long budget = (long long)nFP + nFQ + 4;
-    for (int I = 0; I < nFP && status == 0; ++I) {
-      if (RN_(0)[I] < 0) continue;                       // visited
-      if (nc >= O.ccap) { status = -1; fail(c, DEV_CAPACITY); break; }
-      RN_(0)[I] |= kSeen;
-      int side = 0, V = I;
-      int64_t csz = 0;
-      for (;;) {
-        const int t = RL_(side)[V], L = t < 0 ? -t : t, n = side ? nFQ : nFP;
-        int W = V + (t < 0 ? -1 : 1);
-        if (W >= n) W -= n;
-        if (W < 0) W += n;
-        RO_(side)[V] = (int32_t)(nv - nv0);
-        nv += L;
-        csz += L;
-        const int V2 = RN_(side)[V] & 0x7fffffff;
-        RN_(side)[W] |= kSeen;
-        if (side == 0 && W == I) break;
-        side ^= 1;
-        if (side == 0 && V2 == I) break;
-        RN_(side)[V2] |= kSeen;
-        V = V2;
-        if (--budget < 0) { status = -1; fail(c, DEV_TRACE); break; }
-      }
-      if (status == 0) {
-        if (nv > O.vcap) { status = -1; fail(c, DEV_CAPACITY); break; }
-        O.csz[nc++] = (int32_t)csz;
-      }
-    }
-  }
-  status = g.bcast0(status);
-  if (status != 0) return -1;
-  const int64_t nv0 = O.nv;
-  O.nv = g.bcast0((long long)nv);
-  O.nc = g.bcast0(nc);
-  // ---- phase 3: copy every run to its place; short runs one member each, long runs by
-  // the whole group (no barrier between runs: runs write disjoint ranges)
-  constexpr int kShortRun = 32;      // the run-length threshold of phase 1's longRun
-  for (int sd = 0; sd < 2; ++sd) {
-    const Ring& A = c.R[sd];
-    const int m = A.m;
-    for (int i = g.rank(); i < nF[sd]; i += g.size()) {
-      const int off = RO_(sd)[i];
-      if (off < 0) continue;
-      const int t = RL_(sd)[i], L = t < 0 ? -t : t, dir = t < 0 ? -1 : 1;
-      if (anyLong && L > kShortRun) continue;
-      double* dst = O.xy + 2 * (nv0 + off);
-      int w = A.ls(i);
-      for (int j = 0; j < L; ++j) {
-        w += dir;
-        if (w >= m) w -= m;
-        if (w < 0) w += m;
-        dst[2 * j] = A.x(w);
-        dst[2 * j + 1] = A.y(w);
-      }
-    }
-    for (int i = 0; anyLong && i < nF[sd]; ++i) {
-      const int off = RO_(sd)[i];
-      const int t = RL_(sd)[i], L = t < 0 ? -t : t;
-      if (off < 0 || L <= kShortRun) continue;
-      const int dir = t < 0 ? -1 : 1, s0 = A.ls(i);
-      double* dst = O.xy + 2 * (nv0 + off);
-      for (int j = g.rank(); j < L; j += g.size()) {
-        int w = s0 + dir * (j + 1);
-        w %= m;
-        if (w < 0) w += m;
-        dst[2 * j] = A.x(w);
-        dst[2 * j + 1] = A.y(w);
-      }
+    if (!cross_at(P, v0) && !cross_at(P, v1)) w[1] |= kNoCrossing;
+    if (shared) {
+      shrd.p[t] = (uint32_t)lk[0] | ((uint32_t)lk[1] << 16);
+      shrd.p[n + t] = w[0];
+      shrd.p[2 * n + t] = w[1];
+    } else {
+      const_cast<int32_t*>(glob.l0)[t] = lk[0];
+      const_cast<int32_t*>(glob.l1)[t] = lk[1];
+      const_cast<int32_t*>(glob.w0)[t] = (int32_t)w[0];
+      const_cast<int32_t*>(glob.w1)[t] = (int32_t)w[1];
     }
   }
   g.sync();
+  if (g.any(bad)) return 1;
+  odd = g.any(odd);
+  for (int t = g.rank(); t < n; t += g.size())           // the same links both ways
+    for (int e = 0; e < 2; ++e) {
+      const int l = link(t, e);
+      if (link(l >> 1, l & 1) != 2 * t + e) bad = true;
+    }
+  g.sync();
+  if (g.any(bad)) return 1;
+  if (g.any(beside)) {
+    // A crossing of P beside a segment's end: no loop passes it (where segments are
+    // entered at their ends only), so the walk starts there, runs into a loop and never
+    // comes back to it.
+    if (odd) return 1;
+    if (g.rank() == 0) fail(c, DEV_TRACE);
+    return -1;
+  }
+  // the end at which the walk enters its first segment: the smaller one that is a crossing
+  auto start_end = [&](int t) { return ((t == 0 && wrapFirst) || !cross_at(P, end_p(t, 0))) ? 1 : 0; };
+  // the pieces of one step: along P from `entry` to t's other end, along Q to where it is left
+  struct Step { int sp, lp, sq, lq, dq, left; };
+  auto step_of = [&](int t, int in, int entry, int left) {
+    Step r;
+    const int v = end_p(t, 1 - in);
+    r.sp = entry;
+    r.lp = in ? dist(v, entry, mP) : dist(entry, v, mP);
+    r.sq = P.nb(v);
+    const bool fq = fwd_at(Q, r.sq);
+    r.left = left < 0 ? end_q(seg_q(r.sq), fq ? 1 : 0) : left;
+    r.dq = fq ? 1 : -1;
+    r.lq = fq ? dist(r.sq, r.left, mQ) : dist(r.left, r.sq, mQ);
+    return r;
+  };
+  // ---- the loops' smallest segments and sizes
+  for (int t = g.rank(); t < n; t += g.size()) {
+    int sz = shared ? loop_size(shrd, t, n + 2) : loop_size(glob, t, n + 2);
+    if (sz < 0) { bad = true; sz = 0; }
+    if (odd && sz > 0) {                                 // the pieces depend on the direction: walk them
+      const int in0 = start_end(t), I = end_p(t, in0);
+      int u = t, in = in0, v = I;
+      sz = 0;
+      do {
+        const Step r = step_of(u, in, v, -1);
+        sz += r.lp + r.lq;
+        v = Q.nb(r.left);
+        const int l = link(u, 1 - in);
+        u = l >> 1;
+        in = l & 1;
+      } while (u != t);
+      if (v != I) bad = true;                            // closes elsewhere than at its start
+    }
+    off[t] = sz;
+  }
+  g.sync();
+  if (g.any(bad)) return 1;
+  OutRegion& O = c.O;
+  int32_t* csz = O.csz + O.nc;
+  const int room = O.ccap - O.nc;
+  const int nl = g.list(n, [&](int t) { return off[t] > 0; },
+                        [&](int t, bool hit, int before) {
+                          if (hit) {
+                            lead[before] = t;
+                            if (before < room) csz[before] = off[t];
+                          }
+                          off[t] = INT_MIN;              // stays so in loops without a crossing
+                        });
+  if (nl > room) { if (g.rank() == 0) fail(c, DEV_CAPACITY); return -1; }
+  g.sync();
+  long long total = 0;
+  for (int b = 0; b < nl; b += g.size()) {
+    const int k = b + g.rank();
+    const int v = k < nl ? csz[k] : 0;
+    int tot;
+    const int incl = g.incl_scan(v, tot);
+    if (k < nl) off[lead[k]] = (int32_t)total + incl - v;
+    total += tot;
+  }
+  if (O.nv + total > O.vcap) { if (g.rank() == 0) fail(c, DEV_CAPACITY); return -1; }
+  g.sync();
+  // ---- offsets of the segments
+  for (int k = g.rank(); k < nl; k += g.size()) {
+    const int t0 = lead[k], base = off[t0], in0 = start_end(t0);
+    if (odd) {
+      int u = t0, in = in0, v = end_p(t0, in0), o = base;
+      do {
+        const Step r = step_of(u, in, v, -1);
+        off[u] = in ? ~o : o;
+        eV[u] = v;
+        o += r.lp + r.lq;
+        v = Q.nb(r.left);
+        const int l = link(u, 1 - in);
+        u = l >> 1;
+        in = l & 1;
+      } while (u != t0);
+    } else if (shared) {
+      loop_offsets(shrd, t0, in0, base, csz[k], off);
+    } else {
+      loop_offsets(glob, t0, in0, base, csz[k], off);
+    }
+  }
+  g.sync();
+  // ---- copy the pieces
+  double2* out = reinterpret_cast<double2*>(O.xy) + O.nv;
+  for (int b = 0; b < n; b += g.size()) {
+    const int t = b + g.rank();
+    Step r{0, 0, 0, 0, 1, 0};
+    int op = t < n ? off[t] : INT_MIN, dp = 1;
+    if (op != INT_MIN) {
+      const int in = op < 0 ? 1 : 0, l = link(t, 1 - in);
+      if (in) { op = ~op; dp = -1; }
+      // the next segment's entry is the neighbour of the vertex at which Q is left
+      r = step_of(t, in, odd ? eV[t] : end_p(t, in), P.nb(odd ? eV[l >> 1] : end_p(l >> 1, l & 1)));
+    } else {
+      op = 0;
+    }
+    warp_copy_runs(P, r.sp, r.lp, dp, out + op);
+    warp_copy_runs(Q, r.sq, r.lq, r.dq, out + op + r.lp);
+  }
+  O.nv += total;
+  O.nc += nl;
+  g.sync();
   return 0;
-#undef RL_
-#undef RN_
-#undef RO_
 }
 
 // Tracing when neither ring has added vertices (rings in slot order): each run from V to
@@ -2297,9 +2488,11 @@ __device__ bool grp_trace(const G& g, PairCtx& c) {
     int side = 0, V = I;
     if (g.rank() == 0) P.it(V) = 0;
     g.sync();
+    WalkRepeat again;
     do {
       Ring& C = c.R[side];
       const int m = C.m;
+      if (again.seen(V, side)) { if (g.rank() == 0) fail(c, DEV_TRACE); return false; }
       int8_t st = toggled(C.ee(V));
       const int dir = ((st == E_EXIT) ^ c.uni) ? 1 : -1;
       int L = -1;
@@ -2345,6 +2538,61 @@ __device__ bool grp_trace(const G& g, PairCtx& c) {
     O.end();
     from = I + 1;
   }
+  return true;
+}
+
+// Vertices were added to the rings (linked in after their place, kept in slots past the
+// merged ring): puts both rings back into slot order, so that they are traced like rings
+// without added vertices.  Coordinates go through the free end of the pair's output region,
+// the rest through scratch columns.
+template <class G>
+__device__ bool grp_linearize(const G& g, PairCtx& c) {
+  for (int sd = 0; sd < 2; ++sd) {                       // to: new slot of each vertex
+    Ring& A = c.R[sd];
+    int added = 0;
+    for (int b = 0; b < A.m; b += g.size()) {
+      const int s = b + g.rank();
+      int k = 0;
+      if (s < A.m)
+        for (int v = A.nx(s); v >= A.m && k <= A.used - A.m; v = A.nx(v)) ++k;
+      int tot;
+      const int at = s + added + g.incl_scan(k, tot) - k;
+      if (s < A.m) {
+        A.to(s) = at;
+        int v = A.nx(s);
+        for (int i = 1; i <= k; ++i) { A.to(v) = at + i; v = A.nx(v); }
+      }
+      added += tot;
+    }
+    if (A.m + added != A.used) return false;             // not reached from its place: left to the links
+  }
+  if (c.O.nv + max(c.R[0].used, c.R[1].used) > c.O.vcap) return false;
+  g.sync();
+  double2* stage = reinterpret_cast<double2*>(c.O.xy) + c.O.nv;
+  for (int sd = 0; sd < 2; ++sd) {
+    Ring& A = c.R[sd];
+    const Ring& B = c.R[1 - sd];
+    for (int s = g.rank(); s < A.used; s += g.size()) {
+      const int at = A.to(s), nb = A.nb(s);
+      stage[at] = A.xy(s);
+      A.tn(at) = nb >= 0 && nb < B.used ? B.to(nb) : nb;
+      A.tl(at) = (int)A.it(s) | ((int)(uint8_t)A.lb(s) << 8) | ((int)(uint8_t)A.ee(s) << 16);
+    }
+    g.sync();
+    for (int s = g.rank(); s < A.used; s += g.size()) {
+      A.xy(s) = stage[s];
+      A.nb(s) = A.tn(s);
+      const int v = A.tl(s);
+      A.it(s) = (uint8_t)v;
+      A.lb(s) = (int8_t)(v >> 8);
+      A.ee(s) = (int8_t)(v >> 16);
+      A.nx(s) = s + 1 < A.used ? s + 1 : 0;
+      A.pv(s) = s > 0 ? s - 1 : A.used - 1;
+    }
+    g.sync();
+  }
+  c.R[0].m = c.R[0].used;
+  c.R[1].m = c.R[1].used;
   return true;
 }
 
@@ -2542,7 +2790,7 @@ struct LabelArgs {
   int64_t bigLabelMin;        // rings above: the grid path
   const unsigned long long* midCount;
   unsigned long long* midNext; // work-stealing cursor of the block kernel
-  int blockRunCap;            // runs the block kernel's shared run table holds (0: none)
+  int blockLoopCap;           // segments the block kernel's shared loop table holds (0: none)
   // The one-thread, warp and block pairs in size order, largest first (label_order_kernel):
   // the one-thread kernel takes order[0, nTile), the warp kernel order[nTile, nTile + nWarp),
   // the block kernel the *midCount entries after those.
@@ -2589,7 +2837,13 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
   if (!grp_step4<EX>(g, c, tempAfter, tempSlot)) return;
   if (grp_any_split(g, c.R[0], c.R[1])) {
     bool ok = true;
-    if (lead) ok = seq_step5<EX>(c);
+    int n = -1;
+    if constexpr (!G::kSolo) {
+      Ring& P = c.R[0];
+      n = g.list(P.used, [&](int s) { return (P.fl(s) & 1) != 0; }, [&](int s, bool hit, int before) { if (hit) P.ls(before) = s; });
+      g.sync();
+    }
+    if (lead) ok = seq_step5<EX>(c, n);
     ok = g.bcast0((int)ok);
     c.R[0].used = g.bcast0(c.R[0].used);
     c.R[1].used = g.bcast0(c.R[1].used);
@@ -2597,7 +2851,10 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
     if (!ok) return;
   }
   grp_step6(g, c);
-  const bool added = c.R[0].used != c.R[0].m || c.R[1].used != c.R[1].m;
+  bool added = c.R[0].used != c.R[0].m || c.R[1].used != c.R[1].m;
+  if constexpr (!G::kSolo) {
+    if (added) added = !grp_linearize(g, c);
+  }
   if (added) {
     // vertices were added to a ring: trace through the next/prev links on one member
     int ok = 1;
@@ -2610,8 +2867,8 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
     if (!ok) return;
   } else {
     int r;
-    if constexpr (G::kBlock) r = grp_trace_runs(g, c);
-    else r = grp_trace_runs_slots(g, c);
+    if constexpr (G::kSolo) r = grp_trace_runs_slots(g, c);
+    else r = grp_trace_loops(g, c);
     if (r < 0) return;
     if (r > 0 && !grp_trace(g, c)) return;
   }
@@ -2707,10 +2964,10 @@ __global__ void label_order_kernel(const int32_t* __restrict__ mP, const int32_t
 template <int EX>
 __global__ void __launch_bounds__(kBlockLabelThreads)
 label_trace_block_kernel(LabelArgs a) {
-  __shared__ long long sm[kBlockLabelThreads / 32 + 1];
+  __shared__ long long sm[kBlockScratch];
   __shared__ long long next;
-  extern __shared__ int32_t runTable[];
-  BlockGroup g{sm, runTable, a.blockRunCap};
+  extern __shared__ uint32_t loopTable[];
+  BlockGroup g{sm, loopTable, a.blockLoopCap};
   const unsigned long long n = *a.midCount;
   for (;;) {
     if (threadIdx.x == 0) next = (long long)atomicAdd(a.midNext, 1ull);
@@ -4100,13 +4357,13 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
       ls = aux;
     }
     if (nMid > 0) {
-      // The run table goes to shared memory only when block pairs make up at least a
+      // The loop table goes to shared memory only when block pairs make up at least a
       // quarter of the batch: otherwise the one-thread and warp kernels beside this one
       // need the SMs' L1 more (batched workload: label stage 2.02 -> 2.52 ms with it).
-      const int smem = (4 * nMid >= K) ? kBlockRunTableBytes : 0;
+      const int smem = (4 * nMid >= K) ? kBlockLoopTableBytes : 0;
       auto kern = prm.exact ? label_trace_block_kernel<1> : label_trace_block_kernel<0>;
       if (smem) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      la.blockRunCap = smem / 12;
+      la.blockLoopCap = smem / 12;
       kern<<<(unsigned)std::min<int64_t>(2 * nsm, nMid), kBlockLabelThreads, smem, ls>>>(la);
       note_launch();
     }
