@@ -1845,9 +1845,8 @@ __device__ bool grp_step2(const G& g, PairCtx& c) {
 // copies ring A (slot order, no added vertices) as one output component
 template <class G>
 __device__ void grp_push_ring(const G& g, OutRegion& O, const Ring& A) {
-  O.begin();
-  if (O.overflow) return;
-  if (O.nv + A.m > O.vcap) { O.overflow = true; return; }
+  // (the size is written by one member only: no begin(), whose zero another could write later)
+  if (O.nc >= O.ccap || O.nv + A.m > O.vcap) { O.overflow = true; return; }
   for (int s = g.rank(); s < A.m; s += g.size()) { O.xy[2 * (O.nv + s)] = A.x(s); O.xy[2 * (O.nv + s) + 1] = A.y(s); }
   if (g.rank() == 0) O.csz[O.nc] = A.m;
   O.nv += A.m;
