@@ -295,6 +295,40 @@ GCMFGH_DEV int classify_exact(double p1x, double p1y, double p2x, double p2y,
   return tp;
 }
 
+// classify_exact from both sides, out of line: for the edge pairs that classify_exact_both's
+// filter leaves open.
+__device__ __noinline__ int classify_exact_open(double2 P1, double2 P2, double2 Q1, double2 Q2, double2* ab, bool* qhit);
+
+// classify_exact of (P, Q) and whether classify_exact of (Q, P) finds an intersection.  When
+// the four areas' FP64 values decide their signs (the bound of exact_sign) and none is zero,
+// the edges cross properly or not at all, for both sides alike; everything else goes to the
+// full classification.
+GCMFGH_DEV int classify_exact_both(double2 P1, double2 P2, double2 Q1, double2 Q2, double& alpha, double& beta,
+                                   bool& qhit) {
+  bool open = false;
+  auto area = [&open](double2 a, double2 b, double2 c) {
+    const double left = (b.x - a.x) * (c.y - a.y), right = (b.y - a.y) * (c.x - a.x);
+    const double det = left - right;
+    if (!(fabs(det) >= 3.3306690738754716e-16 * (fabs(left) + fabs(right))) || det == 0.0) open = true;
+    return det;
+  };
+  const double AP1 = area(P1, Q1, Q2), AP2 = area(P2, Q1, Q2);
+  const double AQ1 = area(Q1, P1, P2), AQ2 = area(Q2, P1, P2);
+  if (open) {
+    double2 ab = make_double2(0.0, 0.0);
+    const int t = classify_exact_open(P1, P2, Q1, Q2, &ab, &qhit);
+    alpha = ab.x;
+    beta = ab.y;
+    return t;
+  }
+  const bool hit = (AP1 > 0.0) != (AP2 > 0.0) && (AQ1 > 0.0) != (AQ2 > 0.0);
+  qhit = hit;
+  if (!hit) return 0;
+  alpha = crossing_param(AP1, AP2);
+  beta = crossing_param(AQ1, AQ2);
+  return 1;
+}
+
 GCMFGH_DEV int classify_exact_call(double p1x, double p1y, double p2x, double p2y, double q1x,
                                    double q1y, double q2x, double q2y, double* ab) {
   return classify_exact(p1x, p1y, p2x, p2y, q1x, q1y, q2x, q2y, ab[0], ab[1]);

@@ -43,6 +43,12 @@
 
 namespace gcmfgh {
 
+__device__ __noinline__ int classify_exact_open(double2 P1, double2 P2, double2 Q1, double2 Q2, double2* ab, bool* qhit) {
+  double a2, b2;
+  *qhit = classify_exact(Q1.x, Q1.y, Q2.x, Q2.y, P1.x, P1.y, P2.x, P2.y, a2, b2) != 0;
+  return classify_exact(P1.x, P1.y, P2.x, P2.y, Q1.x, Q1.y, Q2.x, Q2.y, ab->x, ab->y);
+}
+
 namespace {
 
 constexpr int kThreads = 256;
@@ -451,7 +457,7 @@ __global__ void pair_records_kernel(const int64_t* __restrict__ chunkOff, const 
 // is tested exactly once (cell indices are monotone in the coordinate).  All binned pairs
 // go through the same launches: their P and Q edges are numbered consecutively (pair by
 // pair) and each edge finds its pair through an owner table.
-struct BinGrid { double x0, y0, cw, ch; int gx, gy; };
+struct BinGrid { double x0, y0, cw, ch; int gx, gy; float M; };   // M: range of the FP32 copies
 
 __device__ __forceinline__ int cell_1d(double v, double c0, double cs, int g) {
   double t = (v - c0) / cs;
@@ -520,9 +526,10 @@ __global__ void bin_extent_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S,
   }
 }
 
-// Grid of each binned pair: about one Q edge per cell, but never cells smaller than the
-// Q edges' mean box (long edges would otherwise be listed in many cells and each P edge
-// would scan them all again); at most 4096 cells per axis.
+// Grid of each binned pair: about one Q edge per cell, but never cells smaller than half the
+// Q edges' mean box (long edges would otherwise be listed in many cells); at most 4096 cells
+// per axis.  (Count + emit of the 400,000 x 200,000-vertex pair: 22.4 ms with cells of the
+// mean box, 18.6 ms with half, 17.2 ms with a quarter; degenerate batch 10.4, 10.5, 10.8 ms.)
 __global__ void bin_grid_kernel(PairDev D, BinSet S, int n) {
   int i = blockIdx.x * kThreads + threadIdx.x;
   if (i >= n) return;
@@ -535,8 +542,8 @@ __global__ void bin_grid_kernel(PairDev D, BinSet S, int n) {
     gx = ceil(sqrt(target * w / h));
     gx = fmin(fmax(gx, 1.0), 4096.0);
     gy = ceil(target / gx);
-    if (mw > 0) gx = fmin(gx, ceil(w / mw));
-    if (mh > 0) gy = fmin(gy, ceil(h / mh));
+    if (mw > 0) gx = fmin(gx, ceil(2.0 * w / mw));
+    if (mh > 0) gy = fmin(gy, ceil(2.0 * h / mh));
     gx = fmin(fmax(gx, 1.0), 4096.0);
     gy = fmin(fmax(gy, 1.0), 4096.0);
   } else if (w > 0) {
@@ -544,17 +551,41 @@ __global__ void bin_grid_kernel(PairDev D, BinSet S, int n) {
   } else if (h > 0) {
     gy = fmin(target, 4096.0);
   }
-  BinGrid G{c.x, c.y, w > 0 ? w / gx : 1.0, h > 0 ? h / gy : 1.0, (int)gx, (int)gy};
+  BinGrid G{c.x, c.y, w > 0 ? w / gx : 1.0, h > 0 ? h / gy : 1.0, (int)gx, (int)gy,
+            __double2float_ru(2.0 * fmax(fmax(w, h), 0.0))};
   S.grid[i] = G;
   S.ncell[i] = G.gx * G.gy;
 }
 
-// kMode 0: count the listings per cell; kMode 1: list every Q edge in the cells its box covers
+// A Q edge is listed in every cell its box covers.  Within a cell the listings stand in four
+// classes, by whether the cell is in the first column and the first row of the edge's box:
+//   0 first column only, 1 both, 2 first row only, 3 neither
+// so that a P edge's visits meet each Q edge once, in the cell of their overlap's lower
+// left corner, without testing for it: from the corner cell of its own box it takes all
+// classes, from the other cells of the first row those of first-column cells (0, 1), from the
+// other cells of the first column those of first-row cells (1, 2), elsewhere class 1.
+__device__ __forceinline__ int bin_class(bool firstCol, bool firstRow) {
+  return firstCol ? (firstRow ? 1 : 0) : (firstRow ? 2 : 3);
+}
+
+// The FP32 copy of an edge relative to the grid's corner (four NaNs when it leaves the
+// range M: no FP32 test then rejects it).  Each value is within M * 2^-24 of the exact one.
+__device__ __forceinline__ float4 bin_edge_f32(double2 a, double2 b, const BinGrid& G) {
+  const float4 r = make_float4(__double2float_rn(a.x - G.x0), __double2float_rn(a.y - G.y0),
+                               __double2float_rn(b.x - G.x0), __double2float_rn(b.y - G.y0));
+  const float m = fmaxf(fmaxf(fabsf(r.x), fabsf(r.y)), fmaxf(fabsf(r.z), fabsf(r.w)));
+  const float nan = __int_as_float(0x7fffffff);
+  return m <= G.M ? r : make_float4(nan, nan, nan, nan);
+}
+
+// kMode 0: count the listings per cell and class; kMode 1: list every Q edge in the cells its
+// box covers, with its FP32 copy when cellBox is given
 template <int kMode>
 __global__ void bin_cells_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, int64_t nq,
                                  const int64_t* __restrict__ offQ, const int32_t* __restrict__ LQ,
                                  int32_t* __restrict__ cellCnt, const int64_t* __restrict__ cellOff,
-                                 int32_t* __restrict__ cursor, int32_t* __restrict__ cellList) {
+                                 int32_t* __restrict__ cursor, int32_t* __restrict__ cellList,
+                                 float4* __restrict__ cellBox) {
   const int64_t j = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   if (j >= nq) return;
   const int i = S.ownQ[j];
@@ -567,28 +598,30 @@ __global__ void bin_cells_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, 
   const int64_t cb = S.cellBase[i];
   const int x0 = cell_1d(fmin(a.x, b.x), G.x0, G.cw, G.gx), x1 = cell_1d(fmax(a.x, b.x), G.x0, G.cw, G.gx);
   const int y0 = cell_1d(fmin(a.y, b.y), G.y0, G.ch, G.gy), y1 = cell_1d(fmax(a.y, b.y), G.y0, G.ch, G.gy);
+  const float4 box = (kMode == 1 && cellBox) ? bin_edge_f32(a, b, G) : make_float4(0.f, 0.f, 0.f, 0.f);
   for (int y = y0; y <= y1; ++y)
     for (int x = x0; x <= x1; ++x) {
-      const int64_t c = cb + (int64_t)y * G.gx + x;
+      const int64_t c = 4 * (cb + (int64_t)y * G.gx + x) + bin_class(x == x0, y == y0);
       if (kMode == 0) atomicAdd(&cellCnt[c], 1);
-      else cellList[cellOff[c] + atomicAdd(&cursor[c], 1)] = q;
+      else {
+        const int64_t at = cellOff[c] + atomicAdd(&cursor[c], 1);
+        cellList[at] = q;
+        if (cellBox) cellBox[at] = box;
+      }
     }
 }
 
-// kMode 0: per binned P edge, its records (P side) into recCnt, and the pair's Q-side
-// count into binQ; kMode 1: write the records of each P edge at its offset (in cell
-// order: nothing downstream depends on record order).  The offset is the pair's recOff
-// plus the edge's place in the pair, or, with recOff null (after the fused count + emit
-// of the chunked pairs), *recBase plus the edge's place among all binned edges; records
-// at or past cap are not written.
+// The record export's two passes over the binned pairs, a thread per P edge.  kMode 0: per
+// binned P edge, its records (P side) into recCnt, and the pair's Q-side count into binQ;
+// kMode 1: write the records of each P edge at its offset, the pair's recOff plus the edge's
+// place in the pair (in cell order: nothing downstream depends on that).
 template <int kMode, int kExact>
 __global__ void __launch_bounds__(kThreads, kExact ? 2 : 4)
 bin_pairs_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, int64_t np,
                  const int64_t* __restrict__ offP, const int32_t* __restrict__ LP,
                  const int64_t* __restrict__ cellOff, const int32_t* __restrict__ cellList, double eps,
                  int32_t* __restrict__ recCnt, int64_t* __restrict__ binQ,
-                 const int64_t* __restrict__ recPos, const int64_t* __restrict__ recOff, Records R,
-                 const unsigned long long* __restrict__ recBase, int64_t cap) {
+                 const int64_t* __restrict__ recPos, const int64_t* __restrict__ recOff, Records R) {
   const int64_t j = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   if (j >= np) return;
   const int i = S.ownP[j];
@@ -606,18 +639,15 @@ bin_pairs_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, int64_t np,
   const int x0 = cell_1d(pminx, G.x0, G.cw, G.gx), x1 = cell_1d(pmaxx, G.x0, G.cw, G.gx);
   const int y0 = cell_1d(pminy, G.y0, G.ch, G.gy), y1 = cell_1d(pmaxy, G.y0, G.ch, G.gy);
   int recs = 0, qhits = 0;
-  const int64_t base = (kMode == 0) ? 0
-                       : recOff ? recOff[k] + recPos[j] - recPos[S.pBase[i]]
-                                : (int64_t)*recBase + recPos[j];
+  const int64_t base = (kMode == 0) ? 0 : recOff[k] + recPos[j] - recPos[S.pBase[i]];
   for (int y = y0; y <= y1; ++y)
     for (int x = x0; x <= x1; ++x) {
-      const int64_t c = cb + (int64_t)y * G.gx + x;
-      for (int64_t e = cellOff[c]; e < cellOff[c + 1]; ++e) {
+      const int64_t c = 4 * (cb + (int64_t)y * G.gx + x);
+      const int64_t e1 = cellOff[c + (y == y0 ? (x == x0 ? 4 : 2) : (x == x0 ? 3 : 2))];
+      for (int64_t e = cellOff[c + (y == y0 ? 0 : 1)]; e < e1; ++e) {
         const int q = cellList[e];
         const double2 Q1 = __ldg(qv + q), Q2 = __ldg(qv + (q + 1 < nq ? q + 1 : 0));
         if (!edge_boxes_touch(P1.x, P1.y, P2.x, P2.y, Q1.x, Q1.y, Q2.x, Q2.y)) continue;
-        const double cx = fmax(pminx, fmin(Q1.x, Q2.x)), cy = fmax(pminy, fmin(Q1.y, Q2.y));
-        if (cell_1d(cx, G.x0, G.cw, G.gx) != x || cell_1d(cy, G.y0, G.ch, G.gy) != y) continue;
         double alpha = 0, beta = 0;
         const int tp = classify_mode(kExact, P1.x, P1.y, P2.x, P2.y, Q1.x, Q1.y, Q2.x, Q2.y, eps, alpha, beta);
         if (kMode == 0) {
@@ -626,9 +656,7 @@ bin_pairs_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, int64_t np,
           if (tp) ++recs;
         } else if (tp) {
           const int64_t r = base + recs++;
-          if (r < cap) {
-            R.p[r] = p; R.q[r] = q; R.a[r] = alpha; R.b[r] = beta; R.t[r] = (int8_t)tp; R.k[r] = (int32_t)k;
-          }
+          R.p[r] = p; R.q[r] = q; R.a[r] = alpha; R.b[r] = beta; R.t[r] = (int8_t)tp; R.k[r] = (int32_t)k;
         }
       }
     }
@@ -636,6 +664,159 @@ bin_pairs_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, int64_t np,
     recCnt[j] = recs;
     if (qhits) atomicAdd(reinterpret_cast<unsigned long long*>(binQ + k), (unsigned long long)qhits);
   }
+}
+
+// Whether two edges that meet may be rejected on their FP32 copies: true only when the exact
+// boxes are apart, or (exact predicates) both ends of one edge lie strictly on one side
+// of the other, the sign tests having room for the copies' and the arithmetic's rounding.
+// With d = M 2^-24 the copies' error, A and B the 1-norms of the two differences that an
+// area is the cross product of (each at most 4 M), the area's error is below
+// 2 d (A + B) + 4 d min(A, B) + 8 d^2 + 4 2^-24 A B < 24 d (A + B + d); 32 is used.
+template <int kExact>
+__device__ __forceinline__ bool bin_f32_rejects(float4 p, float4 q, float M) {
+  const float slop = M * 2.3841858e-7f;                                  // 2^-22
+  if (fminf(q.x, q.z) > fmaxf(p.x, p.z) + slop || fmaxf(q.x, q.z) < fminf(p.x, p.z) - slop) return true;
+  if (fminf(q.y, q.w) > fmaxf(p.y, p.w) + slop || fmaxf(q.y, q.w) < fminf(p.y, p.w) - slop) return true;
+  if (!kExact) return false;
+  const float d = M * 1.9073486e-6f;                                     // 32 * 2^-24 M
+  const float px = p.z - p.x, py = p.w - p.y, qx = q.z - q.x, qy = q.w - q.y;
+  // An edge of no length is collinear with everything (classify_exact's second branch goes
+  // by projections alone); copies that differ show that the ends do.
+  if ((px == 0.f && py == 0.f) || (qx == 0.f && qy == 0.f)) return false;
+  const float ax = q.x - p.x, ay = q.y - p.y;                            // P1 -> Q1
+  const float bx = q.z - p.x, by = q.w - p.y;                            // P1 -> Q2
+  const float cx = q.x - p.z, cy = q.y - p.w;                            // P2 -> Q1
+  const float A = fabsf(px) + fabsf(py) + M * 5.9604645e-8f, B = fabsf(qx) + fabsf(qy) + M * 5.9604645e-8f;
+  const float s1 = px * ay - py * ax, s2 = px * by - py * bx;            // Q1, Q2 beside P
+  const float e1 = d * (A + fabsf(ax) + fabsf(ay)), e2 = d * (A + fabsf(bx) + fabsf(by));
+  if ((s1 > e1 && s2 > e2) || (s1 < -e1 && s2 < -e2)) return true;
+  const float t1 = qx * ay - qy * ax, t2 = qx * cy - qy * cx;            // P1, P2 beside Q (sign of both flipped)
+  const float f1 = d * (B + fabsf(ax) + fabsf(ay)), f2 = d * (B + fabsf(cx) + fabsf(cy));
+  return (t1 > f1 && t2 > f2) || (t1 < -f1 && t2 < -f2);
+}
+
+// Count and emit of the binned pairs in one pass, a warp per kBinEdges consecutive P edges.
+// The listings of a P edge's cells are taken as one run, 32 at a time (the cells' shares
+// by a scan, so that many small cells fill the lanes as well as one large one), tested on
+// their FP32 copies with coalesced loads, and the few that pass are queued in shared
+// memory until 32 of them can be classified in FP64 by a full warp.  The records go to a
+// range of the global counter taken per classified group, as in intersect_fused_kernel.
+// Bound by instruction issue.  A thread per P edge enumerating its listings in FP64, once to
+// count and once to emit, took 271 ms for the 400,000 x 200,000-vertex pair (2.9e7
+// records) and 31.3 ms for the degenerate batch of 10,007 pairs (2.3e7), this 18.6 and 10.5 ms.
+// (3 blocks per SM at 80 registers: 22.4 ms against 27.2 ms for 2 at 128, cells of the mean box.)
+constexpr int kBinEdges = 8;
+
+template <int kExact>
+__global__ void __launch_bounds__(kThreads, 3)
+bin_append_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, int64_t np,
+                  const int64_t* __restrict__ offP, const int32_t* __restrict__ LP,
+                  const int64_t* __restrict__ cellOff, const int32_t* __restrict__ cellList,
+                  const float4* __restrict__ cellBox, double eps, Records R, FusedRecords F,
+                  unsigned long long* __restrict__ binRec, unsigned long long* __restrict__ binQ) {
+  __shared__ int2 queue[kWarpsPerBlock][64];
+  int2* const wq = queue[threadIdx.x >> 5];
+  const int lane = (int)lane_id();
+  const int64_t j0 = (((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5) * kBinEdges;
+  const int64_t j1 = min(j0 + kBinEdges, np);
+  int cur = -1, queued = 0, np_ = 0, nq = 0;
+  int64_t k = 0;
+  unsigned recs = 0, qhits = 0;
+  const double2* pv = nullptr;
+  const double2* qv = nullptr;
+  BinGrid G{};
+  int64_t cb = 0;
+  // classifies the queue's last n entries
+  auto classify = [&](int n) {
+    int tp = 0, pe = 0, qe = 0;
+    bool tq = false;
+    double alpha = 0, beta = 0;
+    __syncwarp();
+    if (lane < n) {
+      const int2 pq = wq[queued - n + lane];
+      pe = pq.x;
+      qe = pq.y;
+      const double2 P1 = __ldg(pv + pe), P2 = __ldg(pv + (pe + 1 < np_ ? pe + 1 : 0));
+      const double2 Q1 = __ldg(qv + qe), Q2 = __ldg(qv + (qe + 1 < nq ? qe + 1 : 0));
+      if (edge_boxes_touch(P1.x, P1.y, P2.x, P2.y, Q1.x, Q1.y, Q2.x, Q2.y)) {
+        if (kExact) tp = classify_exact_both(P1, P2, Q1, Q2, alpha, beta, tq);
+        else tp = classify_edges_both(P1.x, P1.y, P2.x, P2.y, Q1.x, Q1.y, Q2.x, Q2.y, eps, alpha, beta, tq);
+      }
+    }
+    __syncwarp();
+    queued -= n;
+    const unsigned m = __ballot_sync(0xffffffffu, tp != 0);
+    recs += __popc(m);
+    qhits += __popc(__ballot_sync(0xffffffffu, tq));
+    if (m) {
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(F.total, (unsigned long long)__popc(m));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      const int64_t r = (int64_t)base + __popc(m & lanemask_lt());
+      if (tp != 0 && r < F.cap) {
+        R.p[r] = pe; R.q[r] = qe; R.a[r] = alpha; R.b[r] = beta; R.t[r] = (int8_t)tp; R.k[r] = (int32_t)k;
+      }
+    }
+  };
+  auto finish_pair = [&]() {
+    if (queued) classify(queued);
+    if (lane == 0 && binRec) {
+      if (recs) atomicAdd(binRec + k, (unsigned long long)recs);
+      if (qhits) atomicAdd(binQ + k, (unsigned long long)qhits);
+    }
+    recs = qhits = 0;
+  };
+  for (int64_t j = j0; j < j1; ++j) {
+    const int i = S.ownP[j];
+    if (i != cur) {
+      if (cur >= 0) finish_pair();
+      cur = i;
+      k = S.list[i];
+      const int pside = D.pSide[k];
+      pv = layer_xy(Lb, Lo, pside) + D.pS[k];
+      qv = layer_xy(Lb, Lo, 1 - pside) + D.qS[k];
+      np_ = D.nP[k];
+      nq = D.nQ[k];
+      G = S.grid[i];
+      cb = S.cellBase[i];
+    }
+    const int p = binned_p(S, j, i, offP, LP);
+    const double2 P1 = __ldg(pv + p), P2 = __ldg(pv + (p + 1 < np_ ? p + 1 : 0));
+    const float4 pf = bin_edge_f32(P1, P2, G);
+    const int x0 = cell_1d(fmin(P1.x, P2.x), G.x0, G.cw, G.gx), x1 = cell_1d(fmax(P1.x, P2.x), G.x0, G.cw, G.gx);
+    const int y0 = cell_1d(fmin(P1.y, P2.y), G.y0, G.ch, G.gy), y1 = cell_1d(fmax(P1.y, P2.y), G.y0, G.ch, G.gy);
+    const int wx = x1 - x0 + 1, cells = wx * (y1 - y0 + 1);
+    for (int c0 = 0; c0 < cells; c0 += 32) {
+      int64_t from = 0;
+      int len = 0;
+      if (c0 + lane < cells) {
+        const int cy = (c0 + lane) / wx, cx = (c0 + lane) - cy * wx;
+        const int64_t c = 4 * (cb + (int64_t)(y0 + cy) * G.gx + x0 + cx);
+        from = cellOff[c + (cy == 0 ? 0 : 1)];
+        len = (int)(cellOff[c + (cy == 0 ? (cx == 0 ? 4 : 2) : (cx == 0 ? 3 : 2))] - from);
+      }
+      const int incl = warp_incl_scan(len);
+      const int total = __shfl_sync(0xffffffffu, incl, 31);
+      from -= incl - len;                                // listing of flat index t: from + t
+      for (int t0 = 0; t0 < total; t0 += 32) {
+        const int t = t0 + lane;
+        int lo = 0;                                      // the cell: shares whose scan is <= t
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) {
+          const int v = __shfl_sync(0xffffffffu, incl, lo + w - 1);
+          if (v <= t) lo += w;
+        }
+        const int64_t e = __shfl_sync(0xffffffffu, from, lo & 31) + t;
+        bool keep = false;
+        if (t < total) keep = !bin_f32_rejects<kExact>(pf, __ldg(cellBox + e), G.M);
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) wq[queued + __popc(m & lanemask_lt())] = make_int2(p, cellList[e]);
+        queued += __popc(m);
+        if (queued >= 32) classify(32);
+      }
+    }
+  }
+  if (cur >= 0) finish_pair();
 }
 
 // per binned pair: its records (the P edges' counts summed through their scan)
@@ -3940,8 +4121,11 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     cudaMemsetAsync(recTot, 0, sizeof(unsigned long long), s);
     cudaMemsetAsync(pairRec, 0, K * sizeof(int32_t), s);
     cudaMemsetAsync(pairQ, 0, K * sizeof(int32_t), s);
+    if (sb != s) {                                  // the counter is cleared before either starts
+      cudaEventRecord(bev[0], s);
+      cudaStreamWaitEvent(sb, bev[0], 0);
+    }
     launch_fused(true);
-    if (sb != s) cudaEventRecord(bev[0], s);        // the binned records go after the chunked ones
   } else if (nCh > 0) {
     { (prm.exact ? intersect_kernel<0, 1> : intersect_kernel<0, 0>)<<<blocks_for_warps(nCh), kThreads, 0, s>>>(
         Lb, Lo, D, K, chunkOff, nCh, cP, cQ, offP, offQ, LP, LQ, prm.eps, chunkRec, chunkQ, nullptr, nullptr, R, chunkPair); note_launch(); }
@@ -3955,7 +4139,19 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   int64_t nBinP = 0, nBinQ = 0;
   int64_t* cellOff = nullptr;
   int32_t* cellList = nullptr;
+  float4* cellBox = nullptr;
   int64_t* binRecPos = nullptr;
+  // the binned pairs' records, beside the chunked ones (one counter for both)
+  auto launch_binned = [&](cudaStream_t st, bool countPairs) {
+    if (nBinP == 0) return;
+    const FusedRecords F{recTot, recCap, nullptr, nullptr};
+    auto u64 = [](int64_t* p) { return reinterpret_cast<unsigned long long*>(p); };
+    (prm.exact ? bin_append_kernel<1> : bin_append_kernel<0>)<<<blocks_for_warps((nBinP + kBinEdges - 1) / kBinEdges),
+                                                               kThreads, 0, st>>>(
+        Lb, Lo, D, BS, nBinP, offP, LP, cellOff, cellList, cellBox, prm.eps, R, F, countPairs ? u64(binRec) : nullptr,
+        u64(binQ));
+    note_launch();
+  };
   if (nBigPairs > 0) {
     const int B = nBigPairs;
     BS.list = bigList;
@@ -3988,39 +4184,38 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     cudaMemcpyAsync(hs + 42, d_t + 2, sizeof(int64_t), cudaMemcpyDeviceToHost, sb);
     if (!syncb()) return ST_CUDA_ERROR;
     const int64_t nCells = hs[42];
-    int32_t* cellCnt = A.take_n<int32_t>(nCells + 1);
-    cellOff = A.take_n<int64_t>(nCells + 1);
-    int32_t* cursor = A.take_n<int32_t>(nCells);
-    void* stCell = A.take(scan_temp_bytes(nCells + 1));
-    if (!cellCnt || !cellOff || !cursor || !stCell) return ST_OUT_OF_MEMORY;
-    cudaMemsetAsync(cellCnt, 0, (nCells + 1) * sizeof(int32_t), sb);
-    cudaMemsetAsync(cursor, 0, nCells * sizeof(int32_t), sb);
+    const int64_t nCls = 4 * nCells;                // four listing classes per cell
+    int32_t* cellCnt = A.take_n<int32_t>(nCls + 1);
+    cellOff = A.take_n<int64_t>(nCls + 1);
+    void* stCell = A.take(scan_temp_bytes(nCls + 1));
+    if (!cellCnt || !cellOff || !stCell) return ST_OUT_OF_MEMORY;
+    cudaMemsetAsync(cellCnt, 0, (nCls + 1) * sizeof(int32_t), sb);
     if (nBinQ > 0)
       { bin_cells_kernel<0><<<blocks_for(nBinQ), kThreads, 0, sb>>>(Lb, Lo, D, BS, nBinQ, offQ, LQ, cellCnt, nullptr,
-                                                                   nullptr, nullptr); note_launch(); }
-    exclusive_scan_i32(cellCnt, cellOff, nCells + 1, d_t + 3, stCell, d_err, sb);
+                                                                   nullptr, nullptr, nullptr); note_launch(); }
+    exclusive_scan_i32(cellCnt, cellOff, nCls + 1, d_t + 3, stCell, d_err, sb);
     cudaMemcpyAsync(hs + 43, d_t + 3, sizeof(int64_t), cudaMemcpyDeviceToHost, sb);
+    cudaMemsetAsync(cellCnt, 0, nCls * sizeof(int32_t), sb);        // the listing cursors
     if (!syncb()) return ST_CUDA_ERROR;
     cellList = A.take_n<int32_t>(hs[43]);
-    int32_t* binRecCnt = A.take_n<int32_t>(nBinP + 1);
-    binRecPos = A.take_n<int64_t>(nBinP + 1);
-    void* stP = A.take(scan_temp_bytes(nBinP + 1));
-    if (!cellList || !binRecCnt || !binRecPos || !stP) return ST_OUT_OF_MEMORY;
+    if (fused) cellBox = A.take_n<float4>(hs[43]);
+    if (!cellList || (fused && !cellBox)) return ST_OUT_OF_MEMORY;
     if (nBinQ > 0)
       { bin_cells_kernel<1><<<blocks_for(nBinQ), kThreads, 0, sb>>>(Lb, Lo, D, BS, nBinQ, offQ, LQ, nullptr, cellOff,
-                                                                   cursor, cellList); note_launch(); }
-    cudaMemsetAsync(binRecCnt + nBinP, 0, sizeof(int32_t), sb);     // so the scan's last entry is the total
-    if (nBinP > 0)
-      { (prm.exact ? bin_pairs_kernel<0, 1> : bin_pairs_kernel<0, 0>)<<<blocks_for(nBinP), kThreads, 0, sb>>>(
-            Lb, Lo, D, BS, nBinP, offP, LP, cellOff, cellList, prm.eps, binRecCnt, binQ, nullptr, nullptr, R, nullptr,
-            INT64_MAX); note_launch(); }
-    exclusive_scan_i32(binRecCnt, binRecPos, nBinP + 1, nullptr, stP, d_err, sb);
-    { bin_rec_total_kernel<<<blocks_for(B), kThreads, 0, sb>>>(BS, B, binRecPos, binRec); note_launch(); }
-    if (fused && nBinP > 0) {                       // emit now, after the chunked records
-      if (sb != s) cudaStreamWaitEvent(sb, bev[0], 0);
-      { (prm.exact ? bin_pairs_kernel<1, 1> : bin_pairs_kernel<1, 0>)<<<blocks_for(nBinP), kThreads, 0, sb>>>(
-            Lb, Lo, D, BS, nBinP, offP, LP, cellOff, cellList, prm.eps, nullptr, nullptr, binRecPos, nullptr, R,
-            recTot, recCap); note_launch(); }
+                                                                   cellCnt, cellList, cellBox); note_launch(); }
+    if (fused) {
+      launch_binned(sb, true);
+    } else {
+      int32_t* binRecCnt = A.take_n<int32_t>(nBinP + 1);
+      binRecPos = A.take_n<int64_t>(nBinP + 1);
+      void* stP = A.take(scan_temp_bytes(nBinP + 1));
+      if (!binRecCnt || !binRecPos || !stP) return ST_OUT_OF_MEMORY;
+      cudaMemsetAsync(binRecCnt + nBinP, 0, sizeof(int32_t), sb);   // so the scan's last entry is the total
+      if (nBinP > 0)
+        { (prm.exact ? bin_pairs_kernel<0, 1> : bin_pairs_kernel<0, 0>)<<<blocks_for(nBinP), kThreads, 0, sb>>>(
+              Lb, Lo, D, BS, nBinP, offP, LP, cellOff, cellList, prm.eps, binRecCnt, binQ, nullptr, nullptr, R); note_launch(); }
+      exclusive_scan_i32(binRecCnt, binRecPos, nBinP + 1, nullptr, stP, d_err, sb);
+      { bin_rec_total_kernel<<<blocks_for(B), kThreads, 0, sb>>>(BS, B, binRecPos, binRec); note_launch(); }
     }
   }
   if (sb != s) {
@@ -4038,19 +4233,15 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   if (fused) {
     mk->mark("clip:count+emit", s);
     cudaMemcpyAsync(hs, recTot, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-    if (nBinP > 0) cudaMemcpyAsync(hs + 1, binRecPos + nBinP, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
     if (!sync()) return ST_CUDA_ERROR;
-    nR = hs[0] + (nBinP > 0 ? hs[1] : 0);
+    nR = hs[0];
     if (nR >= (1ll << kLinkKeyShift)) return ST_OUT_OF_MEMORY;
     if (nR > recCap) {                              // the arrays were short: again, at the counted size
       recCap = nR;
       if (!take_records(recCap)) return ST_OUT_OF_MEMORY;
       cudaMemsetAsync(recTot, 0, sizeof(unsigned long long), s);
       launch_fused(false);
-      if (nBinP > 0)
-        { (prm.exact ? bin_pairs_kernel<1, 1> : bin_pairs_kernel<1, 0>)<<<blocks_for(nBinP), kThreads, 0, s>>>(
-              Lb, Lo, D, BS, nBinP, offP, LP, cellOff, cellList, prm.eps, nullptr, nullptr, binRecPos, nullptr, R,
-              recTot, recCap); note_launch(); }
+      launch_binned(s, false);
     }
   } else {
     exclusive_scan_i64(nrec64, recOff, K, tot + 5, stK, d_err, s);
@@ -4071,8 +4262,7 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
           chunkPair); note_launch(); }
     if (nBinP > 0)
       { (prm.exact ? bin_pairs_kernel<1, 1> : bin_pairs_kernel<1, 0>)<<<blocks_for(nBinP), kThreads, 0, sb>>>(
-          Lb, Lo, D, BS, nBinP, offP, LP, cellOff, cellList, prm.eps, nullptr, nullptr, binRecPos, recOff, R, nullptr,
-          INT64_MAX);
+          Lb, Lo, D, BS, nBinP, offP, LP, cellOff, cellList, prm.eps, nullptr, nullptr, binRecPos, recOff, R);
         note_launch(); }
     if (sb != s && nBigPairs > 0) {
       cudaEventRecord(bev[1], sb);
