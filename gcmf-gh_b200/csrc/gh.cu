@@ -909,7 +909,6 @@ struct RingSet {
     clb = reinterpret_cast<int8_t*>(b + 45 * n); cee = reinterpret_cast<int8_t*>(b + 46 * n);
     cfl = reinterpret_cast<uint8_t*>(b + 47 * n);
   }
-  __device__ __forceinline__ double2& xy(int64_t i) const { return cxy[i]; }
   __device__ __forceinline__ double& x(int64_t i) const { return cxy[i].x; }
   __device__ __forceinline__ double& y(int64_t i) const { return cxy[i].y; }
   __device__ __forceinline__ int32_t& nx(int64_t i) const { return cnx[i]; }
@@ -1704,29 +1703,30 @@ __device__ bool seq_trace(PairCtx& c) {
 // clean-up of one component (polyclip.h:791-807): drop the first vertex while it is
 // collinear with its ring neighbours, then one forward pass that removes every vertex
 // collinear with the last kept vertex and its original successor.  Reads n vertices at
-// src, writes the kept ones at dst (dst <= src, ascending); returns how many were kept.
-__device__ int seq_cleanup_component(const double* src, double* dst, int n, double eps) {
+// src and returns how many are kept; kWrite: writes them to dst (which may be src itself,
+// or anything before it).
+template <bool kWrite>
+__device__ int seq_cleanup_component(const double2* src, double2* dst, int n, double eps) {
   if (n == 0) return 0;
-  const double lx = src[2 * (n - 1)], ly = src[2 * (n - 1) + 1];
+  const double2 last = src[n - 1];
   int r = 0;
   while (r < n) {
-    int nxt = (r + 1 < n) ? r + 1 : r;    // a lone vertex is its own neighbour
-    double a = area2(lx, ly, src[2 * r], src[2 * r + 1], src[2 * nxt], src[2 * nxt + 1]);
+    const double2 v = src[r], nx = src[(r + 1 < n) ? r + 1 : r];
+    double a = area2(last.x, last.y, v.x, v.y, nx.x, nx.y);
     if (r == n - 1) a = 0.0;              // ring of the last vertex alone: A(v,v,v)
     if (fabs(a) < eps) ++r; else break;
   }
   if (r >= n) return 0;
-  double kx = src[2 * r], ky = src[2 * r + 1];
-  const double rx = kx, ry = ky;
+  double2 k = src[r];
+  const double2 first = k;
   int kept = 1;
-  dst[0] = kx; dst[1] = ky;
+  if (kWrite) dst[0] = k;
   for (int j = r + 1; j < n; ++j) {
-    double vx = src[2 * j], vy = src[2 * j + 1];
-    double nx = (j + 1 < n) ? src[2 * (j + 1)] : rx, ny = (j + 1 < n) ? src[2 * (j + 1) + 1] : ry;
-    if (fabs(area2(kx, ky, vx, vy, nx, ny)) < eps) continue;
-    dst[2 * kept] = vx; dst[2 * kept + 1] = vy;
+    const double2 v = src[j], nx = (j + 1 < n) ? src[j + 1] : first;
+    if (fabs(area2(k.x, k.y, v.x, v.y, nx.x, nx.y)) < eps) continue;
+    if (kWrite) dst[kept] = v;
     ++kept;
-    kx = vx; ky = vy;
+    k = v;
   }
   return kept;
 }
@@ -1737,7 +1737,8 @@ __device__ void seq_cleanup(PairCtx& c, int32_t* outNC, int64_t* outNV) {
   int nc = 0;
   for (int k = 0; k < O.nc; ++k) {
     const int n = O.csz[k];
-    int kept = seq_cleanup_component(O.xy + 2 * vin, O.xy + 2 * vout, n, c.eps_clean);
+    double2* xy = reinterpret_cast<double2*>(O.xy);
+    int kept = seq_cleanup_component<true>(xy + vin, xy + vout, n, c.eps_clean);
     vin += n;
     if (kept == 0) continue;
     O.csz[nc++] = kept;
@@ -1775,12 +1776,40 @@ __device__ __forceinline__ int wind(double P0x, double P0y, double P1x, double P
   return 0;
 }
 
+// How a piece of a ring changes the state of the entry/exit pass, (d, t) = (parity of the
+// chain ends met, parity of the status changes): d' = d ^ a, t' = t ^ b ^ (c & d), as bits
+// a | b << 1 | c << 2.  Pieces compose, so the pass is a scan over any split of the ring.
+__device__ __forceinline__ unsigned flow_then(unsigned f, unsigned g) {
+  const unsigned fa = f & 1u, gc = (g >> 2) & 1u;
+  return ((f ^ g) & 7u) ^ ((gc & fa) << 1);
+}
+__device__ __forceinline__ unsigned flow_of(int8_t label) {
+  return label == L_CROSSING ? 2u : label == L_DELAYED_BOUNCING ? 3u : label == L_DELAYED_CROSSING ? 5u : 0u;
+}
+__device__ __forceinline__ unsigned warp_flow_scan(unsigned x) {   // inclusive
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+    if ((int)lane_id() >= o) x = flow_then(y, x);
+  }
+  return x;
+}
+
 // ---- cooperative groups for the parallel labelling and tracing of one pair.  The same
 // code runs with a warp per pair (WarpGroup) or, for pairs with long rings, a whole block
-// per pair (BlockGroup); every member executes every group call (uniform control flow).
+// (BlockGroup) or the whole grid (GridGroup) per pair; every member executes every group
+// call (uniform control flow).  kItems: ring slots a member takes between two scans.
 struct WarpGroup {
   static constexpr bool kBlock = false;
+  static constexpr bool kGrid = false;
   static constexpr bool kSolo = false;
+  static constexpr int kItems = 4;
+  // exclusive scan of flows in member order, and their composition
+  __device__ __forceinline__ unsigned flow_excl(unsigned x, unsigned& total) const {
+    const unsigned v = warp_flow_scan(x), e = __shfl_up_sync(kFull, v, 1);
+    total = __shfl_sync(kFull, v, 31);
+    return lane_id() == 0 ? 0u : e;
+  }
   __device__ __forceinline__ int rank() const { return (int)lane_id(); }
   __device__ __forceinline__ int size() const { return 32; }
   __device__ __forceinline__ void sync() const { __syncwarp(); }
@@ -1816,7 +1845,10 @@ struct WarpGroup {
 
 // One thread per pair: every collective is the identity, nothing synchronises.
 struct SoloGroup {
+  static constexpr bool kGrid = false;
   static constexpr bool kSolo = true;
+  static constexpr int kItems = 1;
+  __device__ __forceinline__ unsigned flow_excl(unsigned x, unsigned& total) const { total = x; return 0u; }
   __device__ __forceinline__ int rank() const { return 0; }
   __device__ __forceinline__ int size() const { return 1; }
   __device__ __forceinline__ void sync() const {}
@@ -1840,7 +1872,9 @@ constexpr int kBlockListRounds = 8;   // elements per thread between two barrier
 constexpr int kBlockScratch = kBlockLabelWarps + 1 + (kBlockListRounds * kBlockLabelWarps + 2) / 2;
 struct BlockGroup {
   static constexpr bool kBlock = true;
+  static constexpr bool kGrid = false;
   static constexpr bool kSolo = false;
+  static constexpr int kItems = 16;
   long long* sm;        // kBlockScratch entries
   uint32_t* loops;      // shared memory for the trace's loop table
   int loopsCap;         // segments that fit
@@ -1889,44 +1923,197 @@ struct BlockGroup {
     total = (int)all;
     return (int)(before + x);
   }
+  __device__ __forceinline__ unsigned flow_excl(unsigned x, unsigned& total) const {
+    const unsigned v = warp_flow_scan(x), e = __shfl_up_sync(kFull, v, 1);
+    __syncthreads();
+    if (lane_id() == 31) sm[threadIdx.x >> 5] = v;
+    __syncthreads();
+    unsigned before = 0, all = 0;
+    const int me = (int)(threadIdx.x >> 5);
+    for (int w = 0; w < kBlockLabelWarps; ++w) { if (w == me) before = all; all = flow_then(all, (unsigned)sm[w]); }
+    total = all;
+    return flow_then(before, lane_id() == 0 ? 0u : e);
+  }
+  // One step of list(): the hits of this block's kBlockListRounds * kBlockLabelThreads elements
+  // from b on.  m: this thread's ballots, at[r]: hits of the step before round r of its warp.
+  template <class P>
+  __device__ __forceinline__ int list_step(int b, int n, P pred, unsigned* m, int*& at) const {
+    int* cnt = reinterpret_cast<int*>(sm + kBlockLabelWarps + 1);   // [round][warp], then the total
+    const int warp = (int)(threadIdx.x >> 5), lane = (int)lane_id();
+    constexpr int kCounts = kBlockListRounds * kBlockLabelWarps, kPer = kCounts / 32;
+#pragma unroll
+    for (int r = 0; r < kBlockListRounds; ++r) {
+      const int s = b + r * kBlockLabelThreads + (int)threadIdx.x;
+      m[r] = __ballot_sync(kFull, s < n && pred(s));
+    }
+    __syncthreads();
+    if (lane == 0) {
+#pragma unroll
+      for (int r = 0; r < kBlockListRounds; ++r) cnt[r * kBlockLabelWarps + warp] = __popc(m[r]);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      int v[kPer], t = 0;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) { v[j] = cnt[lane * kPer + j]; t += v[j]; }
+      const int incl = warp_incl_scan(t);
+      int run = incl - t;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) { cnt[lane * kPer + j] = run; run += v[j]; }
+      if (lane == 31) cnt[kCounts] = incl;
+    }
+    __syncthreads();
+    at = cnt + warp;
+    return cnt[kCounts];
+  }
   // As WarpGroup's: each thread takes kBlockListRounds elements per step, so that the
   // barriers and the scan of the warps' counts are paid once per 4,096 elements.
   template <class P, class F>
   __device__ __forceinline__ int list(int n, P pred, F f) const {
-    int* cnt = reinterpret_cast<int*>(sm + kBlockLabelWarps + 1);   // [round][warp], then the total
-    const int warp = (int)(threadIdx.x >> 5), lane = (int)lane_id();
-    constexpr int kCounts = kBlockListRounds * kBlockLabelWarps, kPer = kCounts / 32;
     int carry = 0;
     for (int b = 0; b < n; b += kBlockListRounds * kBlockLabelThreads) {
       unsigned m[kBlockListRounds];
+      int* at;
+      const int total = list_step(b, n, pred, m, at);
 #pragma unroll
       for (int r = 0; r < kBlockListRounds; ++r) {
         const int s = b + r * kBlockLabelThreads + (int)threadIdx.x;
-        m[r] = __ballot_sync(kFull, s < n && pred(s));
+        if (s < n) f(s, ((m[r] >> lane_id()) & 1u) != 0, carry + at[r * kBlockLabelWarps] + __popc(m[r] & lanemask_lt()));
       }
-      __syncthreads();
-      if (lane == 0) {
-#pragma unroll
-        for (int r = 0; r < kBlockListRounds; ++r) cnt[r * kBlockLabelWarps + warp] = __popc(m[r]);
+      carry += total;
+    }
+    return carry;
+  }
+};
+
+// The whole grid on one pair (a cooperative launch: all blocks are resident).  The blocks
+// meet at a counting barrier; its wait is bounded, and once one wait has given up (an error
+// is raised) every later barrier falls through, so the kernel ends.
+constexpr int kGridBlocksMax = 512;
+constexpr long long kGridWaitPolls = 1ll << 26;
+struct GridScratch {
+  unsigned arrive;
+  int dead;
+  unsigned long long slot[3];                            // reductions, in turn
+  unsigned long long blk[2][kGridBlocksMax];             // blocks' parts of a scan, in turn
+};
+
+struct GridGroup {
+  static constexpr bool kBlock = false;
+  static constexpr bool kGrid = true;
+  static constexpr bool kSolo = false;
+  static constexpr int kItems = 16;
+  BlockGroup blk;
+  GridScratch* gs;
+  int* err;
+  mutable unsigned epoch = 0, reds = 0, scans = 0;
+  __device__ __forceinline__ GridGroup(const BlockGroup& b, GridScratch* g, int* e) : blk(b), gs(g), err(e) {}
+  __device__ __forceinline__ int rank() const { return (int)(blockIdx.x * kBlockLabelThreads + threadIdx.x); }
+  __device__ __forceinline__ int size() const { return (int)(gridDim.x * kBlockLabelThreads); }
+  __device__ void sync() const {
+    ++epoch;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const unsigned target = epoch * gridDim.x;
+      __threadfence();
+      atomicAdd(&gs->arrive, 1u);
+      volatile GridScratch* v = gs;
+      for (long long polls = 0; (int)(v->arrive - target) < 0; ++polls) {
+        if (v->dead) break;
+        if (polls > kGridWaitPolls) { v->dead = 1; raise_error(err, DEV_TIMEOUT); break; }
       }
-      __syncthreads();
-      if (warp == 0) {
-        int v[kPer], t = 0;
+      __threadfence();
+    }
+    __syncthreads();
+  }
+  // combine one value per block: add(slot, value) by each block's first thread
+  template <class A>
+  __device__ __forceinline__ unsigned long long reduce(A add) const {
+    unsigned long long* s = &gs->slot[reds % 3];
+    if (rank() == 0) *reinterpret_cast<volatile unsigned long long*>(&gs->slot[(reds + 1) % 3]) = 0ull;
+    ++reds;
+    if (threadIdx.x == 0) add(s);
+    sync();
+    return *reinterpret_cast<volatile unsigned long long*>(s);
+  }
+  __device__ __forceinline__ bool any(bool v) const {
+    const int b = __syncthreads_or(v);
+    return reduce([&](unsigned long long* s) { if (b) atomicOr(s, 1ull); }) != 0;
+  }
+  __device__ __forceinline__ bool all(bool v) const { return !any(!v); }
+  __device__ __forceinline__ int sum(int v) const {
+    const int b = blk.sum(v);
+    return (int)reduce([&](unsigned long long* s) { if (b) atomicAdd(s, (unsigned long long)(long long)b); });
+  }
+  template <class T>
+  __device__ __forceinline__ T bcast0(T v) const {
+    static_assert(sizeof(T) <= sizeof(long long), "bcast0: scalar types only");
+    unsigned long long x = 0;
+    memcpy(&x, &v, sizeof(T));
+    x = reduce([&](unsigned long long* s) { if (blockIdx.x == 0) atomicExch(s, x); });
+    T r;
+    memcpy(&r, &x, sizeof(T));
+    return r;
+  }
+  __device__ __forceinline__ int first(bool hit) const {
+    const int f = blk.first(hit);
+    const unsigned long long top = 1ull << 40;
+    const unsigned long long m = reduce([&](unsigned long long* s) {
+      if (f >= 0) atomicMax(s, top - (unsigned long long)(blockIdx.x * kBlockLabelThreads + f));
+    });
+    return m ? (int)(top - m) : -1;
+  }
+  // parts of all blocks after a barrier: op folds them in block order; before: those of earlier blocks
+  template <class T, class O>
+  __device__ __forceinline__ T block_parts(T mine, T none, O op, T& before) const {
+    unsigned long long* parts = gs->blk[scans++ & 1];
+    if (threadIdx.x == 0) *reinterpret_cast<volatile unsigned long long*>(&parts[blockIdx.x]) = (unsigned long long)mine;
+    sync();
+    T all = none;
+    before = none;
+    for (unsigned b0 = 0; b0 < gridDim.x; b0 += 32) {    // every warp folds them by itself
+      const unsigned b = b0 + lane_id();
+      T v = b < gridDim.x ? (T)*reinterpret_cast<volatile unsigned long long*>(&parts[b]) : none;
 #pragma unroll
-        for (int j = 0; j < kPer; ++j) { v[j] = cnt[lane * kPer + j]; t += v[j]; }
-        const int incl = warp_incl_scan(t);
-        int run = incl - t;
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) { cnt[lane * kPer + j] = run; run += v[j]; }
-        if (lane == 31) cnt[kCounts] = incl;
+      for (int o = 1; o < 32; o <<= 1) {
+        const T u = __shfl_up_sync(kFull, v, o);
+        if ((int)lane_id() >= o) v = op(u, v);
       }
-      __syncthreads();
+      if (blockIdx.x > b0 && blockIdx.x <= b0 + 32) before = op(all, __shfl_sync(kFull, v, (int)(blockIdx.x - b0) - 1));
+      all = op(all, __shfl_sync(kFull, v, 31));
+    }
+    return all;
+  }
+  __device__ __forceinline__ int incl_scan(int v, int& total) const {
+    int mine, before;
+    const int x = blk.incl_scan(v, mine);
+    total = block_parts<int>(mine, 0, [](int a, int b) { return a + b; }, before);
+    return before + x;
+  }
+  __device__ __forceinline__ unsigned flow_excl(unsigned x, unsigned& total) const {
+    unsigned mine, before;
+    const unsigned e = blk.flow_excl(x, mine);
+    total = block_parts<unsigned>(mine, 0u, [](unsigned a, unsigned b) { return flow_then(a, b); }, before);
+    return flow_then(before, e);
+  }
+  template <class P, class F>
+  __device__ __forceinline__ int list(int n, P pred, F f) const {
+    constexpr int kStep = kBlockListRounds * kBlockLabelThreads;
+    int carry = 0;
+    for (int64_t b0 = 0; b0 < n; b0 += (int64_t)kStep * gridDim.x) {
+      const int b = (int)min(b0 + (int64_t)blockIdx.x * kStep, (int64_t)n);   // this block's elements
+      unsigned m[kBlockListRounds];
+      int* at;
+      int before;
+      const int mine = blk.list_step(b, n, pred, m, at);
+      const int total = block_parts<int>(mine, 0, [](int x, int y) { return x + y; }, before);
 #pragma unroll
       for (int r = 0; r < kBlockListRounds; ++r) {
         const int s = b + r * kBlockLabelThreads + (int)threadIdx.x;
-        if (s < n) f(s, ((m[r] >> lane) & 1u) != 0, carry + cnt[r * kBlockLabelWarps + warp] + __popc(m[r] & lanemask_lt()));
+        if (s < n)
+          f(s, ((m[r] >> lane_id()) & 1u) != 0, carry + before + at[r * kBlockLabelWarps] + __popc(m[r] & lanemask_lt()));
       }
-      carry += cnt[kCounts];
+      carry += total;
     }
     return carry;
   }
@@ -2085,10 +2272,11 @@ __device__ void grp_step35(const G& g, PairCtx& c) {
   if (c.ident[0] && c.ident[1]) grp_push_ring(g, c.O, c.R[0]);
 }
 
-// Entry/exit flags as a warp prefix scan over the ring from the start vertex: the status
-// at a vertex is the start status toggled once per earlier CROSSING, DELAYED_BOUNCING and
-// second-of-a-chain DELAYED_CROSSING; "first chain vertex" alternates over the DELAYED
-// vertices met (polyclip.h:582-653).
+// Entry/exit flags as a scan over the ring from the start vertex: the status at a vertex is
+// the start status toggled once per earlier CROSSING, DELAYED_BOUNCING and second-of-a-chain
+// DELAYED_CROSSING; "first chain vertex" alternates over the DELAYED vertices met
+// (polyclip.h:582-653).  Each member takes kItems consecutive slots per step and one scan
+// composes their effects (flow_then).
 template <int EX, class G>
 __device__ bool grp_step4(const G& g, PairCtx& c, int tempAfter[2], int tempSlot[2]) {
   for (int sd = 0; sd < 2; ++sd) {
@@ -2122,41 +2310,46 @@ __device__ bool grp_step4(const G& g, PairCtx& c, int tempAfter[2], int tempSlot
     // the Q pass tests against P's ring including P's temporary vertex
     int8_t st0 = (sd == 1 ? grp_point_in_ring<EX>(g, B, qx, qy, tempAfter[0], tempSlot[0])
                           : grp_point_in_ring<EX>(g, B, qx, qy, -1, -1)) ? E_EXIT : E_ENTRY;
-    int carryD = 0, carryT = 0;
+    unsigned d = 0, t = 0;                               // the state before this step's slots
     const int m = A.m;
-    for (int b = 0; b < m; b += g.size()) {
-      int j = b + g.rank();
-      int s = -1;
-      int8_t L = L_NONE;
-      bool inter = false;
-      if (j < m) {
-        s = V0 + 1 + j;
-        if (s >= m) s -= m;
-        inter = A.it(s);
-        L = inter ? A.lb(s) : L_NONE;
+    constexpr int kI = G::kItems;
+    for (int b = 0; b < m; b += g.size() * kI) {
+      const int j0 = b + g.rank() * kI;
+      auto slot = [&](int j) { const int s = V0 + 1 + j; return s >= m ? s - m : s; };
+      int8_t L[kI];
+      unsigned mine = 0, all;
+#pragma unroll
+      for (int i = 0; i < kI; ++i) {
+        L[i] = L_NONE;
+        if (j0 + i < m && A.it(slot(j0 + i))) L[i] = A.lb(slot(j0 + i));
       }
-      int d = inter && (L == L_DELAYED_CROSSING || L == L_DELAYED_BOUNCING);
-      int dTot, tTot;
-      int dIncl = g.incl_scan(d, dTot);
-      bool first = ((carryD + dIncl - d) & 1) == 0;
-      int t = inter && (L == L_CROSSING || L == L_DELAYED_BOUNCING || (L == L_DELAYED_CROSSING && !first));
-      int tIncl = g.incl_scan(t, tTot);
-      int8_t st = ((carryT + tIncl - t) & 1) ? toggled(st0) : st0;
-      if (inter) {
-        if (L == L_CROSSING) A.ee(s) = st;
-        else if (L == L_BOUNCING) { if ((st == E_EXIT) ^ c.uni) A.fl(s) |= 1; }
-        else if (L == L_DELAYED_CROSSING) {
+#pragma unroll
+      for (int i = 0; i < kI; ++i) mine = flow_then(mine, flow_of(L[i]));
+      const unsigned e = g.flow_excl(mine, all);
+      unsigned td = d ^ (e & 1u), tt = t ^ ((e >> 1) & 1u) ^ ((e >> 2) & d);
+#pragma unroll
+      for (int i = 0; i < kI; ++i) {
+        if (L[i] == L_NONE) continue;
+        const int s = slot(j0 + i);
+        const bool first = td == 0;
+        int8_t st = tt ? toggled(st0) : st0;
+        if (L[i] == L_CROSSING) A.ee(s) = st;
+        else if (L[i] == L_BOUNCING) { if ((st == E_EXIT) ^ c.uni) A.fl(s) |= 1; }
+        else if (L[i] == L_DELAYED_CROSSING) {
           A.ee(s) = st;
           if (first) { if ((st == E_EXIT) ^ c.uni) A.lb(s) = L_CROSSING; }
           else if ((st == E_ENTRY) ^ c.uni) A.lb(s) = L_CROSSING;
-        } else if (L == L_DELAYED_BOUNCING) {
+        } else if (L[i] == L_DELAYED_BOUNCING) {
           A.ee(s) = st;
           if (first) { if ((st == E_EXIT) ^ c.uni) A.fl(s) |= 2; }
           else if ((st == E_ENTRY) ^ c.uni) A.fl(s) |= 2;
         }
+        const unsigned f = flow_of(L[i]);
+        tt ^= ((f >> 1) & 1u) ^ ((f >> 2) & td);
+        td ^= f & 1u;
       }
-      carryD += dTot;
-      carryT += tTot;
+      t ^= ((all >> 1) & 1u) ^ ((all >> 2) & d);
+      d ^= all & 1u;
     }
     g.sync();
   }
@@ -2776,164 +2969,196 @@ __device__ bool grp_linearize(const G& g, PairCtx& c) {
   return true;
 }
 
-// Clean-up: a component where no vertex is collinear with its two ring neighbours keeps
-// every vertex (the sequential pass would remove nothing), so it is only moved into place;
-// any other component is cleaned by one lane with the sequential pass.
+// The clean-up of a long component by one warp: the lanes take consecutive parts of the
+// forward pass, each assuming that the vertex before its part is kept.  Where that was
+// wrong the part is gone over again from the vertex that was kept, until nothing changes
+// (lane 0's part is right from the start, so at most 32 times; parts agree after one
+// or two).  Returns how many vertices are kept; writes them to dst when it is given.
+__device__ int warp_cleanup_component(const double2* src, double2* dst, int n, double eps) {
+  const int lane = (int)lane_id();
+  auto area_is_small = [eps](double2 a, double2 b, double2 c) { return fabs(area2(a.x, a.y, b.x, b.y, c.x, c.y)) < eps; };
+  const double2 last = src[n - 1];
+  int r = 0;
+  while (r < n && (r == n - 1 ? 0.0 < eps : area_is_small(last, src[r], src[r + 1]))) ++r;
+  if (r >= n) return 0;
+  const int len = n - 1 - r, per = (len + 31) / 32;
+  const int a = r + 1 + min(lane * per, len), b = r + 1 + min((lane + 1) * per, len);
+  const double2 first = src[r];
+  // decisions of one part from a kept vertex on
+  auto pass = [&](int prev, double2* out, int& kept) {
+    kept = 0;
+    double2 k = src[prev];
+    for (int j = a; j < b; ++j) {
+      const double2 v = src[j], nx = j + 1 < n ? src[j + 1] : first;
+      if (area_is_small(k, v, nx)) continue;
+      if (out) out[kept] = v;
+      ++kept;
+      k = v;
+      prev = j;
+    }
+    return prev;                                         // the last kept vertex so far
+  };
+  int from = a - 1, kept = 0;                            // (a - 1 >= r)
+  int end = pass(from, nullptr, kept);
+  for (int round = 0; round < 32; ++round) {
+    int before = __shfl_up_sync(kFull, end, 1);
+    if (lane == 0) before = r;
+    const bool wrong = before != from;
+    if (!__any_sync(kFull, wrong)) break;
+    if (wrong) { from = before; end = pass(from, nullptr, kept); }
+  }
+  const int incl = warp_incl_scan(kept), total = __shfl_sync(kFull, incl, 31) + 1;
+  if (dst) {
+    if (lane == 0) dst[0] = first;
+    int again;
+    pass(from, dst + 1 + incl - kept, again);
+  }
+  return total;
+}
+
+// Clean-up (polyclip.h:791-807).  One-thread pairs take their components one after another
+// with the sequential pass.  Wider groups first count what each component keeps -- a warp
+// takes 32 components, short ones a lane each, long ones all lanes together -- and leave
+// the result in place when nothing is removed; else the kept vertices go, in order, to the
+// free part of the pair's output region behind the traced ones (*where: its offset there).
 template <class G>
-__device__ void grp_cleanup(const G& g, PairCtx& c, int32_t* outNC, int64_t* outNV) {
+__device__ void grp_cleanup(const G& g, PairCtx& c, int32_t* outNC, int64_t* outNV, int64_t* where) {
   OutRegion& O = c.O;
-  // Fast pass for pairs with many components: test every vertex of every component at
-  // once (short components one member each, long ones by the whole group).  When nothing
-  // is removable, the output stands as traced; otherwise (and for pairs with few
-  // components) the per-component pass below removes and compacts.
-  if (O.nc > 4) {
-    int32_t* start = &c.R[0].tn(0);      // the trace's scratch is free now
+  if constexpr (G::kSolo) {
+    double2* xy = reinterpret_cast<double2*>(O.xy);
+    int64_t vin = 0, vout = 0;
+    int kc = 0;
+    for (int k = 0; k < O.nc; ++k) {
+      const int n = O.csz[k];
+      double2* v = xy + vin;
+      bool any = n == 0;
+      double2 p = v[n > 0 ? n - 1 : 0], q = v[0];
+      for (int j = 0; j < n && !any; ++j) {
+        const double2 nx = v[j + 1 < n ? j + 1 : 0];
+        any = fabs(area2(p.x, p.y, q.x, q.y, nx.x, nx.y)) < c.eps_clean;
+        p = q;
+        q = nx;
+      }
+      int kept = n;
+      if (any) kept = seq_cleanup_component<true>(v, xy + vout, n, c.eps_clean);
+      else if (vout != vin) for (int j = 0; j < n; ++j) xy[vout + j] = v[j];
+      vin += n;
+      if (kept == 0) continue;
+      if (kc != k || any) O.csz[kc] = kept;
+      ++kc;
+      vout += kept;
+    }
+    *outNC = kc;
+    *outNV = vout;
+  } else {
+    constexpr int kShortComp = 32;
+    const int nc = O.nc, lane = (int)lane_id();
+    if (nc == 0 || 2 * O.nv > O.vcap) {                  // (the region has room for twice a well-formed trace)
+      if (g.rank() == 0) seq_cleanup(c, outNC, outNV);
+      g.sync();
+      return;
+    }
+    const double2* xy = reinterpret_cast<const double2*>(O.xy);
+    double2* out = reinterpret_cast<double2*>(O.xy) + O.nv;
+    int32_t* start = &c.R[0].tn(0);                      // the trace's scratch is free now
+    int32_t* keptA = &c.R[0].ls(0);
+    int32_t* dstA = &c.R[0].tl(0);
     int carry = 0;
-    for (int b = 0; b < O.nc; b += g.size()) {
+    for (int b = 0; b < nc; b += g.size()) {
       const int k = b + g.rank();
-      const int v = (k < O.nc) ? O.csz[k] : 0;
+      const int v = (k < nc) ? O.csz[k] : 0;
       int tot;
       const int incl = g.incl_scan(v, tot);
-      if (k < O.nc) start[k] = carry + incl - v;
+      if (k < nc) start[k] = carry + incl - v;
       carry += tot;
     }
     g.sync();
-    constexpr int kShortComp = 64;
-    bool any = false;
-    for (int k = g.rank(); k < O.nc; k += g.size()) {
-      const int n = O.csz[k];
-      if (n > kShortComp) continue;
-      const double* src = O.xy + 2 * (int64_t)start[k];
-      for (int j = 0; j < n && !any; ++j) {
-        int p = (j > 0) ? j - 1 : n - 1, q = (j + 1 < n) ? j + 1 : 0;
-        if (fabs(area2(src[2 * p], src[2 * p + 1], src[2 * j], src[2 * j + 1], src[2 * q], src[2 * q + 1])) <
-            c.eps_clean)
-          any = true;
-      }
-    }
-    for (int k = 0; k < O.nc; ++k) {
-      const int n = O.csz[k];
-      if (n <= kShortComp) continue;
-      const double* src = O.xy + 2 * (int64_t)start[k];
-      for (int j = g.rank(); j < n && !any; j += g.size()) {
-        int p = (j > 0) ? j - 1 : n - 1, q = (j + 1 < n) ? j + 1 : 0;
-        if (fabs(area2(src[2 * p], src[2 * p + 1], src[2 * j], src[2 * j + 1], src[2 * q], src[2 * q + 1])) <
-            c.eps_clean)
-          any = true;
-      }
-    }
-    if (!g.any(any)) {
-      if (g.rank() == 0) { *outNC = O.nc; *outNV = O.nv; }
-      return;
-    }
-    if constexpr (!G::kSolo) {
-      // Removal with many components: each member cleans whole components in place (a
-      // component's kept vertices move to the front of its own range), then the kept
-      // vertices are compacted, through ring P's coordinate column (free after the
-      // trace) when they fit there.  Per component this is the sequential pass.
-      int32_t* keptA = &c.R[0].ls(0);
-      int32_t* dstA = &c.R[0].tl(0);
-      for (int k = g.rank(); k < O.nc; k += g.size()) {
-        double* src = O.xy + 2 * (int64_t)start[k];
-        keptA[k] = seq_cleanup_component(src, src, O.csz[k], c.eps_clean);
-      }
-      g.sync();
-      long long total = 0;
-      for (int b = 0; b < O.nc; b += g.size()) {
-        const int k = b + g.rank();
-        const int v = (k < O.nc) ? keptA[k] : 0;
-        int tot;
-        const int incl = g.incl_scan(v, tot);
-        if (k < O.nc) dstA[k] = (int32_t)(total + incl - v);
-        total += tot;
-      }
-      g.sync();
-      if (total <= (long long)c.R[0].cap) {
-        double2* stage = &c.R[0].xy(0);
-        for (int k = g.rank(); k < O.nc; k += g.size()) {
-          const int kept = keptA[k];
-          const double* src = O.xy + 2 * (int64_t)start[k];
-          double2* dst = stage + dstA[k];
-          for (int j = 0; j < kept; ++j) dst[j] = make_double2(src[2 * j], src[2 * j + 1]);
+    bool removed = false;
+    for (int b = 0; b < nc; b += g.size()) {
+      const int k = b + g.rank();
+      const int n = k < nc ? O.csz[k] : 0, s0 = k < nc ? start[k] : 0;
+      int kept = n;
+      if (n > 0 && n <= kShortComp) {
+        const double2* v = xy + s0;
+        double2 p = v[n - 1], q = v[0];
+        bool any = false;
+        for (int j = 0; j < n; ++j) {
+          const double2 nx = v[j + 1 < n ? j + 1 : 0];
+          if (fabs(area2(p.x, p.y, q.x, q.y, nx.x, nx.y)) < c.eps_clean) { any = true; break; }
+          p = q;
+          q = nx;
         }
-        g.sync();
-        for (long long t = g.rank(); t < total; t += g.size()) {
-          const double2 v = stage[t];
-          O.xy[2 * t] = v.x;
-          O.xy[2 * t + 1] = v.y;
-        }
-      } else {
-        long long vout = 0;
-        for (int k = 0; k < O.nc; ++k) {
-          const int kept = keptA[k];
-          const double* src = O.xy + 2 * (int64_t)start[k];
-          double* dst = O.xy + 2 * vout;
-          if (kept > 0 && dst != src) {
-            for (int b = 0; b < 2 * kept; b += g.size()) {
-              const int i = b + g.rank();
-              const double v = (i < 2 * kept) ? src[i] : 0.0;
-              g.sync();
-              if (i < 2 * kept) dst[i] = v;
-            }
+        if (any) kept = seq_cleanup_component<false>(v, nullptr, n, c.eps_clean);
+      }
+      unsigned longs = __ballot_sync(kFull, n > kShortComp);
+      while (longs) {
+        const int src = __ffs(longs) - 1;
+        longs &= longs - 1;
+        const int ln = __shfl_sync(kFull, n, src);
+        const double2* v = xy + __shfl_sync(kFull, s0, src);
+        bool any = false;
+        for (int j0 = 0; j0 < ln && !any; j0 += 128) {
+          bool small = false;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int j = j0 + u * 32 + lane;
+            if (j >= ln) continue;
+            const double2 p = v[j > 0 ? j - 1 : ln - 1], q = v[j], nx = v[j + 1 < ln ? j + 1 : 0];
+            if (fabs(area2(p.x, p.y, q.x, q.y, nx.x, nx.y)) < c.eps_clean) small = true;
           }
-          g.sync();
-          vout += kept;
+          any = __any_sync(kFull, small) != 0;
         }
+        const int lk = any ? warp_cleanup_component(v, nullptr, ln, c.eps_clean) : ln;
+        if (lane == src) kept = lk;
       }
-      g.sync();
-      int cc = 0;
-      for (int b = 0; b < O.nc; b += g.size()) {
-        const int k = b + g.rank();
-        const int f = (k < O.nc && keptA[k] > 0) ? 1 : 0;
-        int tot;
-        const int incl = g.incl_scan(f, tot);
-        if (f) O.csz[cc + incl - 1] = keptA[k];
-        cc += tot;
+      if (k < nc) {
+        keptA[k] = kept;
+        if (kept != n) removed = true;
       }
-      if (g.rank() == 0) { *outNC = cc; *outNV = (int64_t)total; }
-      g.sync();
+    }
+    g.sync();
+    if (!g.any(removed)) {
+      if (g.rank() == 0) { *outNC = nc; *outNV = O.nv; }
       return;
     }
-  }
-  int64_t vin = 0, vout = 0;
-  int nc = 0;
-  for (int k = 0; k < O.nc; ++k) {
-    const int n = O.csz[k];
-    const double* src = O.xy + 2 * vin;
-    double* dst = O.xy + 2 * vout;
-    bool flag = false;
-    for (int j = g.rank(); j < n; j += g.size()) {
-      int p = (j > 0) ? j - 1 : n - 1, q = (j + 1 < n) ? j + 1 : 0;
-      if (fabs(area2(src[2 * p], src[2 * p + 1], src[2 * j], src[2 * j + 1], src[2 * q], src[2 * q + 1])) <
-          c.eps_clean)
-        flag = true;
+    int total = 0;
+    for (int b = 0; b < nc; b += g.size()) {
+      const int k = b + g.rank();
+      const int v = (k < nc) ? keptA[k] : 0;
+      int tot;
+      const int incl = g.incl_scan(v, tot);
+      if (k < nc) dstA[k] = total + incl - v;
+      total += tot;
     }
-    flag = g.any(flag);
-    int kept;
-    if (!flag) {
-      if (dst != src) {
-        for (int b = 0; b < 2 * n; b += g.size()) {
-          int i = b + g.rank();
-          double v = (i < 2 * n) ? src[i] : 0.0;
-          g.sync();
-          if (i < 2 * n) dst[i] = v;
-        }
+    g.sync();
+    for (int b = 0; b < nc; b += g.size()) {
+      const int k = b + g.rank();
+      const int n = k < nc ? O.csz[k] : 0, s0 = k < nc ? start[k] : 0, kept = k < nc ? keptA[k] : 0;
+      const int d0 = k < nc ? dstA[k] : 0;
+      if (n <= kShortComp && kept > 0) {
+        if (kept == n) for (int j = 0; j < n; ++j) out[d0 + j] = xy[s0 + j];
+        else seq_cleanup_component<true>(xy + s0, out + d0, n, c.eps_clean);
       }
-      kept = n;
-    } else {
-      kept = 0;
-      if (g.rank() == 0) kept = seq_cleanup_component(src, dst, n, c.eps_clean);
-      kept = g.bcast0(kept);
+      unsigned longs = __ballot_sync(kFull, n > kShortComp && kept > 0);
+      while (longs) {
+        const int src = __ffs(longs) - 1;
+        longs &= longs - 1;
+        const int ln = __shfl_sync(kFull, n, src), lk = __shfl_sync(kFull, kept, src);
+        const double2* v = xy + __shfl_sync(kFull, s0, src);
+        double2* d = out + __shfl_sync(kFull, d0, src);
+        if (lk == ln) for (int j = lane; j < ln; j += 32) d[j] = v[j];
+        else warp_cleanup_component(v, d, ln, c.eps_clean);
+      }
     }
     g.sync();
-    vin += n;
-    if (kept == 0) continue;
-    if (g.rank() == 0) O.csz[nc] = kept;
-    ++nc;
-    vout += kept;
+    // sizes of the components that are left
+    const int left = g.list(nc, [&](int k) { return keptA[k] > 0; },
+                            [&](int k, bool hit, int before) { if (hit) dstA[before] = keptA[k]; });
+    g.sync();
+    for (int k = g.rank(); k < left; k += g.size()) O.csz[k] = dstA[k];
+    if (g.rank() == 0) { *outNC = left; *outNV = total; *where += O.nv; }
     g.sync();
   }
-  if (g.rank() == 0) { *outNC = nc; *outNV = vout; }
 }
 
 // Pulls a pair's ring arrays into L1 in one burst, one request per 128-byte line, so the
@@ -2952,6 +3177,10 @@ __device__ void prefetch_ring(const G& g, const Ring& R) {
   }
 }
 
+// What the sequential phases of a pair start from: 1 the links, 2 the labels, 3 the flags
+// (rings of m slots, `used` with the added vertices; components and vertices already out).
+struct BigSeq { int from, mP, mQ, usedP, usedQ, nc; int64_t nv; };
+
 // Arguments of the labelling kernels (one struct so the warp and block kernels agree).
 struct LabelArgs {
   PairDev D;
@@ -2960,7 +3189,7 @@ struct LabelArgs {
   const int64_t* regP; const int64_t* regQ;
   const int64_t* regSizeP; const int64_t* regSizeQ;
   RingSet SP, SQ;
-  double* outXY; const int64_t* outVOff; const int64_t* outVCap;
+  double* outXY; int64_t* outVOff; const int64_t* outVCap;
   int32_t* outCsz; const int64_t* outCOff; const int32_t* outCCap;
   int32_t* outNC; int64_t* outNV;
   ClipParams prm;
@@ -2976,6 +3205,7 @@ struct LabelArgs {
   // the block kernel the *midCount entries after those.
   const uint32_t* order;
   int64_t nTile, nWarp;
+  BigSeq* seq = nullptr;      // grid kernel: set when a pair is left to the sequential phases
 };
 
 // One pair labelled and traced by group g.  The group phases give the sequential result
@@ -2998,20 +3228,22 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
   c.err = a.err;
   c.status = a.D.status + k;
   c.noInter[0] = c.noInter[1] = c.ident[0] = c.ident[1] = false;
-  prefetch_ring(g, c.R[0]);
-  prefetch_ring(g, c.R[1]);
-
-  if (!grp_links_one_to_one(g, c.R[0], c.R[1])) {
-    if (lead) seq_pair_from<EX>(c, 1, outNC, outNV);
-    g.sync();
-    return;
+  if constexpr (!G::kGrid) {
+    prefetch_ring(g, c.R[0]);
+    prefetch_ring(g, c.R[1]);
   }
+  // where the sequential phases take over; a grid leaves them to a kernel of one thread
+  auto sequential = [&](int from) {
+    if constexpr (G::kGrid) {
+      if (lead) *a.seq = BigSeq{from, c.R[0].m, c.R[1].m, c.R[0].used, c.R[1].used, c.O.nc, c.O.nv};
+    } else {
+      if (lead) seq_pair_from<EX>(c, from, outNC, outNV);
+    }
+    g.sync();
+  };
+  if (!grp_links_one_to_one(g, c.R[0], c.R[1])) { sequential(1); return; }
   grp_step1<EX>(g, c);
-  if (!grp_step2(g, c)) {
-    if (lead) seq_pair_from<EX>(c, 2, outNC, outNV);
-    g.sync();
-    return;
-  }
+  if (!grp_step2(g, c)) { sequential(2); return; }
   grp_step35<EX>(g, c);
   int tempAfter[2], tempSlot[2];
   if (!grp_step4<EX>(g, c, tempAfter, tempSlot)) return;
@@ -3037,6 +3269,7 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
   }
   if (added) {
     // vertices were added to a ring: trace through the next/prev links on one member
+    if constexpr (G::kGrid) { sequential(3); return; }
     int ok = 1;
     if (lead) ok = seq_trace(c) ? 1 : 0;
     ok = g.bcast0(ok);
@@ -3050,13 +3283,16 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
     if constexpr (G::kSolo) r = grp_trace_runs_slots(g, c);
     else r = grp_trace_loops(g, c);
     if (r < 0) return;
-    if (r > 0 && !grp_trace(g, c)) return;
+    if (r > 0) {
+      if constexpr (G::kGrid) { sequential(3); return; }
+      else if (!grp_trace(g, c)) return;
+    }
   }
   if (c.O.overflow) {
     if (lead) fail(c, DEV_CAPACITY);
     return;
   }
-  grp_cleanup(g, c, outNC, outNV);
+  grp_cleanup(g, c, outNC, outNV, a.outVOff + k);
 }
 
 // Two register budgets for the warp and one-thread kernels.  kWide (batches of at least
@@ -3111,7 +3347,8 @@ __global__ void unpermute_offsets_kernel(const uint32_t* __restrict__ order, int
 // Sort keys of the pairs by labelling class and size, for one 8-bit radix pass: one-thread
 // pairs 0..84, warp pairs 85..169, block pairs 170..254 (85 size buckets each, largest
 // first; the block class on a log scale, so that its largest pairs start first and do not
-// trail the stage), the rest 255.  Class counts: cnt[2] one-thread, cnt[3] warp, cnt[0] block.
+// trail the stage), the rest 255.  Class counts: cnt[2] one-thread, cnt[3] warp, cnt[0] block,
+// cnt[4] grid.
 __global__ void label_order_kernel(const int32_t* __restrict__ mP, const int32_t* __restrict__ mQ,
                                    const int32_t* __restrict__ status, int64_t K, int64_t tileMax, int64_t midMin,
                                    int64_t bigMin, uint64_t* __restrict__ key, uint32_t* __restrict__ val,
@@ -3134,6 +3371,8 @@ __global__ void label_order_kernel(const int32_t* __restrict__ mP, const int32_t
     const int b = (int)fmin(84.0, fmax(0.0, 85.0 * r));
     kk = 254 - (uint64_t)b;
     atomicAdd(cnt, 1ull);
+  } else if (status[k] == 0) {
+    atomicAdd(cnt + 4, 1ull);
   }
   key[k] = kk;
   val[k] = (uint32_t)k;
@@ -3163,490 +3402,10 @@ label_trace_block_kernel(LabelArgs a) {
 
 // ================================================================ grid path for huge pairs
 // Pairs whose merged rings exceed ClipParams::big_label_min slots are labelled and traced
-// by grid-wide kernels, one phase per launch over the pair's ring slots, with the
-// host reading the few per-pair flags between phases.  The phases give the sequential
-// result under the same conditions as the warp path; otherwise one thread runs the
-// sequential phases from the first one that could differ.
-struct BigPair {
-  int64_t k, regP, regQ, vOff, vCap, cOff;
-  int32_t mP, mQ, capP, capQ, cCap, pad;
-};
-
-struct BigFlags {
-  int bad;
-  int notNone[2];
-  int notAllOn[2];
-  int firstFree[2];
-  int firstMid[2];
-  int anySplit;
-  int pad;
-  unsigned long long wind;
-};
-
-__device__ __forceinline__ Ring big_ring(const RingSet& S, int64_t reg, int m, int cap, int used) {
-  Ring r = ring_of(S, reg, m, cap);
-  r.used = used;
-  return r;
-}
-
-// 0: P, 1: Q of one pair; slot s of ring A; its ring successor/predecessor before any
-// vertex is added
-__device__ __forceinline__ int nxt_slot(int s, int m) { return (s + 1 < m) ? s + 1 : 0; }
-__device__ __forceinline__ int prv_slot(int s, int m) { return (s > 0) ? s - 1 : m - 1; }
-
-__global__ void big_links_kernel(RingSet SP, RingSet SQ, BigPair bp, BigFlags* f) {
-  Ring P = big_ring(SP, bp.regP, bp.mP, bp.capP, bp.mP), Q = big_ring(SQ, bp.regQ, bp.mQ, bp.capQ, bp.mQ);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)P.m + Q.m;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    bool bad = false;
-    if (i < P.m) {
-      int s = (int)i;
-      if (P.it(s)) { int nb = P.nb(s); bad = nb < 0 || nb >= Q.m || Q.nb(nb) != s; }
-    } else {
-      int s = (int)(i - P.m);
-      if (Q.it(s)) { int nb = Q.nb(s); bad = nb < 0 || nb >= P.m || P.nb(nb) != s; }
-    }
-    if (bad) atomicOr(&f->bad, 1);
-  }
-}
-
-template <int EX>
-__global__ void big_step1_kernel(RingSet SP, RingSet SQ, BigPair bp) {
-  Ring P = big_ring(SP, bp.regP, bp.mP, bp.capP, bp.mP), Q = big_ring(SQ, bp.regQ, bp.mQ, bp.capQ, bp.mQ);
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < P.m; s += gridDim.x * blockDim.x) {
-    if (!P.it(s)) continue;
-    int nb = P.nb(s);
-    int pm = prv_slot(s, P.m), pp = nxt_slot(s, P.m);
-    int a = rel_position<EX>(P, Q, prv_slot(nb, Q.m), pm, s, pp);
-    int b = rel_position<EX>(P, Q, nxt_slot(nb, Q.m), pm, s, pp);
-    int8_t L = initial_label(a, b);
-    if (L != L_NONE) { P.lb(s) = L; Q.lb(nb) = L; }
-  }
-}
-
-// kMode 0: every chain must end at an ON_LEFT/ON_RIGHT intersection vertex; 1: resolve
-template <int kMode>
-__global__ void big_chain_kernel(RingSet SP, RingSet SQ, BigPair bp, BigFlags* f) {
-  Ring P = big_ring(SP, bp.regP, bp.mP, bp.capP, bp.mP), Q = big_ring(SQ, bp.regQ, bp.mQ, bp.capQ, bp.mQ);
-  const int m = P.m;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < m; s += gridDim.x * blockDim.x) {
-    int8_t l0 = P.lb(s);
-    if (!P.it(s) || (l0 != L_LEFT_ON && l0 != L_RIGHT_ON)) continue;
-    int I = nxt_slot(s, m), guard = m;
-    if (kMode == 0) {
-      while (P.lb(I) == L_ON_ON && --guard > 0) I = nxt_slot(I, m);
-      if ((P.lb(I) != L_ON_LEFT && P.lb(I) != L_ON_RIGHT) || !P.it(I)) atomicOr(&f->bad, 1);
-    } else {
-      int x = l0 == L_LEFT_ON ? R_LEFT : R_RIGHT;
-      Q.lb(P.nb(s)) = L_NONE;
-      while (P.lb(I) == L_ON_ON) {
-        P.lb(I) = L_NONE;
-        Q.lb(P.nb(I)) = L_NONE;
-        I = nxt_slot(I, m);
-      }
-      int y = P.lb(I) == L_ON_LEFT ? R_LEFT : R_RIGHT;
-      int8_t ct = (x != y) ? L_DELAYED_CROSSING : L_DELAYED_BOUNCING;
-      P.lb(s) = ct; P.lb(I) = ct;
-      Q.lb(P.nb(s)) = ct; Q.lb(P.nb(I)) = ct;
-    }
-  }
-}
-
-// special-case flags of both rings (polygon.h:453-512 on the rings before any insertion)
-__global__ void big_flags_kernel(RingSet SP, RingSet SQ, BigPair bp, int uni, BigFlags* f) {
-  Ring R[2] = {big_ring(SP, bp.regP, bp.mP, bp.capP, bp.mP), big_ring(SQ, bp.regQ, bp.mQ, bp.capQ, bp.mQ)};
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)R[0].m + R[1].m;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int sd = i < R[0].m ? 0 : 1;
-    int v = (int)(sd == 0 ? i : i - R[0].m);
-    const Ring& A = R[sd];
-    const Ring& B = R[1 - sd];
-    int8_t l = A.lb(v);
-    if (l != L_ON_ON) atomicOr(&f->notAllOn[sd], 1);
-    if (A.it(v)) {
-      if (l == L_CROSSING || l == L_DELAYED_CROSSING) atomicOr(&f->notNone[sd], 1);
-      if (uni && (l == L_BOUNCING || l == L_DELAYED_BOUNCING)) atomicOr(&f->notNone[sd], 1);
-    } else {
-      atomicMin(&f->firstFree[sd], v);
-    }
-    int nb = A.nb(v), nx = nxt_slot(v, A.m);
-    if (nb >= 0 && A.nb(nx) != prv_slot(nb, B.m) && A.nb(nx) != nxt_slot(nb, B.m)) atomicMin(&f->firstMid[sd], v);
-  }
-}
-
-// first midpoint-rule vertex of ring A against ring B through B's current links (B may
-// hold its temporary vertex)
-__global__ void big_first_mid_kernel(RingSet SA, RingSet SB, int64_t regA, int mA, int capA, int64_t regB, int mB,
-                                     int capB, int usedB, int* out) {
-  Ring A = big_ring(SA, regA, mA, capA, mA), B = big_ring(SB, regB, mB, capB, usedB);
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < A.m; v += gridDim.x * blockDim.x) {
-    int nb = A.nb(v), nx = nxt_slot(v, A.m);
-    if (nb >= 0 && A.nb(nx) != B.pv(nb) && A.nb(nx) != B.nx(nb)) atomicMin(out, v);
-  }
-}
-
-// winding parity test (polygon.h:427-448) of a point of ring A against ring B.
-// point: slot v of A (mode 0), midpoint of v and its successor (mode 1).
-// B's edges are (s, s+1); `after`/`T` splice a temporary vertex of B.
-__global__ void big_wind_kernel(RingSet SA, int64_t regA, int mA, int v, int mode, RingSet SB, int64_t regB, int mB,
-                                int after, int T, unsigned long long* wsum) {
-  const double2* a = &SA.xy(regA);
-  double Rx = a[v].x, Ry = a[v].y;
-  if (mode == 1) { int n = nxt_slot(v, mA); Rx = 0.5 * (a[v].x + a[n].x); Ry = 0.5 * (a[v].y + a[n].y); }
-  const double2* q = &SB.xy(regB);
-  long long w = 0;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < mB; s += gridDim.x * blockDim.x) {
-    int n = nxt_slot(s, mB);
-    if (s == after) {
-      w += wind(q[s].x, q[s].y, q[T].x, q[T].y, Rx, Ry, SB.exact);
-      w += wind(q[T].x, q[T].y, q[n].x, q[n].y, Rx, Ry, SB.exact);
-    } else {
-      w += wind(q[s].x, q[s].y, q[n].x, q[n].y, Rx, Ry, SB.exact);
-    }
-  }
-  w = warp_sum(w);
-  if (lane_id() == 0 && w) atomicAdd(wsum, (unsigned long long)w);
-}
-
-__global__ void big_copy_ring_kernel(RingSet S, int64_t reg, int m, double* __restrict__ oxy, int64_t at,
-                                     int32_t* __restrict__ csz, int comp) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < m; s += gridDim.x * blockDim.x) {
-    oxy[2 * (at + s)] = S.x(reg + s);
-    oxy[2 * (at + s) + 1] = S.y(reg + s);
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) csz[comp] = m;
-}
-
-__global__ void big_add_temp_kernel(RingSet S, int64_t reg, int m, int cap, int used, int v) {
-  Ring A = big_ring(S, reg, m, cap, used);
-  int n = A.nx(v);
-  int T = add_vertex(A, 0.5 * (A.x(v) + A.x(n)), 0.5 * (A.y(v) + A.y(n)));
-  if (T >= 0) insert_after(A, T, v);
-}
-
-// step 4 as scans over the ring rotated to start after V0 (see warp_step4)
-__global__ void big_d_kernel(RingSet S, int64_t reg, int m, int V0, int32_t* __restrict__ d) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-    int s = V0 + 1 + j;
-    if (s >= m) s -= m;
-    int8_t L = S.lb(reg + s);
-    d[j] = (S.it(reg + s) && (L == L_DELAYED_CROSSING || L == L_DELAYED_BOUNCING)) ? 1 : 0;
-  }
-}
-
-__global__ void big_t_kernel(RingSet S, int64_t reg, int m, int V0, const int64_t* __restrict__ dEx,
-                             int32_t* __restrict__ t) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-    int s = V0 + 1 + j;
-    if (s >= m) s -= m;
-    int8_t L = S.lb(reg + s);
-    bool first = (dEx[j] & 1) == 0;
-    t[j] = (S.it(reg + s) && (L == L_CROSSING || L == L_DELAYED_BOUNCING || (L == L_DELAYED_CROSSING && !first))) ? 1 : 0;
-  }
-}
-
-__global__ void big_apply4_kernel(RingSet S, int64_t reg, int m, int V0, const int64_t* __restrict__ dEx,
-                                  const int64_t* __restrict__ tEx, int8_t st0, int uni) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-    int s = V0 + 1 + j;
-    if (s >= m) s -= m;
-    const int64_t g = reg + s;
-    if (!S.it(g)) continue;
-    int8_t L = S.lb(g);
-    bool first = (dEx[j] & 1) == 0;
-    int8_t st = (tEx[j] & 1) ? toggled(st0) : st0;
-    if (L == L_CROSSING) S.ee(g) = st;
-    else if (L == L_BOUNCING) { if ((st == E_EXIT) ^ (uni != 0)) S.fl(g) |= 1; }
-    else if (L == L_DELAYED_CROSSING) {
-      S.ee(g) = st;
-      if (first) { if ((st == E_EXIT) ^ (uni != 0)) S.lb(g) = L_CROSSING; }
-      else if ((st == E_ENTRY) ^ (uni != 0)) S.lb(g) = L_CROSSING;
-    } else if (L == L_DELAYED_BOUNCING) {
-      S.ee(g) = st;
-      if (first) { if ((st == E_EXIT) ^ (uni != 0)) S.fl(g) |= 2; }
-      else if ((st == E_ENTRY) ^ (uni != 0)) S.fl(g) |= 2;
-    }
-  }
-}
-
-__global__ void big_split_any_kernel(RingSet SP, RingSet SQ, BigPair bp, BigFlags* f) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < bp.mP; s += gridDim.x * blockDim.x) {
-    if (!(SP.fl(bp.regP + s) & 1)) continue;
-    int nb = SP.nb(bp.regP + s);
-    if (nb >= 0 && (SQ.fl(bp.regQ + nb) & 1)) atomicOr(&f->anySplit, 1);
-  }
-}
-
-__global__ void big_step6_kernel(RingSet SP, RingSet SQ, BigPair bp) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < bp.mP; s += gridDim.x * blockDim.x) {
-    if (!(SP.fl(bp.regP + s) & 2)) continue;
-    int nb = SP.nb(bp.regP + s);
-    if (nb >= 0 && (SQ.fl(bp.regQ + nb) & 2)) { SP.lb(bp.regP + s) = L_CROSSING; SQ.lb(bp.regQ + nb) = L_CROSSING; }
-  }
-}
-
-// the sequential phases from step 5 (split pairs) or from the trace on, one thread
-template <int EX>
-__global__ void big_seq_tail_kernel(RingSet SP, RingSet SQ, BigPair bp, int usedP, int usedQ, int from_trace,
-                                    double* __restrict__ oxy, int32_t* __restrict__ ocsz, int64_t nv0, int nc0,
-                                    ClipParams prm, int* err, int32_t* status, int32_t* outNC, int64_t* outNV) {
-  PairCtx c;
-  c.R[0] = big_ring(SP, bp.regP, bp.mP, bp.capP, usedP);
-  c.R[1] = big_ring(SQ, bp.regQ, bp.mQ, bp.capQ, usedQ);
-  c.O.xy = oxy + 2 * bp.vOff; c.O.csz = ocsz + bp.cOff; c.O.vcap = bp.vCap; c.O.ccap = bp.cCap;
-  c.O.nv = nv0; c.O.nc = nc0; c.O.overflow = false;
-  c.uni = prm.union_mode != 0;
-  c.eps_clean = prm.eps_clean;
-  c.err = err;
-  c.status = status + bp.k;
-  if (!from_trace) {
-    if (!seq_step5<EX>(c)) return;
-    seq_step6(c);
-  }
-  if (!seq_trace(c)) return;
-  seq_cleanup(c, outNC + bp.k, outNV + bp.k);
-}
-
-// the whole pair sequentially from `step` (links not one-to-one, malformed chains)
-template <int EX>
-__global__ void big_seq_pair_kernel(RingSet SP, RingSet SQ, BigPair bp, int step, double* __restrict__ oxy,
-                                    int32_t* __restrict__ ocsz, ClipParams prm, int* err, int32_t* status,
-                                    int32_t* outNC, int64_t* outNV) {
-  PairCtx c;
-  c.R[0] = big_ring(SP, bp.regP, bp.mP, bp.capP, bp.mP);
-  c.R[1] = big_ring(SQ, bp.regQ, bp.mQ, bp.capQ, bp.mQ);
-  c.O.xy = oxy + 2 * bp.vOff; c.O.csz = ocsz + bp.cOff; c.O.vcap = bp.vCap; c.O.ccap = bp.cCap;
-  c.O.nv = 0; c.O.nc = 0; c.O.overflow = false;
-  c.uni = prm.union_mode != 0;
-  c.eps_clean = prm.eps_clean;
-  c.err = err;
-  c.status = status + bp.k;
-  c.noInter[0] = c.noInter[1] = c.ident[0] = c.ident[1] = false;
-  seq_pair_from<EX>(c, step, outNC + bp.k, outNV + bp.k);
-}
-
-// ---- parallel tracing.  With no added vertices, when every vertex carrying an entry/exit
-// flag is an unvisited CROSSING vertex and vice versa, flags alternate along each ring
-// and linked vertices carry opposite flags, a run from a flagged vertex V ends at the
-// next flagged vertex in its direction, W(V), and continues at the twin of W(V).  Runs
-// from ENTRY vertices form cycles (one per result component); the reference traces each
-// component from its smallest-slot flagged P vertex I, forwards if I starts a run of the
-// cycle, else (I ends one) along the reversed cycle.
-__global__ void big_labeled_kernel(RingSet S, int64_t reg, int m, uint8_t* __restrict__ lab, BigFlags* f) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < m; s += gridDim.x * blockDim.x) {
-    int8_t e = S.ee(reg + s);
-    bool flagged = (e == E_ENTRY || e == E_EXIT);
-    bool crossing = S.it(reg + s) && S.lb(reg + s) == L_CROSSING;
-    lab[s] = flagged ? 1 : 0;
-    if (flagged != crossing) atomicOr(&f->bad, 1);
-  }
-}
-
-__global__ void big_lab_list_kernel(const uint8_t* __restrict__ lab, const int64_t* __restrict__ idx, int m,
-                                    int32_t* __restrict__ list) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < m; s += gridDim.x * blockDim.x)
-    if (lab[s]) list[idx[s]] = s;
-}
-
-// per flagged vertex u (P: [0,nP), Q: [nP,nP+nQ)): checks, run stop, length, successor
-__global__ void big_runs_kernel(RingSet SP, RingSet SQ, BigPair bp, const int32_t* __restrict__ listP,
-                                const int32_t* __restrict__ listQ, const int64_t* __restrict__ idxP,
-                                const int64_t* __restrict__ idxQ, int nP, int nQ, int uni, int32_t* __restrict__ succ,
-                                int32_t* __restrict__ len, int32_t* __restrict__ stop, BigFlags* f) {
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < nP + nQ; u += gridDim.x * blockDim.x) {
-    const bool onP = u < nP;
-    const RingSet& A = onP ? SP : SQ;
-    const RingSet& B = onP ? SQ : SP;
-    const int64_t ra = onP ? bp.regP : bp.regQ, rb = onP ? bp.regQ : bp.regP;
-    const int m = onP ? bp.mP : bp.mQ;
-    const int n = onP ? nP : nQ;
-    const int i = onP ? u : u - nP;
-    const int32_t* list = onP ? listP : listQ;
-    const int s = list[i];
-    const int8_t e = A.ee(ra + s);
-    bool bad = n < 2;
-    int nxt = list[(i + 1 < n) ? i + 1 : 0];
-    if (A.ee(ra + nxt) == e) bad = true;                         // alternation
-    int nb = A.nb(ra + s);
-    if (nb < 0 || B.ee(rb + nb) != toggled(e)) bad = true;        // twin carries the opposite flag
-    const int8_t st = toggled(e);
-    const int dir = ((st == E_EXIT) ^ (uni != 0)) ? 1 : -1;
-    int W = list[(i + dir + n) % n];
-    int L = dir > 0 ? W - s : s - W;
-    if (L <= 0) L += m;
-    int nbW = A.nb(ra + W);
-    if (nbW < 0) bad = true;
-    int v = 0;
-    if (!bad) v = onP ? nP + (int)idxQ[nbW] : (int)idxP[nbW];
-    succ[u] = v;
-    len[u] = L;
-    stop[u] = W;
-    if (bad) atomicOr(&f->bad, 1);
-  }
-}
-
-// pointer jumping over ENTRY-start vertices: cycle minima of the P-start slots (a) and
-// of the P-stop slots (b)
-__global__ void big_cycle_min_kernel(const int32_t* __restrict__ J, const int32_t* __restrict__ a,
-                                     const int32_t* __restrict__ b, int32_t* __restrict__ J2, int32_t* __restrict__ a2,
-                                     int32_t* __restrict__ b2, const uint8_t* __restrict__ isE, int N) {
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < N; u += gridDim.x * blockDim.x) {
-    if (!isE[u]) continue;
-    int j = J[u];
-    a2[u] = min(a[u], a[j]);
-    b2[u] = min(b[u], b[j]);
-    J2[u] = J[j];
-  }
-}
-
-__global__ void big_cycle_init_kernel(RingSet SP, RingSet SQ, BigPair bp, const int32_t* __restrict__ listP,
-                                      const int32_t* __restrict__ listQ, int nP, int nQ, const int32_t* __restrict__ succ,
-                                      const int32_t* __restrict__ stop, int32_t* __restrict__ J, int32_t* __restrict__ a,
-                                      int32_t* __restrict__ b, uint8_t* __restrict__ isE) {
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < nP + nQ; u += gridDim.x * blockDim.x) {
-    const bool onP = u < nP;
-    const int s = onP ? listP[u] : listQ[u - nP];
-    const int8_t e = onP ? SP.ee(bp.regP + s) : SQ.ee(bp.regQ + s);
-    isE[u] = e == E_ENTRY ? 1 : 0;
-    J[u] = succ[u];
-    a[u] = onP ? s : INT_MAX;
-    b[u] = onP ? stop[u] : INT_MAX;
-  }
-}
-
-// per ENTRY vertex: the cycle's list-ranking start B and direction; list break
-__global__ void big_cycle_start_kernel(const int32_t* __restrict__ a, const int32_t* __restrict__ b,
-                                       const uint8_t* __restrict__ isE, const int64_t* __restrict__ idxP,
-                                       const int32_t* __restrict__ listP, int nP, int N, int dirE,
-                                       const int32_t* __restrict__ succ, const int32_t* __restrict__ len,
-                                       int32_t* __restrict__ Bst, uint8_t* __restrict__ rev, int32_t* __restrict__ nxt,
-                                       int64_t* __restrict__ sfx) {
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < N; u += gridDim.x * blockDim.x) {
-    if (!isE[u]) continue;
-    int B;
-    if (a[u] < b[u]) {
-      B = (int)idxP[a[u]];                       // I starts a run: forwards from I
-      rev[u] = 0;
-    } else {
-      int iI = (int)idxP[b[u]];                  // I ends the run of A
-      int iA = ((iI - dirE) % nP + nP) % nP;
-      B = succ[iA];
-      rev[u] = 1;
-    }
-    Bst[u] = B;
-    nxt[u] = (succ[u] == B) ? -1 : succ[u];
-    sfx[u] = len[u];
-  }
-}
-
-__global__ void big_rank_kernel(const int32_t* __restrict__ nxt, const int64_t* __restrict__ sfx,
-                                int32_t* __restrict__ nxt2, int64_t* __restrict__ sfx2, const uint8_t* __restrict__ isE,
-                                int N) {
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < N; u += gridDim.x * blockDim.x) {
-    if (!isE[u]) continue;
-    int j = nxt[u];
-    if (j >= 0) { sfx2[u] = sfx[u] + sfx[j]; nxt2[u] = nxt[j]; }
-    else { sfx2[u] = sfx[u]; nxt2[u] = -1; }
-  }
-}
-
-// one writer per cycle: its length at the slot of I (components in ascending I)
-__global__ void big_comp_len_kernel(const uint8_t* __restrict__ isE, const int32_t* __restrict__ Bst,
-                                    const int64_t* __restrict__ sfx, const int32_t* __restrict__ a,
-                                    const int32_t* __restrict__ b, int N, int64_t* __restrict__ compLen,
-                                    uint8_t* __restrict__ compFlag) {
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < N; u += gridDim.x * blockDim.x) {
-    if (!isE[u] || Bst[u] != u) continue;
-    int I = min(a[u], b[u]);
-    compLen[I] = sfx[u];
-    compFlag[I] = 1;
-  }
-}
-
-// warp per run: copies the run's vertices to their places in the component
-__global__ void big_write_kernel(RingSet SP, RingSet SQ, BigPair bp, const int32_t* __restrict__ listP,
-                                 const int32_t* __restrict__ listQ, int nP, int N, const uint8_t* __restrict__ isE,
-                                 const int32_t* __restrict__ len, const int32_t* __restrict__ Bst,
-                                 const uint8_t* __restrict__ rev, const int64_t* __restrict__ sfx,
-                                 const int32_t* __restrict__ a, const int32_t* __restrict__ b,
-                                 const int64_t* __restrict__ compBase, const int64_t* __restrict__ compIdx,
-                                 int64_t nv0, int nc0, int uni, double* __restrict__ oxy, int32_t* __restrict__ ocsz) {
-  const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= N || !isE[w]) return;
-  const int u = (int)w;
-  const bool onP = u < nP;
-  const RingSet& A = onP ? SP : SQ;
-  const int64_t ra = onP ? bp.regP : bp.regQ;
-  const int m = onP ? bp.mP : bp.mQ;
-  const int s = onP ? listP[u] : listQ[u - nP];
-  const int8_t st = toggled(A.ee(ra + s));
-  const int dir = ((st == E_EXIT) ^ (uni != 0)) ? 1 : -1;
-  const int I = min(a[u], b[u]);
-  const int64_t L = sfx[Bst[u]];
-  const int64_t off = L - sfx[u];
-  const int lu = len[u];
-  const bool r = rev[u];
-  const int64_t base = nv0 + compBase[I];
-  for (int j = lane_id(); j < lu; j += 32) {
-    int v = s + dir * (j + 1);
-    v = ((v % m) + m) % m;
-    int64_t f = off + j;
-    int64_t pos = r ? ((f < L - 1) ? L - 2 - f : L - 1) : f;
-    oxy[2 * (base + pos)] = A.x(ra + v);
-    oxy[2 * (base + pos) + 1] = A.y(ra + v);
-  }
-  if (lane_id() == 0 && Bst[u] == u) ocsz[bp.cOff + nc0 + compIdx[I]] = (int32_t)L;
-}
-
-// warp per component of the pair: clean-up in place (see warp_cleanup)
-__global__ void big_cleanup_kernel(double* __restrict__ xy, const int32_t* __restrict__ csz,
-                                   const int64_t* __restrict__ cstart, int nc, double eps, int32_t* __restrict__ kept) {
-  const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= nc) return;
-  const int n = csz[w];
-  double* src = xy + 2 * cstart[w];
-  bool flag = false;
-  for (int j = lane_id(); j < n; j += 32) {
-    int p = (j > 0) ? j - 1 : n - 1, q = (j + 1 < n) ? j + 1 : 0;
-    if (fabs(area2(src[2 * p], src[2 * p + 1], src[2 * j], src[2 * j + 1], src[2 * q], src[2 * q + 1])) < eps)
-      flag = true;
-  }
-  flag = __any_sync(kFull, flag);
-  if (lane_id() == 0) kept[w] = flag ? seq_cleanup_component(src, src, n, eps) : n;
-}
-
-__global__ void big_compact_kernel(const double* __restrict__ xy, const int64_t* __restrict__ cstart,
-                                   const int32_t* __restrict__ kept, const int64_t* __restrict__ kstart, int nc,
-                                   double* __restrict__ tmp) {
-  const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= nc) return;
-  const double* src = xy + 2 * cstart[w];
-  double* dst = tmp + 2 * kstart[w];
-  for (int i = lane_id(); i < 2 * kept[w]; i += 32) dst[i] = src[i];
-}
-
-__global__ void big_finish_kernel(const int32_t* __restrict__ kept, const int64_t* __restrict__ cidx, int nc,
-                                  int32_t* __restrict__ csz) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x)
-    if (kept[c] > 0) csz[cidx[c]] = kept[c];
-}
-
-__global__ void big_info_label_kernel(const int64_t* __restrict__ list, int n, const int64_t* __restrict__ regP,
-                                      const int64_t* __restrict__ regQ, const int32_t* __restrict__ mP,
-                                      const int32_t* __restrict__ mQ, const int64_t* __restrict__ regSizeP,
-                                      const int64_t* __restrict__ regSizeQ, const int64_t* __restrict__ vOff,
-                                      const int64_t* __restrict__ vCap, const int64_t* __restrict__ cOff,
-                                      const int32_t* __restrict__ cCap, BigPair* __restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int64_t k = list[i];
-  BigPair b;
-  b.k = k; b.regP = regP[k]; b.regQ = regQ[k]; b.vOff = vOff[k]; b.vCap = vCap[k]; b.cOff = cOff[k];
-  b.mP = mP[k]; b.mQ = mQ[k]; b.capP = (int32_t)regSizeP[k]; b.capQ = (int32_t)regSizeQ[k]; b.cCap = cCap[k];
-  b.pad = 0;
-  out[i] = b;
-}
-
+// by the whole GPU, one after another in one cooperative launch: the same phases with the
+// grid as the group.  A kernel per phase with host reads between them, the loops found by
+// pointer jumping over all runs, took 182 ms for the 400,000 x 200,000-vertex pair (5.8e7
+// slots, 2.9e7 crossings).
 __global__ void big_label_list_kernel(const int32_t* __restrict__ mP, const int32_t* __restrict__ mQ,
                                       const int32_t* __restrict__ status, int64_t K, int64_t minSlots,
                                       int64_t* __restrict__ list, unsigned long long* __restrict__ n) {
@@ -3655,282 +3414,39 @@ __global__ void big_label_list_kernel(const int32_t* __restrict__ mP, const int3
   if ((int64_t)mP[k] + mQ[k] > minSlots) list[atomicAdd(n, 1ull)] = k;
 }
 
-__global__ void big_kflag_kernel(const int32_t* __restrict__ kept, int nc, uint8_t* __restrict__ f) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) f[c] = kept[c] > 0;
+template <int EX>
+__global__ void __launch_bounds__(kBlockLabelThreads)
+label_trace_grid_kernel(LabelArgs a, const int64_t* __restrict__ list, int n, GridScratch* gs, BigSeq* seq) {
+  __shared__ long long sm[kBlockScratch];
+  const GridGroup g(BlockGroup{sm, nullptr, 0}, gs, a.err);
+  for (int i = 0; i < n; ++i) {
+    a.seq = seq + i;
+    label_trace_pair<EX>(g, a, list[i]);
+    g.sync();
+  }
 }
 
-__global__ void big_set_counts_kernel(int32_t* outNC, int64_t* outNV, int nc, int64_t nv) {
-  *outNC = nc;
-  *outNV = nv;
-}
-
-__global__ void big_fail_kernel(int32_t* status, int* err, int code) {
-  *status = 3;
-  raise_error(err, code);
-}
-
-// Host driver of the grid path for one huge pair.
-struct BigCtx {
-  Arena& A;
-  cudaStream_t s;
-  int64_t* hs;
-  int* d_err;
-  RingSet SP, SQ;
-  double* oxy;
-  int32_t* ocsz;
-  int32_t* status;
-  int32_t* outNC;
-  int64_t* outNV;
-  ClipParams prm;
-};
-
-static unsigned grid_for(int64_t n) {
-  int64_t b = (n + 255) / 256;
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, 148 * 32));
-}
-
-static int run_big_label_pair(BigCtx& c, const BigPair& bp, BigFlags* df) {
-  cudaStream_t s = c.s;
-  const bool uni = c.prm.union_mode != 0;
-  auto sync = [&]() { return cudaStreamSynchronize(s) == cudaSuccess; };
-  BigFlags h{};
-  h.firstFree[0] = h.firstMid[0] = bp.mP;
-  h.firstFree[1] = h.firstMid[1] = bp.mQ;
-  cudaMemcpyAsync(df, &h, sizeof(BigFlags), cudaMemcpyHostToDevice, s);
-  auto read_flags = [&]() {
-    cudaMemcpyAsync(&h, df, sizeof(BigFlags), cudaMemcpyDeviceToHost, s);
-    return sync();
-  };
-  auto seq_pair = [&](int step) {
-    { (c.prm.exact ? big_seq_pair_kernel<1> : big_seq_pair_kernel<0>)<<<1, 1, 0, s>>>(c.SP, c.SQ, bp, step, c.oxy, c.ocsz, c.prm, c.d_err, c.status, c.outNC,
-                                         c.outNV); note_launch(); }
-    return ST_OK;
-  };
-  const int64_t nAll = (int64_t)bp.mP + bp.mQ;
-  // ---- links one-to-one?
-  { big_links_kernel<<<grid_for(nAll), 256, 0, s>>>(c.SP, c.SQ, bp, df); note_launch(); }
-  if (!read_flags()) return ST_CUDA_ERROR;
-  if (h.bad) return seq_pair(1);
-  // ---- step 1, chains
-  { (c.prm.exact ? big_step1_kernel<1> : big_step1_kernel<0>)<<<grid_for(bp.mP), 256, 0, s>>>(c.SP, c.SQ, bp); note_launch(); }
-  { big_chain_kernel<0><<<grid_for(bp.mP), 256, 0, s>>>(c.SP, c.SQ, bp, df); note_launch(); }
-  if (!read_flags()) return ST_CUDA_ERROR;
-  if (h.bad) return seq_pair(2);
-  { big_chain_kernel<1><<<grid_for(bp.mP), 256, 0, s>>>(c.SP, c.SQ, bp, df); note_launch(); }
-  // ---- special cases (3.5)
-  { big_flags_kernel<<<grid_for(nAll), 256, 0, s>>>(c.SP, c.SQ, bp, uni ? 1 : 0, df); note_launch(); }
-  if (!read_flags()) return ST_CUDA_ERROR;
-  const int m[2] = {bp.mP, bp.mQ};
-  const int64_t reg[2] = {bp.regP, bp.regQ};
-  const int cap[2] = {bp.capP, bp.capQ};
-  const RingSet* S[2] = {&c.SP, &c.SQ};
-  bool noInter[2], ident[2];
-  for (int sd = 0; sd < 2; ++sd) {
-    noInter[sd] = !h.notNone[sd];
-    ident[sd] = noInter[sd] && !h.notAllOn[sd];
-  }
-  int64_t nv = 0;
-  int nc = 0;
-  unsigned long long* dwind = &df->wind;
-  auto winding = [&](int sa, int v, int mode, int sb, int after, int T, bool& inside) {
-    cudaMemsetAsync(dwind, 0, sizeof(unsigned long long), s);
-    { big_wind_kernel<<<grid_for(m[sb]), 256, 0, s>>>(*S[sa], reg[sa], m[sa], v, mode, *S[sb], reg[sb], m[sb], after, T,
-                                                      dwind); note_launch(); }
-    unsigned long long w = 0;
-    cudaMemcpyAsync(&w, dwind, sizeof(w), cudaMemcpyDeviceToHost, s);
-    if (!sync()) return false;
-    inside = ((long long)w % 2) != 0;
-    return true;
-  };
-  auto push_ring = [&](int sd) {
-    if (nv + m[sd] > bp.vCap || nc >= bp.cCap) return false;
-    { big_copy_ring_kernel<<<grid_for(m[sd]), 256, 0, s>>>(*S[sd], reg[sd], m[sd], c.oxy, bp.vOff + nv,
-                                                           c.ocsz + bp.cOff, nc); note_launch(); }
-    nv += m[sd];
-    ++nc;
-    return true;
-  };
-  auto fail = [&](int code) {
-    { big_fail_kernel<<<1, 1, 0, s>>>(c.status + bp.k, c.d_err, code); note_launch(); }
-    return ST_OK;
-  };
-  for (int sd = 0; sd < 2; ++sd) {
-    if (!noInter[sd] || ident[sd]) continue;
-    int v = -1, mode = 0;
-    if (h.firstFree[sd] < m[sd]) v = h.firstFree[sd];
-    else if (h.firstMid[sd] < m[sd]) { v = h.firstMid[sd]; mode = 1; }
-    if (v < 0) continue;
-    bool inside;
-    if (!winding(sd, v, mode, 1 - sd, -1, -1, inside)) return ST_CUDA_ERROR;
-    if (inside ^ uni)
-      if (!push_ring(sd)) return fail(DEV_CAPACITY);
-  }
-  if (ident[0] && ident[1])
-    if (!push_ring(0)) return fail(DEV_CAPACITY);
-  // ---- step 4 (entry/exit) as device scans over the rotated rings
-  int used[2] = {bp.mP, bp.mQ};
-  int tempAfter[2] = {-1, -1}, tempSlot[2] = {-1, -1};
-  {
-    const int mm = std::max(bp.mP, bp.mQ);
-    int32_t* d = c.A.take_n<int32_t>(mm);
-    int32_t* t = c.A.take_n<int32_t>(mm);
-    int64_t* dEx = c.A.take_n<int64_t>(mm);
-    int64_t* tEx = c.A.take_n<int64_t>(mm);
-    void* st = c.A.take(scan_temp_bytes(mm));
-    if (!d || !t || !dEx || !tEx || !st) return ST_OUT_OF_MEMORY;
-    for (int sd = 0; sd < 2; ++sd) {
-      if (noInter[sd]) continue;
-      int V0 = -1, qslot = -1;
-      if (h.firstFree[sd] < m[sd]) {
-        V0 = qslot = h.firstFree[sd];
-      } else {
-        int mid = h.firstMid[sd];
-        if (sd == 1 && tempSlot[0] >= 0) {        // against P's links including P's temporary vertex
-          int* dm = &df->firstMid[1];
-          cudaMemcpyAsync(dm, &m[1], sizeof(int), cudaMemcpyHostToDevice, s);
-          { big_first_mid_kernel<<<grid_for(m[1]), 256, 0, s>>>(c.SQ, c.SP, reg[1], m[1], cap[1], reg[0], m[0], cap[0],
-                                                                used[0], dm); note_launch(); }
-          if (!read_flags()) return ST_CUDA_ERROR;
-          mid = h.firstMid[1];
-        }
-        if (mid >= m[sd]) continue;
-        if (used[sd] >= cap[sd]) return fail(DEV_CAPACITY);
-        { big_add_temp_kernel<<<1, 1, 0, s>>>(*S[sd], reg[sd], m[sd], cap[sd], used[sd], mid); note_launch(); }
-        tempAfter[sd] = mid;
-        tempSlot[sd] = used[sd]++;
-        V0 = mid;
-        qslot = tempSlot[sd];
-      }
-      bool inside;
-      if (!winding(sd, qslot, 0, 1 - sd, sd == 1 ? tempAfter[0] : -1, sd == 1 ? tempSlot[0] : -1, inside))
-        return ST_CUDA_ERROR;
-      const int8_t st0 = inside ? E_EXIT : E_ENTRY;
-      { big_d_kernel<<<grid_for(m[sd]), 256, 0, s>>>(*S[sd], reg[sd], m[sd], V0, d); note_launch(); }
-      exclusive_scan_i32(d, dEx, m[sd], nullptr, st, c.d_err, s);
-      { big_t_kernel<<<grid_for(m[sd]), 256, 0, s>>>(*S[sd], reg[sd], m[sd], V0, dEx, t); note_launch(); }
-      exclusive_scan_i32(t, tEx, m[sd], nullptr, st, c.d_err, s);
-      { big_apply4_kernel<<<grid_for(m[sd]), 256, 0, s>>>(*S[sd], reg[sd], m[sd], V0, dEx, tEx, st0, uni ? 1 : 0); note_launch(); }
-    }
-  }
-  auto seq_tail = [&](int from_trace) {
-    { (c.prm.exact ? big_seq_tail_kernel<1> : big_seq_tail_kernel<0>)<<<1, 1, 0, s>>>(c.SP, c.SQ, bp, used[0], used[1], from_trace, c.oxy, c.ocsz, nv, nc, c.prm,
-                                          c.d_err, c.status, c.outNC, c.outNV); note_launch(); }
-    return ST_OK;
-  };
-  // ---- split pairs (sequential), crossing candidates
-  { big_split_any_kernel<<<grid_for(bp.mP), 256, 0, s>>>(c.SP, c.SQ, bp, df); note_launch(); }
-  if (!read_flags()) return ST_CUDA_ERROR;
-  if (h.anySplit) return seq_tail(0);
-  { big_step6_kernel<<<grid_for(bp.mP), 256, 0, s>>>(c.SP, c.SQ, bp); note_launch(); }
-  if (used[0] != bp.mP || used[1] != bp.mQ) return seq_tail(1);
-  // ---- parallel tracing
-  uint8_t* labP = c.A.take_n<uint8_t>(bp.mP);
-  uint8_t* labQ = c.A.take_n<uint8_t>(bp.mQ);
-  int64_t* idxP = c.A.take_n<int64_t>(bp.mP);
-  int64_t* idxQ = c.A.take_n<int64_t>(bp.mQ);
-  int64_t* tots = c.A.take_n<int64_t>(4);
-  void* st = c.A.take(scan_temp_bytes(std::max(bp.mP, bp.mQ)));
-  if (!labP || !labQ || !idxP || !idxQ || !tots || !st) return ST_OUT_OF_MEMORY;
-  { big_labeled_kernel<<<grid_for(bp.mP), 256, 0, s>>>(c.SP, bp.regP, bp.mP, labP, df); note_launch(); }
-  { big_labeled_kernel<<<grid_for(bp.mQ), 256, 0, s>>>(c.SQ, bp.regQ, bp.mQ, labQ, df); note_launch(); }
-  exclusive_scan_u8(labP, idxP, bp.mP, tots + 0, st, c.d_err, s);
-  exclusive_scan_u8(labQ, idxQ, bp.mQ, tots + 1, st, c.d_err, s);
-  cudaMemcpyAsync(c.hs, tots, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  if (!read_flags()) return ST_CUDA_ERROR;
-  if (h.bad) return seq_tail(1);
-  const int nP = (int)c.hs[0], nQ = (int)c.hs[1], N = nP + nQ;
-  int64_t TV = 0, TC = 0;
-  if (N > 0) {
-    int32_t* listP = c.A.take_n<int32_t>(nP);
-    int32_t* listQ = c.A.take_n<int32_t>(nQ);
-    int32_t* succ = c.A.take_n<int32_t>(N);
-    int32_t* len = c.A.take_n<int32_t>(N);
-    int32_t* stop = c.A.take_n<int32_t>(N);
-    int32_t* J[2] = {c.A.take_n<int32_t>(N), c.A.take_n<int32_t>(N)};
-    int32_t* a[2] = {c.A.take_n<int32_t>(N), c.A.take_n<int32_t>(N)};
-    int32_t* b[2] = {c.A.take_n<int32_t>(N), c.A.take_n<int32_t>(N)};
-    uint8_t* isE = c.A.take_n<uint8_t>(N);
-    int32_t* Bst = c.A.take_n<int32_t>(N);
-    uint8_t* rev = c.A.take_n<uint8_t>(N);
-    int32_t* nx[2] = {c.A.take_n<int32_t>(N), c.A.take_n<int32_t>(N)};
-    int64_t* sf[2] = {c.A.take_n<int64_t>(N), c.A.take_n<int64_t>(N)};
-    int64_t* compLen = c.A.take_n<int64_t>(bp.mP);
-    uint8_t* compFlag = c.A.take_n<uint8_t>(bp.mP);
-    int64_t* compBase = c.A.take_n<int64_t>(bp.mP);
-    int64_t* compIdx = c.A.take_n<int64_t>(bp.mP);
-    if (!listP || !listQ || !succ || !len || !stop || !J[0] || !J[1] || !a[0] || !a[1] || !b[0] || !b[1] || !isE ||
-        !Bst || !rev || !nx[0] || !nx[1] || !sf[0] || !sf[1] || !compLen || !compFlag || !compBase || !compIdx)
-      return ST_OUT_OF_MEMORY;
-    { big_lab_list_kernel<<<grid_for(bp.mP), 256, 0, s>>>(labP, idxP, bp.mP, listP); note_launch(); }
-    { big_lab_list_kernel<<<grid_for(bp.mQ), 256, 0, s>>>(labQ, idxQ, bp.mQ, listQ); note_launch(); }
-    { big_runs_kernel<<<grid_for(N), 256, 0, s>>>(c.SP, c.SQ, bp, listP, listQ, idxP, idxQ, nP, nQ, uni ? 1 : 0, succ,
-                                                  len, stop, df); note_launch(); }
-    if (!read_flags()) return ST_CUDA_ERROR;
-    if (h.bad) return seq_tail(1);
-    { big_cycle_init_kernel<<<grid_for(N), 256, 0, s>>>(c.SP, c.SQ, bp, listP, listQ, nP, nQ, succ, stop, J[0], a[0],
-                                                        b[0], isE); note_launch(); }
-    int rounds = 1;
-    while ((1ll << rounds) < (int64_t)N) ++rounds;
-    int cur = 0;
-    for (int r = 0; r <= rounds; ++r) {
-      { big_cycle_min_kernel<<<grid_for(N), 256, 0, s>>>(J[cur], a[cur], b[cur], J[1 - cur], a[1 - cur], b[1 - cur],
-                                                         isE, N); note_launch(); }
-      cur = 1 - cur;
-    }
-    const int dirE = uni ? -1 : 1;   // ENTRY vertices run forwards in intersection mode
-    { big_cycle_start_kernel<<<grid_for(N), 256, 0, s>>>(a[cur], b[cur], isE, idxP, listP, nP, N, dirE, succ, len, Bst,
-                                                         rev, nx[0], sf[0]); note_launch(); }
-    int rc = 0;
-    for (int r = 0; r <= rounds; ++r) {
-      { big_rank_kernel<<<grid_for(N), 256, 0, s>>>(nx[rc], sf[rc], nx[1 - rc], sf[1 - rc], isE, N); note_launch(); }
-      rc = 1 - rc;
-    }
-    cudaMemsetAsync(compLen, 0, bp.mP * sizeof(int64_t), s);
-    cudaMemsetAsync(compFlag, 0, bp.mP, s);
-    { big_comp_len_kernel<<<grid_for(N), 256, 0, s>>>(isE, Bst, sf[rc], a[cur], b[cur], N, compLen, compFlag); note_launch(); }
-    exclusive_scan_i64(compLen, compBase, bp.mP, tots + 2, st, c.d_err, s);
-    exclusive_scan_u8(compFlag, compIdx, bp.mP, tots + 3, st, c.d_err, s);
-    cudaMemcpyAsync(c.hs, tots + 2, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-    if (!sync()) return ST_CUDA_ERROR;
-    TV = c.hs[0];
-    TC = c.hs[1];
-    if (nv + TV > bp.vCap || nc + TC > bp.cCap) return fail(DEV_CAPACITY);
-    { big_write_kernel<<<(unsigned)(((int64_t)N * 32 + 255) / 256), 256, 0, s>>>(
-        c.SP, c.SQ, bp, listP, listQ, nP, N, isE, len, Bst, rev, sf[rc], a[cur], b[cur], compBase, compIdx, nv, nc,
-        uni ? 1 : 0, c.oxy + 2 * bp.vOff, c.ocsz); note_launch(); }
-  }
-  nv += TV;
-  nc += (int)TC;
-  // ---- clean-up of every component of the pair, then compaction
-  if (nc == 0) {
-    { big_set_counts_kernel<<<1, 1, 0, s>>>(c.outNC + bp.k, c.outNV + bp.k, 0, 0); note_launch(); }
-    return ST_OK;
-  }
-  int32_t* csz = c.ocsz + bp.cOff;
-  double* xy = c.oxy + 2 * bp.vOff;
-  int64_t* cstart = c.A.take_n<int64_t>(nc);
-  int32_t* kept = c.A.take_n<int32_t>(nc);
-  int64_t* kstart = c.A.take_n<int64_t>(nc);
-  uint8_t* kflag = c.A.take_n<uint8_t>(nc);
-  int64_t* cidx = c.A.take_n<int64_t>(nc);
-  double* tmp = c.A.take_n<double>(2 * nv);
-  void* st3 = c.A.take(scan_temp_bytes(nc));
-  if (!cstart || !kept || !kstart || !kflag || !cidx || !tmp || !st3) return ST_OUT_OF_MEMORY;
-  exclusive_scan_i32(csz, cstart, nc, nullptr, st3, c.d_err, s);
-  { big_cleanup_kernel<<<(unsigned)(((int64_t)nc * 32 + 255) / 256), 256, 0, s>>>(xy, csz, cstart, nc, c.prm.eps_clean,
-                                                                                  kept); note_launch(); }
-  exclusive_scan_i32(kept, kstart, nc, tots + 0, st3, c.d_err, s);
-  { big_kflag_kernel<<<grid_for(nc), 256, 0, s>>>(kept, nc, kflag); note_launch(); }
-  exclusive_scan_u8(kflag, cidx, nc, tots + 1, st3, c.d_err, s);
-  { big_compact_kernel<<<(unsigned)(((int64_t)nc * 32 + 255) / 256), 256, 0, s>>>(xy, cstart, kept, kstart, nc, tmp); note_launch(); }
-  cudaMemcpyAsync(c.hs, tots, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  if (!sync()) return ST_CUDA_ERROR;
-  const int64_t KV = c.hs[0];
-  const int KC = (int)c.hs[1];
-  cudaMemcpyAsync(xy, tmp, 2 * KV * sizeof(double), cudaMemcpyDeviceToDevice, s);
-  { big_finish_kernel<<<grid_for(nc), 256, 0, s>>>(kept, cidx, nc, csz); note_launch(); }
-  { big_set_counts_kernel<<<1, 1, 0, s>>>(c.outNC + bp.k, c.outNV + bp.k, KC, KV); note_launch(); }
-  return ST_OK;
+// the pairs that the grid left to the sequential phases, a thread each
+template <int EX>
+__global__ void big_seq_kernel(LabelArgs a, const int64_t* __restrict__ list, const BigSeq* __restrict__ seq) {
+  const BigSeq q = seq[blockIdx.x];
+  if (q.from == 0) return;
+  const int64_t k = list[blockIdx.x];
+  PairCtx c;
+  c.R[0] = ring_of(a.SP, a.regP[k], q.mP, (int)a.regSizeP[k]);
+  c.R[1] = ring_of(a.SQ, a.regQ[k], q.mQ, (int)a.regSizeQ[k]);
+  c.R[0].used = q.usedP;
+  c.R[1].used = q.usedQ;
+  c.O.xy = a.outXY + 2 * a.outVOff[k]; c.O.csz = a.outCsz + a.outCOff[k];
+  c.O.vcap = a.outVCap[k]; c.O.ccap = a.outCCap[k];
+  c.O.nv = q.nv; c.O.nc = q.nc; c.O.overflow = false;
+  c.uni = a.prm.union_mode != 0;
+  c.eps_clean = a.prm.eps_clean;
+  c.err = a.err;
+  c.status = a.D.status + k;
+  c.noInter[0] = c.noInter[1] = c.ident[0] = c.ident[1] = false;
+  if (q.from < 3) seq_pair_from<EX>(c, q.from, a.outNC + k, a.outNV + k);
+  else if (seq_trace(c)) seq_cleanup(c, a.outNC + k, a.outNV + k);
 }
 
 // ---------------------------------------------------------------- G8 compaction
@@ -4339,10 +3855,10 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   // the pairs labelled side by side have neighbouring regions.  The record export keeps
   // the regions in pair order.
   const int64_t midMin = std::min(prm.mid_label_min, prm.big_label_min);
-  unsigned long long* mcnt = A.take_n<unsigned long long>(4);
+  unsigned long long* mcnt = A.take_n<unsigned long long>(8);
   uint32_t* oval = A.take_n<uint32_t>(K);
   if (!mcnt || !oval) return ST_OUT_OF_MEMORY;
-  cudaMemsetAsync(mcnt, 0, 4 * sizeof(unsigned long long), s);
+  cudaMemsetAsync(mcnt, 0, 8 * sizeof(unsigned long long), s);
   if (!ex) {
     uint64_t* okey = A.take_n<uint64_t>(K);
     uint64_t* okeyAlt = A.take_n<uint64_t>(K);
@@ -4517,13 +4033,13 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   // with the ring layout; the counts are read with the output sizes
   cudaMemcpyAsync(hs, tot + 13, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
   cudaMemcpyAsync(hs + 2, mcnt, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(hs + 3, mcnt + 2, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(hs + 5, tot + 6, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  cudaMemcpyAsync(hs + 3, mcnt + 2, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  cudaMemcpyAsync(hs + 6, tot + 6, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
   if (!sync()) return ST_CUDA_ERROR;
-  C.n_ring_vertices = hs[5];
+  C.n_ring_vertices = hs[6];
   double* oxy = A.take_n<double>(2 * hs[0]);
   int32_t* ocsz = A.take_n<int32_t>(hs[1]);
-  const int64_t nMid = hs[2], nTile = hs[3], nWarp = hs[4];
+  const int64_t nMid = hs[2], nTile = hs[3], nWarp = hs[4], nGrid = hs[5];
   if (!oxy || !ocsz) return ST_OUT_OF_MEMORY;
   mk->mark("clip:fill+link", s);
   {
@@ -4584,32 +4100,27 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     }
     if (fork) cudaEventDestroy(fork);
     if (join) cudaEventDestroy(join);
-  }
-  // ---- G7 grid path for huge pairs
-  {
-    int64_t* blist = A.take_n<int64_t>(K);
-    unsigned long long* nbl = A.take_n<unsigned long long>(1);
-    BigFlags* dflags = A.take_n<BigFlags>(1);
-    if (!blist || !nbl || !dflags) return ST_OUT_OF_MEMORY;
-    cudaMemsetAsync(nbl, 0, sizeof(unsigned long long), s);
-    { big_label_list_kernel<<<blocks_for(K), kThreads, 0, s>>>(mP, mQ, D.status, K, prm.big_label_min, blist, nbl); note_launch(); }
-    cudaMemcpyAsync(hs, nbl, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-    if (!sync()) return ST_CUDA_ERROR;
-    const int nbig = (int)hs[0];
-    if (nbig > 0) {
-      BigPair* dbp = A.take_n<BigPair>(nbig);
-      if (!dbp) return ST_OUT_OF_MEMORY;
-      { big_info_label_kernel<<<blocks_for(nbig), kThreads, 0, s>>>(blist, nbig, regP, regQ, mP, mQ, regSizeP, regSizeQ,
-                                                                    vOff, vcap, cOff, ccap, dbp); note_launch(); }
-      std::vector<BigPair> hbp(nbig);
-      cudaMemcpyAsync(hbp.data(), dbp, nbig * sizeof(BigPair), cudaMemcpyDeviceToHost, s);
-      if (!sync()) return ST_CUDA_ERROR;
-      std::sort(hbp.begin(), hbp.end(), [](const BigPair& x, const BigPair& y) { return x.k < y.k; });
-      BigCtx bc{A, s, hs, d_err, SP, SQ, oxy, ocsz, D.status, nc, nv, prm};
-      for (const BigPair& bp : hbp) {
-        int st = run_big_label_pair(bc, bp, dflags);
-        if (st != ST_OK) return st;
-      }
+    // huge pairs: the grid path
+    if (nGrid > 0) {
+      int64_t* blist = A.take_n<int64_t>(K);
+      unsigned long long* nbl = A.take_n<unsigned long long>(1);
+      GridScratch* gs = A.take_n<GridScratch>(1);
+      BigSeq* seq = A.take_n<BigSeq>(nGrid);
+      if (!blist || !nbl || !gs || !seq) return ST_OUT_OF_MEMORY;
+      cudaMemsetAsync(nbl, 0, sizeof(unsigned long long), s);
+      cudaMemsetAsync(gs, 0, sizeof(GridScratch), s);
+      cudaMemsetAsync(seq, 0, nGrid * sizeof(BigSeq), s);
+      { big_label_list_kernel<<<blocks_for(K), kThreads, 0, s>>>(mP, mQ, D.status, K, prm.big_label_min, blist, nbl); note_launch(); }
+      const void* kern = prm.exact ? (const void*)label_trace_grid_kernel<1> : (const void*)label_trace_grid_kernel<0>;
+      int per = 0, n = (int)nGrid;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kBlockLabelThreads, 0) != cudaSuccess || per < 1)
+        return ST_CUDA_ERROR;
+      void* args[] = {&la, &blist, &n, &gs, &seq};
+      if (cudaLaunchCooperativeKernel(kern, dim3((unsigned)std::min(per * nsm, kGridBlocksMax)), dim3(kBlockLabelThreads),
+                                      args, 0, s) != cudaSuccess)
+        return ST_CUDA_ERROR;
+      note_launch();
+      { (prm.exact ? big_seq_kernel<1> : big_seq_kernel<0>)<<<(unsigned)nGrid, 1, 0, s>>>(la, blist, seq); note_launch(); }
     }
   }
   mk->mark("clip:label+trace", s);
