@@ -215,6 +215,7 @@ ClipParams clip_params(const gcmfgh_ctx* c, const gcmfgh_layer* b, const gcmfgh_
   if (!c->tuning_explicit) {
     const TuneRecord* t = find_tuning(c, floor_log2((double)std::max<int64_t>(n, 1)), mean_verts_log2(b, o), p.exact);
     if (t) apply_tuning(p, *t);
+    else p.tile_label_max = default_tile_label(n);
   }
   return p;
 }

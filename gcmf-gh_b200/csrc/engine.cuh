@@ -105,6 +105,15 @@ struct ClipParams {
   int64_t rec_hint = 0;                // records expected (the last clip's count; 0 unknown)
 };
 
+// The one-thread labelling's limit for a clip of n pairs when no threshold is set.  A thread
+// takes as long as its pair's slots (0.35 ms at 96), which only a batch that fills the GPU
+// with threads hides; below that a warp per pair is faster.  Label + trace with limits 96 /
+// 32 / 0: 0.38 / 0.11 / 0.04 ms at 1,300 pairs, 0.63 / 0.44 / 0.33 at 20,000 (exact),
+// 0.68 / 0.37 / 0.52 at 56,000, 1.38 / 1.52 / 3.40 at 470,000.
+inline int64_t default_tile_label(int64_t n_pairs) {
+  return n_pairs < (1ll << 15) ? 0 : n_pairs < (1ll << 16) ? 32 : 96;
+}
+
 // Clip outputs (device, owned by the clip arena).
 struct ClipDev {
   int64_t n_pairs = 0, n_components = 0, n_vertices = 0;

@@ -136,7 +136,8 @@ const char* gcmfgh_status_string(gcmfgh_status s);
 #define GCMFGH_TUNE_BIG_LABEL 1
 #define GCMFGH_TUNE_MID_LABEL 2
 /* GCMFGH_TUNE_TILE_LABEL: a pair whose merged rings have at most this many vertices is
- * labelled and traced by one thread, 32 pairs per warp (default 96; 0: never) */
+ * labelled and traced by one thread, 32 pairs per warp (0: never; default 96 in batches of
+ * at least 2^16 pairs, 32 from 2^15 pairs, 0 in smaller ones) */
 #define GCMFGH_TUNE_TILE_LABEL 3
 /* GCMFGH_TUNE_WIDE_LABEL: clip batches of at least this many pairs are labelled by the
  * kernels built for a full GPU (fewer registers, more resident warps); smaller batches
