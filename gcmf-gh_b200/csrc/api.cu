@@ -227,6 +227,7 @@ JoinEdges join_edges(const gcmfgh_ctx* c) {
   if (!J.clip_cand || !J.bOff) return e;
   e.cand = J.clip_cand; e.flag = J.join_flag; e.bE = J.bE; e.oE = J.oE;
   e.bOff = J.bOff; e.oOff = J.oOff; e.bList = J.bList; e.oList = J.oList;
+  e.max_ring = J.max_ring;
   return e;
 }
 

@@ -408,6 +408,56 @@ GCMFGH_DEV T warp_incl_scan(T v) {
   return v;
 }
 
+// A whole block's ordered list: f(i, hits before i) for every i in [0, n) that pred accepts;
+// returns the number of hits.  Each thread takes kRounds elements between two barriers.
+// cnt: shared, kRounds * (kBlock / 32) + 1 entries.
+template <int kBlock, int kRounds, class P, class F>
+GCMFGH_DEV int block_list(int n, int* cnt, P pred, F f) {
+  constexpr int kWarps = kBlock / 32, kCounts = kRounds * kWarps, kPer = kCounts / 32;
+  static_assert(kCounts % 32 == 0, "one warp scans the counts");
+  const int warp = (int)(threadIdx.x >> 5), lane = (int)lane_id();
+  int carry = 0;
+  for (int b = 0; b < n; b += kRounds * kBlock) {
+    unsigned m[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int i = b + r * kBlock + (int)threadIdx.x;
+      m[r] = __ballot_sync(0xffffffffu, i < n && pred(i));
+    }
+    __syncthreads();
+    if (lane == 0) {
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r) cnt[r * kWarps + warp] = __popc(m[r]);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      int v[kPer], t = 0;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) { v[j] = cnt[lane * kPer + j]; t += v[j]; }
+      const int incl = warp_incl_scan(t);
+      int run = incl - t;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) { cnt[lane * kPer + j] = run; run += v[j]; }
+      if (lane == 31) cnt[kCounts] = incl;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int i = b + r * kBlock + (int)threadIdx.x;
+      if ((m[r] >> lane) & 1u) f(i, carry + cnt[r * kWarps + warp] + __popc(m[r] & lanemask_lt()));
+    }
+    carry += cnt[kCounts];
+  }
+  return carry;
+}
+
+// Pairs that a pass leaves to its block-per-pair kernel (ids == nullptr: none are left).
+struct LongPairs {
+  int32_t* ids = nullptr;
+  unsigned* n = nullptr;
+  GCMFGH_DEV void add(int64_t k) const { ids[atomicAdd(n, 1u)] = (int32_t)k; }
+};
+
 // largest i in [0,n) with a[i] <= x (a sorted ascending, a[0] <= x)
 template <class T>
 GCMFGH_DEV int64_t upper_index(const T* a, int64_t n, T x) {

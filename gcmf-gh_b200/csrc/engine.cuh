@@ -73,6 +73,7 @@ struct JoinDev {
   int32_t* bList = nullptr;      // edges of the common-MBR filter (join_flag pairs), ascending
   int32_t* oList = nullptr;
   int64_t n_blist = 0, n_olist = 0;   // list entries (the next join's capacity hints)
+  int64_t max_ring = INT32_MAX;       // stored vertices of the largest base and overlay polygon together (bound)
 };
 
 // The join's common-MBR edge lists seen from its clip set (gh_clip_joined): the clip's
@@ -86,7 +87,13 @@ struct JoinEdges {
   const int64_t* oOff = nullptr;
   const int32_t* bList = nullptr;
   const int32_t* oList = nullptr;
+  int64_t max_ring = INT32_MAX;    // bound on the stored vertices of a pair's two rings
 };
+
+// Pairs with more stored vertices than this are left to block-per-pair kernels in the
+// stages that otherwise take a warp per pair: one polygon of 100,000 vertices kept a warp
+// busy for 1.5 ms per pass over it (MBR 1.7 ms, edge filters 2.9 ms, whole stages 0.3).
+constexpr int64_t kLongRing = 2048;
 
 // Clip parameters (reference defaults: EPSILON 1e-7 in GH-CUDA/lib/constants.h:4).
 struct ClipParams {
@@ -156,7 +163,8 @@ int run_join(const LayerDev& base, const LayerDev& ovl, Arena& arena, JoinDev& o
 int join_from_keys(const LayerDev& Lb, const LayerDev& Lo, const uint64_t* pkeys, int64_t K, int obits,
                    Arena& A, JoinDev& J, int64_t* d_total, unsigned long long* d_cnt, int* d_err,
                    int64_t* h_scratch, cudaStream_t s, Marks* marks = nullptr,
-                   cudaStream_t aux = nullptr, int64_t hintB = 0, int64_t hintO = 0, bool twoPass = false);
+                   cudaStream_t aux = nullptr, int64_t hintB = 0, int64_t hintO = 0, bool twoPass = false,
+                   int64_t maxB = INT32_MAX, int64_t maxO = INT32_MAX);
 
 // Merged rings of pair 0 after the neighbour links, as the reference's
 // calculateIntersections hands them back (gppolyclip_mDIV512.cu:1298-1640): vertices in

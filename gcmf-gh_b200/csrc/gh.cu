@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 #include "common.cuh"
 #include "engine.cuh"
@@ -119,12 +120,38 @@ __device__ __forceinline__ bool ring_closed(const double2* v, int n) {
   return a.x == b.x && a.y == b.y;
 }
 
+// member `me` of `of` takes its part of a pair's lists from the join; false: the join has none
+template <int kMode>
+__device__ __forceinline__ bool join_lists(const LayerDev& Lb, const LayerDev& Lo, const PairDev& D, int64_t w, int pside,
+                                           const JoinEdges& je, int32_t* cP, int32_t* cQ, const int64_t* offP,
+                                           const int64_t* offQ, int32_t* LP, int32_t* LQ, int me, int of) {
+  if (!je.cand) return false;
+  const int64_t cd = je.cand[w];
+  if (!je.flag[cd] || !ring_closed(layer_xy(Lb, Lo, pside) + D.pS[w], D.nP[w]) ||
+      !ring_closed(layer_xy(Lb, Lo, 1 - pside) + D.qS[w], D.nQ[w]))
+    return false;
+  for (int side = 0; side < 2; ++side) {
+    const bool base = (side == 0 ? pside : 1 - pside) == 0;
+    const int n = side == 0 ? D.nP[w] : D.nQ[w];
+    const int E = (base ? je.bE : je.oE)[cd];
+    const int32_t* src = base ? je.bList + je.bOff[cd] : je.oList + je.oOff[cd];
+    const int cnt = E - ((E > 0 && src[E - 1] == n) ? 1 : 0);
+    if (kMode == 0) {
+      if (me == 0) (side == 0 ? cP : cQ)[w] = cnt;
+    } else {
+      int32_t* dst = side == 0 ? LP + offP[w] : LQ + offQ[w];
+      for (int j = me; j < cnt; j += of) dst[j] = src[j];
+    }
+  }
+  return true;
+}
+
 template <int kMode, int W>
 __global__ void __launch_bounds__(kThreads, 6)
 edge_filter_kernel(LayerDev Lb, LayerDev Lo, PairDev D, int64_t K, int32_t* __restrict__ cP,
                    int32_t* __restrict__ cQ, const int64_t* __restrict__ offP,
                    const int64_t* __restrict__ offQ, int32_t* __restrict__ LP, int32_t* __restrict__ LQ,
-                   int64_t lo, int64_t hi, JoinEdges je) {
+                   int64_t lo, int64_t hi, JoinEdges je, LongPairs longs) {
   constexpr unsigned kBits = (W == 32) ? 0xffffffffu : ((1u << (W & 31)) - 1u);
   const int64_t w = ((int64_t)blockIdx.x * kThreads + threadIdx.x) / W;
   const int tl = (int)(threadIdx.x & (W - 1));
@@ -134,29 +161,13 @@ edge_filter_kernel(LayerDev Lb, LayerDev Lo, PairDev D, int64_t K, int32_t* __re
   if (D.status[w] != 0) { if (kMode == 0 && W != 32 && tl == 0) { cP[w] = 0; cQ[w] = 0; } return; }
   {
     const int64_t size = (int64_t)D.nP[w] + D.nQ[w];
-    if (size <= lo || size > hi) return;             // the other pass takes this pair
-  }
-  const int pside = D.pSide[w];
-  if (je.cand) {
-    const int64_t cd = je.cand[w];
-    if (je.flag[cd] && ring_closed(layer_xy(Lb, Lo, pside) + D.pS[w], D.nP[w]) &&
-        ring_closed(layer_xy(Lb, Lo, 1 - pside) + D.qS[w], D.nQ[w])) {
-      for (int side = 0; side < 2; ++side) {
-        const bool base = (side == 0 ? pside : 1 - pside) == 0;
-        const int n = side == 0 ? D.nP[w] : D.nQ[w];
-        const int E = (base ? je.bE : je.oE)[cd];
-        const int32_t* src = base ? je.bList + je.bOff[cd] : je.oList + je.oOff[cd];
-        const int cnt = E - ((E > 0 && src[E - 1] == n) ? 1 : 0);
-        if (kMode == 0) {
-          if (tl == 0) (side == 0 ? cP : cQ)[w] = cnt;
-        } else {
-          int32_t* dst = side == 0 ? LP + offP[w] : LQ + offQ[w];
-          for (int j = tl; j < cnt; j += W) dst[j] = src[j];
-        }
-      }
+    if (size <= lo || size > hi) {                   // another pass takes this pair
+      if (kMode == 0 && W == 32 && size > hi && longs.ids && tl == 0) longs.add(w);
       return;
     }
   }
+  const int pside = D.pSide[w];
+  if (join_lists<kMode>(Lb, Lo, D, w, pside, je, cP, cQ, offP, offQ, LP, LQ, tl, W)) return;
   double4 c = reinterpret_cast<const double4*>(D.cmbr)[w];
   for (int side = 0; side < 2; ++side) {
     const double2* v = layer_xy(Lb, Lo, side == 0 ? pside : 1 - pside) + (side == 0 ? D.pS[w] : D.qS[w]);
@@ -188,6 +199,56 @@ edge_filter_kernel(LayerDev Lb, LayerDev Lo, PairDev D, int64_t K, int32_t* __re
       }
     }
     if (kMode == 0 && tl == 0) { if (side == 0) cP[w] = cnt; else cQ[w] = cnt; }
+  }
+}
+
+// A block per pair: the listed pairs (too long for a warp), or, with n given, the first n pairs
+// of a batch that has no more pairs than blocks.
+constexpr int kFilterLongThreads = 512;
+constexpr int kFilterLongRounds = 4;
+constexpr int kFilterLongBlocks = 2 * 148;
+
+template <int kMode>
+__global__ void __launch_bounds__(kFilterLongThreads)
+edge_filter_long_kernel(LayerDev Lb, LayerDev Lo, PairDev D, int32_t* __restrict__ cP, int32_t* __restrict__ cQ,
+                        const int64_t* __restrict__ offP, const int64_t* __restrict__ offQ, int32_t* __restrict__ LP,
+                        int32_t* __restrict__ LQ, JoinEdges je, LongPairs longs, int n) {
+  __shared__ int cnt[kFilterLongRounds * (kFilterLongThreads / 32) + 1];
+  const unsigned total = longs.ids ? *longs.n : (unsigned)n;
+  for (unsigned j = blockIdx.x; j < total; j += gridDim.x) {
+    const int64_t w = longs.ids ? longs.ids[j] : (int64_t)j;
+    if (D.status[w] != 0) {
+      if (kMode == 0 && threadIdx.x == 0) { cP[w] = 0; cQ[w] = 0; }
+      continue;
+    }
+    const int pside = D.pSide[w];
+    if (join_lists<kMode>(Lb, Lo, D, w, pside, je, cP, cQ, offP, offQ, LP, LQ, (int)threadIdx.x, kFilterLongThreads)) continue;
+    const double4 c = reinterpret_cast<const double4*>(D.cmbr)[w];
+    for (int side = 0; side < 2; ++side) {
+      const double2* v = layer_xy(Lb, Lo, side == 0 ? pside : 1 - pside) + (side == 0 ? D.pS[w] : D.qS[w]);
+      const int m = side == 0 ? D.nP[w] : D.nQ[w];
+      auto touches = [&](int k) {
+        const double2 a = __ldg(v + k), b = __ldg(v + (k + 1 < m ? k + 1 : 0));
+        return edge_touches_box(a.x, a.y, b.x, b.y, c.x, c.y, c.z, c.w);
+      };
+      if (kMode == 0) {
+        int mine = 0;
+#pragma unroll 4
+        for (int k = threadIdx.x; k < m; k += kFilterLongThreads) mine += touches(k) ? 1 : 0;
+        mine = warp_sum(mine);
+        __syncthreads();
+        if (lane_id() == 0) cnt[threadIdx.x >> 5] = mine;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          int sum = 0;
+          for (int i = 0; i < kFilterLongThreads / 32; ++i) sum += cnt[i];
+          (side == 0 ? cP : cQ)[w] = sum;
+        }
+      } else {
+        int32_t* dst = side == 0 ? LP + offP[w] : LQ + offQ[w];
+        block_list<kFilterLongThreads, kFilterLongRounds>(m, cnt, touches, [&](int k, int before) { dst[before] = k; });
+      }
+    }
   }
 }
 
@@ -3461,18 +3522,58 @@ __global__ void out_sizes_kernel(const int32_t* __restrict__ mP, const int32_t* 
   ccap[k] = mP[k] + 2 * nrec[k] + 8;
 }
 
+// A warp copies a pair's result; results of more than kCopyPiece vertices are listed in pieces
+// of that size for out_compact_pieces_kernel (one warp on the 5.4e6 vertices of the large
+// pair took 31 ms).
+constexpr int kCopyPiece = 4096;
+struct CopyPieces { int2* at; unsigned* n; };
+
 __global__ void __launch_bounds__(kThreads, 8)   // 32 registers: compact 0.33 -> 0.20 ms
-out_compact_kernel(int64_t K, const double* __restrict__ xy, const int64_t* __restrict__ vOff,
+out_compact_kernel(int64_t K, const double2* __restrict__ xy, const int64_t* __restrict__ vOff,
                    const int32_t* __restrict__ csz, const int64_t* __restrict__ cOff,
                    const int32_t* __restrict__ nc, const int64_t* __restrict__ nv,
                    const int64_t* __restrict__ fVOff, const int64_t* __restrict__ fCOff,
-                   double* __restrict__ oxy, int32_t* __restrict__ ocsz) {
+                   double2* __restrict__ oxy, int32_t* __restrict__ ocsz, CopyPieces pieces) {
   int64_t w = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
   if (w >= K) return;
-  const double* s = xy + 2 * vOff[w];
-  double* d = oxy + 2 * fVOff[w];
-  for (int64_t i = lane_id(); i < 2 * nv[w]; i += 32) d[i] = s[i];
-  for (int i = lane_id(); i < nc[w]; i += 32) ocsz[fCOff[w] + i] = csz[cOff[w] + i];
+  const double2* s = xy + vOff[w];
+  double2* d = oxy + fVOff[w];
+  const int64_t n = nv[w];
+  const int comps = nc[w];
+  if (n > kCopyPiece) {
+    // the pieces of the vertices, then those of the component sizes (as negative numbers)
+    const int pv = (int)((n + kCopyPiece - 1) / kCopyPiece), pc = (comps + kCopyPiece - 1) / kCopyPiece;
+    unsigned at = 0;
+    if (lane_id() == 0) at = atomicAdd(pieces.n, (unsigned)(pv + pc));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    for (int i = lane_id(); i < pv + pc; i += 32) pieces.at[at + i] = make_int2((int)w, i < pv ? i : ~(i - pv));
+    return;
+  }
+  for (int64_t i = lane_id(); i < n; i += 32) d[i] = s[i];
+  for (int i = lane_id(); i < comps; i += 32) ocsz[fCOff[w] + i] = csz[cOff[w] + i];
+}
+
+__global__ void __launch_bounds__(kThreads)
+out_compact_pieces_kernel(CopyPieces pieces, const double2* __restrict__ xy, const int64_t* __restrict__ vOff,
+                          const int32_t* __restrict__ csz, const int64_t* __restrict__ cOff,
+                          const int32_t* __restrict__ nc, const int64_t* __restrict__ nv,
+                          const int64_t* __restrict__ fVOff, const int64_t* __restrict__ fCOff,
+                          double2* __restrict__ oxy, int32_t* __restrict__ ocsz) {
+  const unsigned n = *pieces.n;
+  for (unsigned p = blockIdx.x; p < n; p += gridDim.x) {
+    const int2 pc = pieces.at[p];
+    const int64_t w = pc.x;
+    if (pc.y >= 0) {
+      const int64_t a = (int64_t)pc.y * kCopyPiece, b = min(a + kCopyPiece, nv[w]);
+      const double2* s = xy + vOff[w];
+      double2* d = oxy + fVOff[w];
+#pragma unroll 4
+      for (int64_t i = a + threadIdx.x; i < b; i += kThreads) d[i] = s[i];
+    } else {
+      const int a = ~pc.y * kCopyPiece, b = min(a + kCopyPiece, nc[w]);
+      for (int i = a + (int)threadIdx.x; i < b; i += kThreads) ocsz[fCOff[w] + i] = csz[cOff[w] + i];
+    }
+  }
 }
 
 }  // namespace
@@ -3535,14 +3636,38 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   cudaStream_t sw = two ? aux : s;
   auto fork_aux = [&]() { if (two) { cudaEventRecord(fev[0], s); cudaStreamWaitEvent(aux, fev[0], 0); } };
   auto join_aux = [&]() { if (two) { cudaEventRecord(fev[1], aux); cudaStreamWaitEvent(s, fev[1], 0); } };
-  // ---- G1 edge filter
-  fork_aux();
-  { edge_filter_kernel<0, kFilterTile><<<(unsigned)((K * kFilterTile + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-        Lb, Lo, D, K, cP, cQ, nullptr, nullptr, nullptr, nullptr, -1, kFilterTileMax, jed); note_launch(); }
-  { edge_filter_kernel<0, 32><<<blocks_for_warps(K), kThreads, 0, sw>>>(Lb, Lo, D, K, cP, cQ, nullptr, nullptr,
-                                                                       nullptr, nullptr, kFilterTileMax,
-                                                                       INT64_MAX, jed); note_launch(); }
-  join_aux();
+  // ---- G1 edge filter: narrow tiles, warps, and blocks for the pairs too long for a warp
+  // (left out where the join or the layers' sizes rule such pairs out); a batch of fewer
+  // pairs than blocks takes a block per pair throughout
+  const bool fewPairs = K <= kFilterLongBlocks;
+  const bool longPairs = !fewPairs && jed.max_ring > kLongRing &&
+                         !(Lb.nverts > 0 && Lo.nverts > 0 && Lb.nverts + Lo.nverts <= kLongRing);
+  LongPairs lpF;
+  if (longPairs) {
+    lpF.ids = A.take_n<int32_t>(K);
+    lpF.n = A.take_n<unsigned>(1);
+    if (!lpF.ids || !lpF.n) return ST_OUT_OF_MEMORY;
+    cudaMemsetAsync(lpF.n, 0, sizeof(unsigned), s);
+  }
+  auto edge_filter = [&](auto mode, int32_t* lp, int32_t* lq) {
+    constexpr int kMode = decltype(mode)::value;
+    if (fewPairs) {
+      edge_filter_long_kernel<kMode><<<(unsigned)K, kFilterLongThreads, 0, s>>>(Lb, Lo, D, cP, cQ, offP, offQ, lp, lq, jed,
+                                                                              LongPairs{}, (int)K);
+      note_launch();
+      return;
+    }
+    fork_aux();
+    { edge_filter_kernel<kMode, kFilterTile><<<(unsigned)((K * kFilterTile + kThreads - 1) / kThreads), kThreads, 0, s>>>(
+          Lb, Lo, D, K, cP, cQ, offP, offQ, lp, lq, -1, kFilterTileMax, jed, LongPairs{}); note_launch(); }
+    { edge_filter_kernel<kMode, 32><<<blocks_for_warps(K), kThreads, 0, sw>>>(
+          Lb, Lo, D, K, cP, cQ, offP, offQ, lp, lq, kFilterTileMax, longPairs ? kLongRing : INT64_MAX, jed, lpF); note_launch(); }
+    if (longPairs)
+      { edge_filter_long_kernel<kMode><<<kFilterLongBlocks, kFilterLongThreads, 0, sw>>>(Lb, Lo, D, cP, cQ, offP, offQ, lp,
+                                                                                       lq, jed, lpF, 0); note_launch(); }
+    join_aux();
+  };
+  edge_filter(std::integral_constant<int, 0>{}, nullptr, nullptr);
   exclusive_scan_i32(cP, offP, K, tot + 0, stK, d_err, s);
   exclusive_scan_i32(cQ, offQ, K, tot + 1, stK, d_err, s);
   exclusive_scan_i32(D.nP, eoffP, K, tot + 2, stK, d_err, s);
@@ -3590,12 +3715,7 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   if (nCh > 0) { chunk_pair_kernel<<<blocks_for_warps(K), kThreads, 0, s>>>(chunkOff, nchunk, K, chunkPair); note_launch(); }
   cudaMemsetAsync(binRec, 0, K * sizeof(int64_t), s);
   cudaMemsetAsync(binQ, 0, K * sizeof(int64_t), s);
-  fork_aux();
-  { edge_filter_kernel<1, kFilterTile><<<(unsigned)((K * kFilterTile + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-        Lb, Lo, D, K, cP, cQ, offP, offQ, LP, LQ, -1, kFilterTileMax, jed); note_launch(); }
-  { edge_filter_kernel<1, 32><<<blocks_for_warps(K), kThreads, 0, sw>>>(Lb, Lo, D, K, cP, cQ, offP, offQ, LP, LQ,
-                                                                       kFilterTileMax, INT64_MAX, jed); note_launch(); }
-  join_aux();
+  edge_filter(std::integral_constant<int, 1>{}, LP, LQ);
   // The binned pairs (below) go to the auxiliary stream when there is one: fork here, before
   // the chunked count is queued on s, so that the two run side by side.
   cudaStream_t sb = s;
@@ -4138,8 +4258,22 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   C.xy = A.take_n<double>(2 * C.n_vertices);
   C.comp_size = A.take_n<int32_t>(C.n_components);
   if (!C.xy || !C.comp_size) return ST_OUT_OF_MEMORY;
-  { out_compact_kernel<<<blocks_for_warps(K), kThreads, 0, s>>>(K, oxy, vOff, ocsz, cOff, nc, nv, fVOff,
-                                                              C.comp_off, C.xy, C.comp_size); note_launch(); }
+  // at most one piece per kCopyPiece vertices of a listed pair and one more, and as many for
+  // its components (each has a vertex)
+  const int64_t maxPieces = C.n_vertices > kCopyPiece ? 4 * (C.n_vertices / kCopyPiece) + 4 : 0;
+  CopyPieces pieces{nullptr, nullptr};
+  if (maxPieces > 0) {
+    pieces = CopyPieces{A.take_n<int2>(maxPieces), A.take_n<unsigned>(1)};
+    if (!pieces.at || !pieces.n) return ST_OUT_OF_MEMORY;
+    cudaMemsetAsync(pieces.n, 0, sizeof(unsigned), s);
+  }
+  const double2* oxy2 = reinterpret_cast<const double2*>(oxy);
+  double2* cxy2 = reinterpret_cast<double2*>(C.xy);
+  { out_compact_kernel<<<blocks_for_warps(K), kThreads, 0, s>>>(K, oxy2, vOff, ocsz, cOff, nc, nv, fVOff, C.comp_off, cxy2,
+                                                              C.comp_size, pieces); note_launch(); }
+  if (maxPieces > 0)
+    { out_compact_pieces_kernel<<<(unsigned)std::min<int64_t>(maxPieces, 8 * 148), kThreads, 0, s>>>(
+          pieces, oxy2, vOff, ocsz, cOff, nc, nv, fVOff, C.comp_off, cxy2, C.comp_size); note_launch(); }
   C.vert_off = fVOff;
   mk->mark("clip:compact", s);
   return ST_OK;

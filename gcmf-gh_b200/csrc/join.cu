@@ -24,6 +24,10 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarpsPerBlock = kThreads / 32;
 
+constexpr int kLongThreads = 512;       // block-per-pair kernels (kLongRing)
+constexpr int kLongRounds = 4;
+constexpr int kLongBlocks = 2 * 148;    // two of them per SM, taking the listed pairs in turn
+
 inline unsigned blocks_for_warps(int64_t warps) {
   return (unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
 }
@@ -98,16 +102,63 @@ __device__ __forceinline__ bool mbr_write(int64_t w, int nv, double x1, double y
 constexpr int kMbrPerWarp = 4;
 constexpr int kMbrSmallMax = 64;
 
+// A whole block's MBR of one polygon (long rings: four loads in flight per thread), valid
+// in thread 0.
+template <int kBlock>
+__device__ __forceinline__ void block_mbr(const LayerDev& L, int64_t w, float2* xyf, double (*part)[4], double& x1,
+                                          double& y1, double& x2, double& y2) {
+  const int nv = L.vnum[w];
+  const int64_t s = L.vps[w] - nv;
+  const double2* v = reinterpret_cast<const double2*>(L.xy) + s;
+  x1 = y1 = INFINITY;
+  x2 = y2 = -INFINITY;
+  for (int k0 = 0; k0 < nv; k0 += 4 * kBlock) {
+    double2 p[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = k0 + u * kBlock + (int)threadIdx.x;
+      p[u] = __ldg(v + (k < nv ? k : 0));
+      if (xyf && k < nv) xyf[s + k] = make_float2(__double2float_rn(p[u].x), __double2float_rn(p[u].y));
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      x1 = fmin(x1, p[u].x); x2 = fmax(x2, p[u].x);
+      y1 = fmin(y1, p[u].y); y2 = fmax(y2, p[u].y);
+    }
+  }
+  mbr_reduce<32>(x1, y1, x2, y2);
+  const int warp = (int)(threadIdx.x >> 5);
+  __syncthreads();
+  if (lane_id() == 0) { part[warp][0] = x1; part[warp][1] = y1; part[warp][2] = x2; part[warp][3] = y2; }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int j = 1; j < kBlock / 32; ++j) {
+      x1 = fmin(x1, part[j][0]); y1 = fmin(y1, part[j][1]);
+      x2 = fmax(x2, part[j][2]); y2 = fmax(y2, part[j][3]);
+    }
+}
+
+// Rings of more than kMbrLong stored vertices are taken by their whole block once its warps
+// are done with the others.  n_valid[8]: the layer's largest ring, if beyond kMbrNoteMin.
+constexpr int kMbrLong = 1024;
+constexpr int kMbrNoteMin = 128;
+
 __global__ void __launch_bounds__(kThreads)
 mbr_kernel(LayerDev L, double* __restrict__ mbr, uint8_t* __restrict__ valid,
            uint64_t* __restrict__ key, uint32_t* __restrict__ id, unsigned long long* n_valid,
            float2* __restrict__ xyf) {
+  __shared__ int32_t longs[kWarpsPerBlock * kMbrPerWarp];
+  __shared__ double part[kWarpsPerBlock][4];
+  __shared__ int nLong;
+  if (threadIdx.x == 0) nLong = 0;
+  __syncthreads();
   const int64_t p0 = (((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5) * kMbrPerWarp;
-  if (p0 >= L.n) return;
   const int lane = (int)lane_id();
   const int mine = (lane < kMbrPerWarp && p0 + lane < L.n) ? L.vnum[p0 + lane] : 0;
+  const int top = __reduce_max_sync(0xffffffffu, mine);
+  if (lane == 0 && top > kMbrNoteMin) atomicMax(n_valid + 8, (unsigned long long)top);
   int ok = 0;
-  if (__all_sync(0xffffffffu, mine <= kMbrSmallMax)) {
+  if (top <= kMbrSmallMax) {
     constexpr int W = 32 / kMbrPerWarp;
     const int g = lane / W, t = lane % W;
     const int64_t w = p0 + g;
@@ -129,6 +180,10 @@ mbr_kernel(LayerDev L, double* __restrict__ mbr, uint8_t* __restrict__ valid,
     for (int g = 0; g < kMbrPerWarp && p0 + g < L.n; ++g) {
       const int64_t w = p0 + g;
       const int nv = __shfl_sync(0xffffffffu, mine, g);
+      if (nv > kMbrLong) {
+        if (lane == 0) longs[atomicAdd(&nLong, 1)] = (int32_t)(w - (int64_t)blockIdx.x * (kWarpsPerBlock * kMbrPerWarp));
+        continue;
+      }
       const int64_t s = L.vps[w] - nv;
       const double2* v = reinterpret_cast<const double2*>(L.xy) + s;
       double x1 = INFINITY, y1 = INFINITY, x2 = -INFINITY, y2 = -INFINITY;
@@ -141,6 +196,13 @@ mbr_kernel(LayerDev L, double* __restrict__ mbr, uint8_t* __restrict__ valid,
       mbr_reduce<32>(x1, y1, x2, y2);
       if (lane == 0) ok += mbr_write(w, nv, x1, y1, x2, y2, mbr, valid, key, id) ? 1 : 0;
     }
+  }
+  __syncthreads();
+  for (int j = 0; j < nLong; ++j) {
+    const int64_t w = (int64_t)blockIdx.x * (kWarpsPerBlock * kMbrPerWarp) + longs[j];
+    double x1, y1, x2, y2;
+    block_mbr<kThreads>(L, w, xyf, part, x1, y1, x2, y2);
+    if (threadIdx.x == 0) ok += mbr_write(w, L.vnum[w], x1, y1, x2, y2, mbr, valid, key, id) ? 1 : 0;
   }
   ok = __reduce_add_sync(0xffffffffu, ok);
   if (lane == 0 && ok) atomicAdd(n_valid, (unsigned long long)ok);
@@ -387,11 +449,19 @@ __global__ void cmbr_kernel(const uint64_t* __restrict__ keys, int64_t K, int ob
 // Crossing parity of the contained candidate's first vertex against the other polygon's
 // stored ring, edges (i, i-1) for every stored vertex i (GPU_Join.h:856-939).  A warp per
 // candidate pair; the parity of the per-lane parities equals the reference's XOR scan.
+// whether edge (i, i - 1) of the stored ring v[0, nv) toggles the parity of P
+__device__ __forceinline__ bool pip_crosses(const double2* v, int i, int nv, double2 P) {
+  const double2 a = __ldg(v + i), c = __ldg(v + (i == 0 ? nv - 1 : i - 1));
+  const double Y1 = a.y, Y2 = c.y, X1 = a.x, X2 = c.x;
+  if ((Y1 > P.y) == (Y2 > P.y)) return false;
+  return P.x < (X2 - X1) * (P.y - Y1) / (Y2 - Y1) + X1;
+}
+
 template <int W>
 __global__ void __launch_bounds__(kThreads, 6)
 pip_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const int32_t* __restrict__ po,
            const int8_t* __restrict__ pip_type, int64_t K, int8_t* __restrict__ pip_flag,
-           int8_t* __restrict__ join_flag, int64_t lo, int64_t hi) {
+           int8_t* __restrict__ join_flag, int64_t lo, int64_t hi, LongPairs longs) {
   const JTile<W> T;
   const int64_t w = JTile<W>::unit();
   if (w >= K) return;
@@ -407,18 +477,36 @@ pip_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const int32
   const double2* pt = reinterpret_cast<const double2*>(Lp.xy) + (Lp.vps[ip] - Lp.vnum[ip]);
   const double2 P = pt[0];
   const int nv = Lr.vnum[ir];
-  if (nv <= lo || nv > hi) return;                 // the other pass takes this pair
+  if (nv <= lo || nv > hi) {                       // another pass takes this pair
+    if (W == 32 && nv > hi && longs.ids && T.lane == 0) longs.add(w);
+    return;
+  }
   const double2* v = reinterpret_cast<const double2*>(Lr.xy) + (Lr.vps[ir] - nv);
   int par = 0;
-  for (int i = T.lane; i < nv; i += W) {
-    int j = (i == 0) ? nv - 1 : i - 1;
-    double2 a = __ldg(v + i), c = __ldg(v + j);
-    double Y1 = a.y, Y2 = c.y, X1 = a.x, X2 = c.x;
-    if ((Y1 > P.y) == (Y2 > P.y)) continue;
-    if (P.x < (X2 - X1) * (P.y - Y1) / (Y2 - Y1) + X1) par ^= 1;
-  }
+  for (int i = T.lane; i < nv; i += W) par ^= pip_crosses(v, i, nv, P) ? 1 : 0;
   int inside = __popc(T.ballot(par)) & 1;
   if (T.lane == 0) { pip_flag[w] = (int8_t)inside; join_flag[w] = inside ? 0 : 1; }
+}
+
+// a block per pair: the pairs whose ring is too long for a warp
+__global__ void __launch_bounds__(kLongThreads)
+pip_long_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const int32_t* __restrict__ po,
+                const int8_t* __restrict__ pip_type, int8_t* __restrict__ pip_flag, int8_t* __restrict__ join_flag,
+                LongPairs longs) {
+  for (unsigned j = blockIdx.x; j < *longs.n; j += gridDim.x) {
+    const int64_t w = longs.ids[j];
+    const bool base = pip_type[w] == 1;                // the base polygon's first vertex in the overlay's ring
+    const LayerDev& Lp = base ? Lb : Lo;
+    const LayerDev& Lr = base ? Lo : Lb;
+    const int ip = base ? pb[w] : po[w], ir = base ? po[w] : pb[w], nv = Lr.vnum[ir];
+    const double2 P = reinterpret_cast<const double2*>(Lp.xy)[Lp.vps[ip] - Lp.vnum[ip]];
+    const double2* v = reinterpret_cast<const double2*>(Lr.xy) + (Lr.vps[ir] - nv);
+    int par = 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nv; i += kLongThreads) par ^= pip_crosses(v, i, nv, P) ? 1 : 0;
+    const int inside = __syncthreads_count(par) & 1;
+    if (threadIdx.x == 0) { pip_flag[w] = (int8_t)inside; join_flag[w] = inside ? 0 : 1; }
+  }
 }
 
 // ---------------------------------------------------------------- J5: common-MBR filter
@@ -445,7 +533,7 @@ cmf_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const int32
            const double* __restrict__ cmbr, int64_t K, int8_t* __restrict__ join_flag,
            int32_t* __restrict__ bE, int32_t* __restrict__ oE,
            const int64_t* __restrict__ bOff, const int64_t* __restrict__ oOff,
-           int32_t* __restrict__ bList, int32_t* __restrict__ oList, int64_t lo, int64_t hi) {
+           int32_t* __restrict__ bList, int32_t* __restrict__ oList, int64_t lo, int64_t hi, LongPairs longs) {
   const JTile<W> T;
   const int64_t w = JTile<W>::unit();
   if (w >= K) return;
@@ -456,7 +544,10 @@ cmf_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const int32
   if (kMode == 1 && bE[w] == 0) return;
   {
     const int64_t size = (int64_t)Lb.vnum[pb[w]] + Lo.vnum[po[w]];
-    if (size <= lo || size > hi) return;             // the other pass takes this pair
+    if (size <= lo || size > hi) {                   // another pass takes this pair
+      if (kMode == 0 && W == 32 && size > hi && longs.ids && T.lane == 0) longs.add(w);
+      return;
+    }
   }
   double4 c = reinterpret_cast<const double4*>(cmbr)[w];
   const float cx1d = kF32 ? __double2float_rd(c.x) : 0.f, cy1d = kF32 ? __double2float_rd(c.y) : 0.f;
@@ -512,7 +603,8 @@ template <int W, int kF32>
 __global__ void __launch_bounds__(kThreads, 8)
 cmf_append_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const int32_t* __restrict__ po,
                   const double* __restrict__ cmbr, int64_t K, int8_t* __restrict__ join_flag,
-                  int32_t* __restrict__ bE, int32_t* __restrict__ oE, CmfOut out, int64_t lo, int64_t hi) {
+                  int32_t* __restrict__ bE, int32_t* __restrict__ oE, CmfOut out, int64_t lo, int64_t hi,
+                  LongPairs longs) {
   constexpr int kTiles = kThreads / W;
   __shared__ int sCnt[2][kTiles];
   __shared__ unsigned long long sBase[2];
@@ -523,7 +615,8 @@ cmf_append_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, cons
   if (w < K && !join_flag[w] && W != 32 && T.lane == 0) { bE[w] = 0; oE[w] = 0; }
   if (mine) {
     const int64_t size = (int64_t)Lb.vnum[pb[w]] + Lo.vnum[po[w]];
-    mine = size > lo && size <= hi;                 // else the other pass takes this pair
+    mine = size > lo && size <= hi;                 // else another pass takes this pair
+    if (W == 32 && size > hi && longs.ids && T.lane == 0) longs.add(w);
   }
   double4 c = make_double4(0, 0, 0, 0);
   float cx1d = 0.f, cy1d = 0.f, cx2u = 0.f, cy2u = 0.f;
@@ -593,6 +686,82 @@ cmf_append_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, cons
   }
 }
 
+// A block per pair: the pairs whose rings are too long for a warp.  kMode 0 counts, 1 writes
+// at the given offsets (cmf_kernel's passes), 2 does both, taking its own ranges of the
+// lists as cmf_append_kernel does.
+template <int kMode, int kF32>
+__global__ void __launch_bounds__(kLongThreads)
+cmf_long_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const int32_t* __restrict__ po,
+                const double* __restrict__ cmbr, int8_t* __restrict__ join_flag, int32_t* __restrict__ bE,
+                int32_t* __restrict__ oE, CmfOut out, LongPairs longs) {
+  __shared__ int cnt[kLongRounds * (kLongThreads / 32) + 1];
+  __shared__ unsigned long long sBase[2];
+  for (unsigned j = blockIdx.x; j < *longs.n; j += gridDim.x) {
+    const int64_t w = longs.ids[j];
+    const double4 c = reinterpret_cast<const double4*>(cmbr)[w];
+    const float cx1d = __double2float_rd(c.x), cy1d = __double2float_rd(c.y);
+    const float cx2u = __double2float_ru(c.z), cy2u = __double2float_ru(c.w);
+    auto ring = [&](int side) {
+      const LayerDev& L = side == 0 ? Lb : Lo;
+      const int id = side == 0 ? pb[w] : po[w];
+      return make_longlong2(L.vps[id] - L.vnum[id], L.vnum[id]);
+    };
+    auto touches = [&](const LayerDev& L, longlong2 r, int k) {
+      const double2* v = reinterpret_cast<const double2*>(L.xy) + r.x;
+      const int k2 = (k < (int)r.y - 1) ? k + 1 : 0;
+      if (kF32 && f32_rejects(__ldg(L.xyf + r.x + k), __ldg(L.xyf + r.x + k2), cx1d, cy1d, cx2u, cy2u)) return false;
+      const double2 a = __ldg(v + k), b = __ldg(v + k2);
+      return edge_touches_box(a.x, a.y, b.x, b.y, c.x, c.y, c.z, c.w);
+    };
+    if (kMode != 1) {
+      int n[2];
+      for (int side = 0; side < 2; ++side) {
+        const LayerDev& L = side == 0 ? Lb : Lo;
+        const longlong2 r = ring(side);
+        int mine = 0;
+#pragma unroll 4
+        for (int k = threadIdx.x; k < (int)r.y; k += kLongThreads) mine += touches(L, r, k) ? 1 : 0;
+        mine = warp_sum(mine);
+        __syncthreads();
+        if (lane_id() == 0) cnt[threadIdx.x >> 5] = mine;
+        __syncthreads();
+        n[side] = 0;
+        for (int i = 0; i < kLongThreads / 32; ++i) n[side] += cnt[i];
+      }
+      const bool keep = n[0] > 0 && n[1] > 0;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        if (!keep) { join_flag[w] = 0; bE[w] = 0; oE[w] = 0; }
+        else {
+          bE[w] = n[0];
+          oE[w] = n[1];
+          if (kMode == 2) {
+            out.bOff[w] = (int64_t)(sBase[0] = atomicAdd(out.total, (unsigned long long)n[0]));
+            out.oOff[w] = (int64_t)(sBase[1] = atomicAdd(out.total + 1, (unsigned long long)n[1]));
+          }
+        }
+      }
+      __syncthreads();
+      if (!keep || kMode == 0) continue;
+    } else {
+      if (!join_flag[w] || bE[w] == 0) continue;
+      __syncthreads();
+      if (threadIdx.x == 0) { sBase[0] = (unsigned long long)out.bOff[w]; sBase[1] = (unsigned long long)out.oOff[w]; }
+      __syncthreads();
+    }
+    for (int side = 0; side < 2; ++side) {
+      const LayerDev& L = side == 0 ? Lb : Lo;
+      const longlong2 r = ring(side);
+      int32_t* list = side == 0 ? out.bList : out.oList;
+      const int64_t cap = side == 0 ? out.bCap : out.oCap, base = (int64_t)sBase[side];
+      block_list<kLongThreads, kLongRounds>(
+          (int)r.y, cnt, [&](int k) { return touches(L, r, k); },
+          [&](int k, int before) { if (base + before < cap) list[base + before] = k; });
+    }
+    __syncthreads();
+  }
+}
+
 // ---------------------------------------------------------------- J6: refine
 // Does any surviving (base edge, overlay edge) pair intersect?  The closed-form test of
 // GPU_Join.h:373-446 in its operation order: zero-length base edges are skipped, box
@@ -632,13 +801,16 @@ refine_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const in
               const int32_t* __restrict__ bE, const int32_t* __restrict__ oE,
               const int64_t* __restrict__ bOff, const int64_t* __restrict__ oOff,
               const int32_t* __restrict__ bList, const int32_t* __restrict__ oList,
-              int8_t* __restrict__ seg_flag, int64_t lo, int64_t hi) {
+              int8_t* __restrict__ seg_flag, int64_t lo, int64_t hi, LongPairs longs) {
   const JTile<W> T;
   const int64_t w = JTile<W>::unit();
   if (w >= K) return;
   if (!join_flag[w]) { if (W != 32 && T.lane == 0) seg_flag[w] = 0; return; }
   const int nb = bE[w], no = oE[w];
-  if ((int64_t)nb * no <= lo || (int64_t)nb * no > hi) return;   // the other pass takes this pair
+  if ((int64_t)nb * no <= lo || (int64_t)nb * no > hi) {         // another pass takes this pair
+    if (W == 32 && (int64_t)nb * no > hi && longs.ids && T.lane == 0) longs.add(w);
+    return;
+  }
   const int b = pb[w], o = po[w];
   const int bV = Lb.vnum[b], oV = Lo.vnum[o];
   const double2* bv = reinterpret_cast<const double2*>(Lb.xy) + (Lb.vps[b] - bV);
@@ -667,6 +839,50 @@ refine_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const in
     found = T.ballot(hit) != 0u;
   }
   if (T.lane == 0) seg_flag[w] = (int8_t)found;
+}
+
+// A block per pair: the pairs whose edge grid is too large for a warp (one without a hit
+// has to be gone through whole: 4.3 ms for one warp on a join of two layers with polygons
+// of 45,000 vertices).
+__global__ void __launch_bounds__(kLongThreads)
+refine_long_kernel(LayerDev Lb, LayerDev Lo, const int32_t* __restrict__ pb, const int32_t* __restrict__ po,
+                   const int32_t* __restrict__ bE, const int32_t* __restrict__ oE,
+                   const int64_t* __restrict__ bOff, const int64_t* __restrict__ oOff,
+                   const int32_t* __restrict__ bList, const int32_t* __restrict__ oList,
+                   int8_t* __restrict__ seg_flag, LongPairs longs) {
+  for (unsigned j = blockIdx.x; j < *longs.n; j += gridDim.x) {
+    const int64_t w = longs.ids[j];
+    const int nb = bE[w], no = oE[w], b = pb[w], o = po[w];
+    const int bV = Lb.vnum[b], oV = Lo.vnum[o];
+    const double2* bv = reinterpret_cast<const double2*>(Lb.xy) + (Lb.vps[b] - bV);
+    const double2* ov = reinterpret_cast<const double2*>(Lo.xy) + (Lo.vps[o] - oV);
+    const int32_t* bl = bList + bOff[w];
+    const int32_t* ol = oList + oOff[w];
+    const int64_t total = (int64_t)nb * no;
+    int found = 0;
+    for (int64_t t0 = 0; t0 < total && !found; t0 += 8 * kLongThreads) {
+      bool hit = false;
+#pragma unroll 2
+      for (int u = 0; u < 8; ++u) {
+        const int64_t t = t0 + u * kLongThreads + threadIdx.x;
+        if (t >= total) break;
+        int be, oe;
+        if (total <= INT32_MAX) {
+          const int tt = (int)t, r = tt / no;
+          be = bl[r];
+          oe = ol[tt - r * no];
+        } else {
+          be = bl[t / no];
+          oe = ol[t % no];
+        }
+        const double2 b1 = __ldg(bv + be), b2 = __ldg(bv + ((be < bV - 1) ? be + 1 : 0));
+        const double2 o1 = __ldg(ov + oe), o2 = __ldg(ov + ((oe < oV - 1) ? oe + 1 : 0));
+        hit = hit || segment_hit(b1.x, b1.y, b2.x, b2.y, o1.x, o1.y, o2.x, o2.y);
+      }
+      found = __syncthreads_or(hit);
+    }
+    if (threadIdx.x == 0) seg_flag[w] = found ? 1 : 0;
+  }
 }
 
 // ---------------------------------------------------------------- clip set + stats
@@ -699,21 +915,30 @@ __global__ void clip_compact_kernel(const int8_t* __restrict__ clip, const int64
   cand[off[k]] = k;
 }
 
-// MBRs only (the clip pipeline's common MBRs), same definition as mbr_kernel
+// MBRs only (the clip pipeline's common MBRs), same definition as mbr_kernel: a warp per
+// polygon, long ones by the whole block afterwards
 __global__ void __launch_bounds__(kThreads)
 mbr_only_kernel(LayerDev L, double* __restrict__ mbr) {
-  int64_t w = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
-  if (w >= L.n) return;
-  const int nv = L.vnum[w];
-  const double2* v = reinterpret_cast<const double2*>(L.xy) + (L.vps[w] - nv);
-  double x1 = INFINITY, y1 = INFINITY, x2 = -INFINITY, y2 = -INFINITY;
-  for (int k = lane_id(); k < nv; k += 32) {
-    double2 p = __ldg(v + k);
-    x1 = fmin(x1, p.x); x2 = fmax(x2, p.x);
-    y1 = fmin(y1, p.y); y2 = fmax(y2, p.y);
+  __shared__ double part[kWarpsPerBlock][4];
+  const int64_t w0 = (int64_t)blockIdx.x * kWarpsPerBlock, w = w0 + (threadIdx.x >> 5);
+  if (w < L.n && L.vnum[w] <= kMbrLong) {
+    const int nv = L.vnum[w];
+    const double2* v = reinterpret_cast<const double2*>(L.xy) + (L.vps[w] - nv);
+    double x1 = INFINITY, y1 = INFINITY, x2 = -INFINITY, y2 = -INFINITY;
+    for (int k = lane_id(); k < nv; k += 32) {
+      double2 p = __ldg(v + k);
+      x1 = fmin(x1, p.x); x2 = fmax(x2, p.x);
+      y1 = fmin(y1, p.y); y2 = fmax(y2, p.y);
+    }
+    mbr_reduce<32>(x1, y1, x2, y2);
+    if (lane_id() == 0) reinterpret_cast<double4*>(mbr)[w] = make_double4(x1, y1, x2, y2);
   }
-  x1 = warp_min(x1); y1 = warp_min(y1); x2 = warp_max(x2); y2 = warp_max(y2);
-  if (lane_id() == 0) reinterpret_cast<double4*>(mbr)[w] = make_double4(x1, y1, x2, y2);
+  for (int64_t k = w0; k < w0 + kWarpsPerBlock && k < L.n; ++k) {
+    if (L.vnum[k] <= kMbrLong) continue;
+    double x1, y1, x2, y2;
+    block_mbr<kThreads>(L, k, nullptr, part, x1, y1, x2, y2);
+    if (threadIdx.x == 0) reinterpret_cast<double4*>(mbr)[k] = make_double4(x1, y1, x2, y2);
+  }
 }
 
 int bits_for(int64_t n) {
@@ -756,7 +981,7 @@ int run_join(const LayerDev& Lb0, const LayerDev& Lo0, Arena& A, JoinDev& J, int
   uint32_t* vAlt = A.take_n<uint32_t>(nb);
   uint64_t* kAltO = A.take_n<uint64_t>(no);
   uint32_t* vAltO = A.take_n<uint32_t>(no);
-  unsigned long long* d_cnt = A.take_n<unsigned long long>(8);
+  unsigned long long* d_cnt = A.take_n<unsigned long long>(16);
   float2* xyfB = nullptr;
   float2* xyfO = nullptr;
   if (f32cmf) {
@@ -771,7 +996,7 @@ int run_join(const LayerDev& Lb0, const LayerDev& Lo0, Arena& A, JoinDev& J, int
   if (!J.mbr_b || !J.mbr_o || !J.valid_b || !J.valid_o || !keyB || !keyO || !idB || !idO || !kAlt ||
       !vAlt || !kAltO || !vAltO || !d_cnt || !tmp || !tmpO)
     return ST_OUT_OF_MEMORY;
-  cudaMemsetAsync(d_cnt, 0, 8 * sizeof(unsigned long long), s);
+  cudaMemsetAsync(d_cnt, 0, 16 * sizeof(unsigned long long), s);
   // The two layers' MBRs and sorts are independent and each fills under half of the GPU
   // (about 100 blocks per pass), so the overlay's run on the auxiliary stream.
   cudaStream_t so = s;
@@ -798,11 +1023,12 @@ int run_join(const LayerDev& Lb0, const LayerDev& Lo0, Arena& A, JoinDev& J, int
     cudaEventRecord(join, so);
     cudaStreamWaitEvent(s, join, 0);
   }
-  cudaMemcpyAsync(h_scratch, d_cnt, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  cudaMemcpyAsync(h_scratch, d_cnt, 10 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
   std::vector<double> hpart(7 * kExtentBlocks);
   if (!forceSweep) cudaMemcpyAsync(hpart.data(), part, hpart.size() * sizeof(double), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return ST_CUDA_ERROR;
   const int64_t nvb = h_scratch[0], nvo = h_scratch[1];
+  const int64_t maxB = std::max<int64_t>(h_scratch[8], kMbrNoteMin), maxO = std::max<int64_t>(h_scratch[9], kMbrNoteMin);
   const int obits = bits_for(no);
   const int bbits = bits_for(nb);
   if (obits + bbits > 64) return ST_INVALID_ARGUMENT;
@@ -965,20 +1191,22 @@ int run_join(const LayerDev& Lb0, const LayerDev& Lo0, Arena& A, JoinDev& J, int
   }
   if (K == 0) return ST_OK;
   return join_from_keys(Lb, Lo, pkeys, K, obits, A, J, d_total, d_cnt, d_err, h_scratch, s, mk, aux, list_hint_b,
-                        list_hint_o, (joinOpts & 8) != 0);
+                        list_hint_o, (joinOpts & 8) != 0, maxB, maxO);
 }
 
 // Stages J3-J6 and the clip set over candidate pairs given as packed keys
 // (b << obits | o) sorted ascending; J.mbr_b/J.mbr_o hold the layers' MBRs.  d_total
-// (4 entries) and d_cnt (8 entries, zeroed) are device scratch counters.
+// (4 entries) and d_cnt (8 entries, zeroed) are device scratch counters; maxB, maxO bound the
+// layers' stored vertices per polygon.
 // lanes per pair of the narrow-tile passes, and the pair size up to which they are used
 constexpr int kJoinTile = 4;
 constexpr int64_t kJoinTileMax = 64;
+constexpr int64_t kJoinGridMax = 1 << 14;     // edge grids beyond this: a block instead of a warp
 
 int join_from_keys(const LayerDev& Lb, const LayerDev& Lo, const uint64_t* pkeys, int64_t K, int obits,
                    Arena& A, JoinDev& J, int64_t* d_total, unsigned long long* d_cnt, int* d_err,
                    int64_t* h_scratch, cudaStream_t s, Marks* mk, cudaStream_t aux, int64_t hintB,
-                   int64_t hintO, bool twoPass) {
+                   int64_t hintO, bool twoPass, int64_t maxB, int64_t maxO) {
   Marks dummy;
   if (!mk) mk = &dummy;
   J.n_pairs = K;
@@ -993,6 +1221,22 @@ int join_from_keys(const LayerDev& Lb, const LayerDev& Lo, const uint64_t* pkeys
   cudaStream_t sw = two ? aux : s;
   auto fork_aux = [&]() { if (two) { cudaEventRecord(ev[0], s); cudaStreamWaitEvent(aux, ev[0], 0); } };
   auto join_aux = [&]() { if (two) { cudaEventRecord(ev[1], aux); cudaStreamWaitEvent(s, ev[1], 0); } };
+  // Pairs too large for a warp, listed by each stage's warp pass for a block-per-pair kernel
+  // behind it; stages that cannot have any (by the layers' largest polygons) skip both.
+  J.max_ring = std::min<int64_t>(maxB + maxO, INT32_MAX);
+  const bool longPip = std::max(maxB, maxO) > kLongRing, longCmf = maxB + maxO > kLongRing;
+  const bool longGrid = maxB > 0 && maxO > kJoinGridMax / maxB;
+  LongPairs lpPip, lpCmf, lpGrid;
+  if (longPip || longCmf || longGrid) {
+    int32_t* ids = A.take_n<int32_t>(3 * K);
+    unsigned* n = A.take_n<unsigned>(4);
+    if (!ids || !n) return ST_OUT_OF_MEMORY;
+    cudaMemsetAsync(n, 0, 4 * sizeof(unsigned), s);
+    if (longPip) lpPip = LongPairs{ids, n};
+    if (longCmf) lpCmf = LongPairs{ids + K, n + 1};
+    if (longGrid) lpGrid = LongPairs{ids + 2 * K, n + 2};
+  }
+  const int64_t hiRing = longCmf ? kLongRing : INT64_MAX;
   // ---- J3 CMBR + containment candidates
   J.b = A.take_n<int32_t>(K); J.o = A.take_n<int32_t>(K);
   J.cmbr = A.take_n<double>(4 * K);
@@ -1014,9 +1258,13 @@ int join_from_keys(const LayerDev& Lb, const LayerDev& Lo, const uint64_t* pkeys
   // test), then whole warps for the rest
   fork_aux();
   { pip_kernel<kJoinTile><<<blocks_for_tiles(K, kJoinTile), kThreads, 0, s>>>(
-        Lb, Lo, J.b, J.o, J.pip_type, K, J.pip_flag, J.join_flag, -1, kJoinTileMax); note_launch(); }
+        Lb, Lo, J.b, J.o, J.pip_type, K, J.pip_flag, J.join_flag, -1, kJoinTileMax, LongPairs{}); note_launch(); }
   { pip_kernel<32><<<blocks_for_warps(K), kThreads, 0, sw>>>(Lb, Lo, J.b, J.o, J.pip_type, K, J.pip_flag,
-                                                           J.join_flag, kJoinTileMax, INT64_MAX); note_launch(); }
+                                                           J.join_flag, kJoinTileMax, longPip ? kLongRing : INT64_MAX,
+                                                           lpPip); note_launch(); }
+  if (longPip)
+    { pip_long_kernel<<<kLongBlocks, kLongThreads, 0, sw>>>(Lb, Lo, J.b, J.o, J.pip_type, J.pip_flag, J.join_flag,
+                                                           lpPip); note_launch(); }
   join_aux();
   mk->mark("join:cmbr+pip", s);
   // ---- J5 common-MBR edge filter: count, offsets, lists
@@ -1027,10 +1275,13 @@ int join_from_keys(const LayerDev& Lb, const LayerDev& Lo, const uint64_t* pkeys
     fork_aux();
     { (f32 ? cmf_kernel<0, kJoinTile, 1> : cmf_kernel<0, kJoinTile, 0>)<<<blocks_for_tiles(K, kJoinTile), kThreads, 0, s>>>(
           Lb, Lo, J.b, J.o, J.cmbr, K, J.join_flag, J.bE, J.oE, nullptr, nullptr, nullptr, nullptr, -1,
-          kJoinTileMax); note_launch(); }
+          kJoinTileMax, LongPairs{}); note_launch(); }
     { (f32 ? cmf_kernel<0, 32, 1> : cmf_kernel<0, 32, 0>)<<<blocks_for_warps(K), kThreads, 0, sw>>>(Lb, Lo, J.b, J.o, J.cmbr, K, J.join_flag, J.bE,
                                                                 J.oE, nullptr, nullptr, nullptr, nullptr, kJoinTileMax,
-                                                                INT64_MAX); note_launch(); }
+                                                                hiRing, lpCmf); note_launch(); }
+    if (longCmf)
+      { (f32 ? cmf_long_kernel<0, 1> : cmf_long_kernel<0, 0>)<<<kLongBlocks, kLongThreads, 0, sw>>>(
+            Lb, Lo, J.b, J.o, J.cmbr, J.join_flag, J.bE, J.oE, CmfOut{}, lpCmf); note_launch(); }
     join_aux();
     exclusive_scan_i32(J.bE, bOff, K, d_total + 1, stmpK, d_err, s);
     exclusive_scan_i32(J.oE, oOff, K, d_total + 2, stmpK, d_err, s);
@@ -1043,10 +1294,13 @@ int join_from_keys(const LayerDev& Lb, const LayerDev& Lo, const uint64_t* pkeys
     J.n_blist = nBl; J.n_olist = nOl;
     fork_aux();
     { (f32 ? cmf_kernel<1, kJoinTile, 1> : cmf_kernel<1, kJoinTile, 0>)<<<blocks_for_tiles(K, kJoinTile), kThreads, 0, s>>>(
-          Lb, Lo, J.b, J.o, J.cmbr, K, J.join_flag, J.bE, J.oE, bOff, oOff, bList, oList, -1, kJoinTileMax); note_launch(); }
+          Lb, Lo, J.b, J.o, J.cmbr, K, J.join_flag, J.bE, J.oE, bOff, oOff, bList, oList, -1, kJoinTileMax, LongPairs{}); note_launch(); }
     { (f32 ? cmf_kernel<1, 32, 1> : cmf_kernel<1, 32, 0>)<<<blocks_for_warps(K), kThreads, 0, sw>>>(Lb, Lo, J.b, J.o, J.cmbr, K, J.join_flag, J.bE,
                                                                 J.oE, bOff, oOff, bList, oList, kJoinTileMax,
-                                                                INT64_MAX); note_launch(); }
+                                                                hiRing, LongPairs{}); note_launch(); }
+    if (longCmf)
+      { (f32 ? cmf_long_kernel<1, 1> : cmf_long_kernel<1, 0>)<<<kLongBlocks, kLongThreads, 0, sw>>>(
+            Lb, Lo, J.b, J.o, J.cmbr, J.join_flag, J.bE, J.oE, CmfOut{bOff, oOff, bList, oList, nBl, nOl, nullptr}, lpCmf); note_launch(); }
     join_aux();
   } else {
     // one pass (cmf_append_kernel) into lists sized from the last join's totals, or a
@@ -1060,11 +1314,15 @@ int join_from_keys(const LayerDev& Lb, const LayerDev& Lo, const uint64_t* pkeys
       if (!bList || !oList) return ST_OUT_OF_MEMORY;
       out.bList = bList; out.oList = oList;
       cudaMemsetAsync(d_total + 1, 0, 2 * sizeof(int64_t), s);
+      if (longCmf) cudaMemsetAsync(lpCmf.n, 0, sizeof(unsigned), s);
       fork_aux();
       { (f32 ? cmf_append_kernel<kJoinTile, 1> : cmf_append_kernel<kJoinTile, 0>)<<<blocks_for_tiles(K, kJoinTile), kThreads, 0, s>>>(
-            Lb, Lo, J.b, J.o, J.cmbr, K, J.join_flag, J.bE, J.oE, out, -1, kJoinTileMax); note_launch(); }
+            Lb, Lo, J.b, J.o, J.cmbr, K, J.join_flag, J.bE, J.oE, out, -1, kJoinTileMax, LongPairs{}); note_launch(); }
       { (f32 ? cmf_append_kernel<32, 1> : cmf_append_kernel<32, 0>)<<<blocks_for_warps(K), kThreads, 0, sw>>>(
-            Lb, Lo, J.b, J.o, J.cmbr, K, J.join_flag, J.bE, J.oE, out, kJoinTileMax, INT64_MAX); note_launch(); }
+            Lb, Lo, J.b, J.o, J.cmbr, K, J.join_flag, J.bE, J.oE, out, kJoinTileMax, hiRing, lpCmf); note_launch(); }
+      if (longCmf)
+        { (f32 ? cmf_long_kernel<2, 1> : cmf_long_kernel<2, 0>)<<<kLongBlocks, kLongThreads, 0, sw>>>(
+              Lb, Lo, J.b, J.o, J.cmbr, J.join_flag, J.bE, J.oE, out, lpCmf); note_launch(); }
       join_aux();
       cudaMemcpyAsync(h_scratch, d_total + 1, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
       if (cudaStreamSynchronize(s) != cudaSuccess) return ST_CUDA_ERROR;
@@ -1079,10 +1337,13 @@ int join_from_keys(const LayerDev& Lb, const LayerDev& Lo, const uint64_t* pkeys
   fork_aux();
   { refine_kernel<kJoinTile><<<blocks_for_tiles(K, kJoinTile), kThreads, 0, s>>>(
         Lb, Lo, J.b, J.o, K, J.join_flag, J.bE, J.oE, bOff, oOff, bList, oList, J.seg_flag, -1,
-        kJoinTileMax * 4); note_launch(); }
+        kJoinTileMax * 4, LongPairs{}); note_launch(); }
   { refine_kernel<32><<<blocks_for_warps(K), kThreads, 0, sw>>>(Lb, Lo, J.b, J.o, K, J.join_flag, J.bE, J.oE,
                                                               bOff, oOff, bList, oList, J.seg_flag, kJoinTileMax * 4,
-                                                              INT64_MAX); note_launch(); }
+                                                              longGrid ? kJoinGridMax : INT64_MAX, lpGrid); note_launch(); }
+  if (longGrid)
+    { refine_long_kernel<<<kLongBlocks, kLongThreads, 0, sw>>>(Lb, Lo, J.b, J.o, J.bE, J.oE, bOff, oOff, bList, oList,
+                                                              J.seg_flag, lpGrid); note_launch(); }
   join_aux();
   mk->mark("join:refine", s);
   // ---- clip set = containment pairs + pairs with intersecting edges

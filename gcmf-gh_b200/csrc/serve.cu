@@ -283,9 +283,10 @@ int gcmfgh_server::run_batch(std::vector<std::shared_ptr<Request>>& batch, int64
       prm.exact = opt.exact ? 1 : 0;
       prm.tile_label_max = default_tile_label(J.n_clip);
       // the clip's edge filter takes the join's common-MBR edge lists of the clip set
-      const JoinEdges je{J.clip_cand, J.join_flag, J.bE, J.oE, J.bOff, J.oOff, J.bList, J.oList};
+      // and the MBRs of the queries and of the resident layer
+      const JoinEdges je{J.clip_cand, J.join_flag, J.bE, J.oE, J.bOff, J.oOff, J.bList, J.oList, J.max_ring};
       st = run_clip(Lq, resident(), J.clip_b, J.clip_o, J.n_clip, prm, C, CD, d_err, h_scratch, s, nullptr, aux,
-                    nullptr, nullptr, nullptr, nullptr, &je);
+                    nullptr, nullptr, J.mbr_b, J.mbr_o, &je);
       if (st != ST_OK) return st;
     }
   } else {
