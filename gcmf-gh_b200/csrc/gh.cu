@@ -1005,10 +1005,11 @@ __global__ void pair_ring_kernel(const int64_t* __restrict__ eoff, const int64_t
 // ---------------------------------------------------------------- G5 ring fill
 // Thread per edge: the edge's source vertex, then its inserted vertices sorted by
 // (parameter ascending, other edge descending).  side 0 fills P rings, side 1 Q rings.
-// An edge of the smaller polygon can cross thousands of edges of a large one; edges with
-// more than kLightEdge insertions are left to heavy_fill_kernel, which sorts them with a
-// block-wide bitonic network.
-constexpr int kLightEdge = 32;
+// An edge of the smaller polygon can cross thousands of edges of a large one: edges with
+// more than kLightEdge insertions are listed for mid_fill_kernel (a warp each), those with more than
+// kMidEdge for heavy_fill_kernel (a block each).
+constexpr int kLightEdge = 8;
+constexpr int kMidEdge = 512;
 
 struct EdgeFill {
   int64_t k, base;
@@ -1073,6 +1074,7 @@ __global__ void __launch_bounds__(kThreads, 4) ring_fill_kernel(LayerDev Lb, Lay
                                  const int64_t* __restrict__ insCursorBase, int32_t* __restrict__ insCursor,
                                  const int64_t* __restrict__ insList, int64_t* __restrict__ heavy,
                                  unsigned long long* __restrict__ nHeavy) {
+  // heavy: the mid edges from the front (nHeavy[1]), the heavy ones from the back (nHeavy[0])
   int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   if (e >= nE) return;
   EdgeFill f;
@@ -1087,7 +1089,8 @@ __global__ void __launch_bounds__(kThreads, 4) ring_fill_kernel(LayerDev Lb, Lay
   const int64_t l0 = insCursorBase[e];
   const int cnt = insCursor[e];
   if (cnt > kLightEdge) {
-    heavy[atomicAdd(nHeavy, 1ull)] = e;
+    if (cnt > kMidEdge) heavy[nE - 1 - (int64_t)atomicAdd(nHeavy, 1ull)] = e;
+    else heavy[atomicAdd(nHeavy + 1, 1ull)] = e;
     return;
   }
   // insertion sort of the (few) records by (parameter asc, other edge desc)
@@ -1109,6 +1112,89 @@ __global__ void __launch_bounds__(kThreads, 4) ring_fill_kernel(LayerDev Lb, Lay
     lst[j + 1] = r;
   }
   for (int i = 0; i < cnt; ++i) write_inserted<kSide>(f, R, lst[i], i, S, slotOfRec);
+}
+
+// A warp per mid edge: the records' (parameter bits, ~other edge) sorted in the warp's part of
+// shared memory, up to 32 by counting each record's predecessors with shuffles, more with
+// a bitonic network; then the vertices are written in order.  A block per edge beyond 32
+// insertions (512 threads over 64 elements, a barrier per step) took 2.8 of the fill's 4.0 ms on
+// 2,500 degenerate pairs, and most of 16 ms on the large pair, whose edges all have 70 to 140.
+constexpr int kMidThreads = 128;
+
+template <int kSide>
+__global__ void __launch_bounds__(kMidThreads)
+mid_fill_kernel(LayerDev Lb, LayerDev Lo, PairDev D, Records R, const int64_t* __restrict__ eoff,
+                const int32_t* __restrict__ edgePair,
+                const int64_t* __restrict__ vpos, const int64_t* __restrict__ regOff,
+                const int32_t* __restrict__ m, RingSet S, int64_t* __restrict__ slotOfRec,
+                const int64_t* __restrict__ insCursorBase, const int32_t* __restrict__ insCursor,
+                const int64_t* __restrict__ insList, const int64_t* __restrict__ mid,
+                const unsigned long long* __restrict__ nMid) {
+  __shared__ uint64_t skey[kMidThreads / 32][kMidEdge];
+  __shared__ uint32_t stie[kMidThreads / 32][kMidEdge];
+  __shared__ uint16_t sidx[kMidThreads / 32][kMidEdge];
+  const int lane = (int)lane_id(), warp = (int)(threadIdx.x >> 5);
+  uint64_t* key = skey[warp];
+  uint32_t* tie = stie[warp];
+  uint16_t* idx = sidx[warp];
+  const unsigned long long n = *nMid;
+  for (unsigned long long h = (unsigned long long)blockIdx.x * (kMidThreads / 32) + warp; h < n;
+       h += (unsigned long long)gridDim.x * (kMidThreads / 32)) {
+    const int64_t e = mid[h];
+    EdgeFill f;
+    edge_fill_info<kSide>(Lb, Lo, D, eoff, edgePair, vpos, regOff, m, e, f);
+    const int64_t l0 = insCursorBase[e];
+    const int cnt = insCursor[e];
+    if (cnt <= 32) {
+      int64_t r = 0;
+      uint64_t k = ~0ull;
+      uint32_t t = ~0u;
+      if (lane < cnt) {
+        r = insList[l0 + lane];
+        k = ordered_key(kSide == 0 ? R.a[r] : R.b[r]);
+        t = 0xffffffffu - (uint32_t)(kSide == 0 ? R.q[r] : R.p[r]);
+      }
+      int rank = 0;
+      for (int j = 0; j < cnt; ++j) {
+        const uint64_t kj = __shfl_sync(0xffffffffu, k, j);
+        const uint32_t tj = __shfl_sync(0xffffffffu, t, j);
+        rank += (kj < k || (kj == k && tj < t)) ? 1 : 0;
+      }
+      if (lane < cnt) write_inserted<kSide>(f, R, r, rank, S, slotOfRec);
+      continue;
+    }
+    int npad = 64;
+    while (npad < cnt) npad <<= 1;
+    for (int i = lane; i < npad; i += 32) {
+      key[i] = ~0ull;
+      tie[i] = 0xffffffffu;
+      idx[i] = (uint16_t)i;
+      if (i < cnt) {
+        const int64_t r = insList[l0 + i];
+        key[i] = ordered_key(kSide == 0 ? R.a[r] : R.b[r]);
+        tie[i] = 0xffffffffu - (uint32_t)(kSide == 0 ? R.q[r] : R.p[r]);
+      }
+    }
+    __syncwarp();
+    for (int size = 2; size <= npad; size <<= 1)
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (int i = lane; i < (npad >> 1); i += 32) {
+          const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
+          const uint64_t ka = key[lo], kb = key[hi];
+          const uint32_t ta = tie[lo], tb = tie[hi];
+          if (((ka > kb) || (ka == kb && ta > tb)) == ((lo & size) == 0)) {
+            key[lo] = kb; key[hi] = ka;
+            tie[lo] = tb; tie[hi] = ta;
+            const uint16_t x = idx[lo];
+            idx[lo] = idx[hi];
+            idx[hi] = x;
+          }
+        }
+        __syncwarp();
+      }
+    for (int i = lane; i < cnt; i += 32) write_inserted<kSide>(f, R, insList[l0 + idx[i]], i, S, slotOfRec);
+    __syncwarp();
+  }
 }
 
 // Block per heavy edge: bitonic sort of (parameter bits, ~other edge, list position) --
@@ -1145,7 +1231,7 @@ heavy_fill_kernel(LayerDev Lb, LayerDev Lo, PairDev D, Records R, const int64_t*
                   const int64_t* __restrict__ vpos, const int64_t* __restrict__ regOff,
                   const int32_t* __restrict__ m, RingSet S, int64_t* __restrict__ slotOfRec,
                   const int64_t* __restrict__ insCursorBase, const int32_t* __restrict__ insCursor,
-                  const int64_t* __restrict__ insList, const int64_t* __restrict__ heavy,
+                  const int64_t* __restrict__ insList, const int64_t* __restrict__ heavy, int64_t nE,
                   const unsigned long long* __restrict__ nHeavy, uint64_t* gkey, uint32_t* gtie, uint32_t* gidx) {
   extern __shared__ unsigned char smem[];
   uint64_t* skey = reinterpret_cast<uint64_t*>(smem);
@@ -1154,7 +1240,7 @@ heavy_fill_kernel(LayerDev Lb, LayerDev Lo, PairDev D, Records R, const int64_t*
   __shared__ EdgeFill f;
   const unsigned long long nh = *nHeavy;
   for (unsigned long long h = blockIdx.x; h < nh; h += gridDim.x) {
-    const int64_t e = heavy[h];
+    const int64_t e = heavy[nE - 1 - (int64_t)h];
     if (threadIdx.x == 0) edge_fill_info<kSide>(Lb, Lo, D, eoff, edgePair, vpos, regOff, m, e, f);
     __syncthreads();
     const int64_t l0 = insCursorBase[e];
@@ -1551,11 +1637,14 @@ __device__ void seq_step1(PairCtx& c) {
   }
 }
 
-// step 2: intersection chains (polyclip.h:405-451)
-__device__ void seq_step2(PairCtx& c) {
+// step 2: intersection chains (polyclip.h:405-451).  n >= 0: the chain starts are among the n
+// slots listed in P.ls, in order
+__device__ void seq_step2(PairCtx& c, int n = -1) {
   Ring& P = c.R[0];
   Ring& Q = c.R[1];
-  for (int s = 0; s < P.m; ++s) {
+  const int count = n < 0 ? P.m : n;
+  for (int i = 0; i < count; ++i) {
+    const int s = n < 0 ? i : P.ls(i);
     if (!P.it(s) || (P.lb(s) != L_LEFT_ON && P.lb(s) != L_RIGHT_ON)) continue;
     int x = P.lb(s) == L_LEFT_ON ? R_LEFT : R_RIGHT;
     int X = s, I = s, guard = P.m + 1;
@@ -2235,6 +2324,30 @@ __device__ void grp_step1(const G& g, PairCtx& c) {
   g.sync();
 }
 
+// Step 1 for links that are not one-to-one: of the P vertices linked to one Q vertex the
+// last one with a label gives it to that vertex, as in the sequential loop.
+template <int EX, class G>
+__device__ void grp_step1_shared(const G& g, PairCtx& c) {
+  Ring& P = c.R[0];
+  Ring& Q = c.R[1];
+  for (int s = g.rank(); s < Q.m; s += g.size()) Q.tn(s) = -1;
+  g.sync();
+  for (int s = g.rank(); s < P.m; s += g.size()) {
+    const int nb = P.it(s) ? P.nb(s) : -1;
+    if (nb < 0) continue;
+    const int pm = (s > 0) ? s - 1 : P.m - 1, pp = (s + 1 < P.m) ? s + 1 : 0;
+    const int8_t L = initial_label(rel_position<EX>(P, Q, (nb > 0) ? nb - 1 : Q.m - 1, pm, s, pp),
+                                   rel_position<EX>(P, Q, (nb + 1 < Q.m) ? nb + 1 : 0, pm, s, pp));
+    if (L != L_NONE) { P.lb(s) = L; atomicMax(&Q.tn(nb), s); }
+  }
+  g.sync();
+  for (int s = g.rank(); s < P.m; s += g.size()) {
+    const int nb = P.it(s) ? P.nb(s) : -1;
+    if (nb >= 0 && P.lb(s) != L_NONE && Q.tn(nb) == s) Q.lb(nb) = P.lb(s);
+  }
+  g.sync();
+}
+
 // Chains run from a LEFT_ON/RIGHT_ON vertex over ON_ON vertices to an ON_LEFT/ON_RIGHT
 // vertex.  When every chain ends so, chains are disjoint and can be resolved in parallel
 // with the sequential result; otherwise returns false and nothing is changed.
@@ -2783,18 +2896,56 @@ __device__ int grp_trace_loops(const G& g, PairCtx& c) {
   g.sync();
   if (g.any(bad)) return 1;
   odd = g.any(odd);
-  for (int t = g.rank(); t < n; t += g.size())           // the same links both ways
+  bool lop = false;                                      // links that differ by direction
+  for (int t = g.rank(); t < n; t += g.size())
     for (int e = 0; e < 2; ++e) {
       const int l = link(t, e);
-      if (link(l >> 1, l & 1) != 2 * t + e) bad = true;
+      if (link(l >> 1, l & 1) != 2 * t + e) lop = true;
     }
-  g.sync();
-  if (g.any(bad)) return 1;
-  if (g.any(beside)) {
-    // A crossing of P beside a segment's end: no loop passes it (where segments are
-    // entered at their ends only), so the walk starts there, runs into a loop and never
-    // comes back to it.
-    if (odd) return 1;
+  if (g.any(lop || beside)) {
+    // The walk may run into a loop that it did not start on, and never close.  Take the walk
+    // that entered t at end e as a state: every state has one successor, so beyond the
+    // tails the states form cycles, and walks that close go round one of them.  A crossing
+    // of P that no cycle passes is therefore met by no closed walk; it will start one that
+    // does not close, and the pair fails.  Otherwise the general walk decides.
+    int32_t* deg[2] = {eV, lead};                        // predecessors of the state
+    int32_t* way[2] = {&P.nx(0), &P.nx(mP >> 1)};        // the cycle's way into the segment, from its entry to its end
+    for (int t = g.rank(); t < n; t += g.size())
+      for (int e = 0; e < 2; ++e) { deg[e][t] = 0; way[e][t] = 0; }
+    g.sync();
+    for (int t = g.rank(); t < n; t += g.size())
+      for (int e = 0; e < 2; ++e) { const int l = link(t, e); atomicAdd(&deg[l & 1][l >> 1], 1); }
+    g.sync();
+    for (int t = g.rank(); t < n; t += g.size())
+      for (int e = 0; e < 2; ++e) if (deg[e][t] == 0) way[e][t] = -1;
+    g.sync();
+    for (int t = g.rank(); t < n; t += g.size())         // peel the tails from their first states on
+      for (int e = 0; e < 2; ++e) {
+        if (way[e][t] != -1) continue;
+        int l = link(t, 1 - e);
+        while (atomicSub(&deg[l & 1][l >> 1], 1) == 1) l = link(l >> 1, 1 - (l & 1));
+      }
+    g.sync();
+    auto way_in = [&](int s, int t, int e) { return e ? dist(end_p(t, 0), s, mP) : dist(s, end_p(t, 1), mP); };
+    for (int t = g.rank(); t < n; t += g.size())
+      for (int e = 0; e < 2; ++e) {
+        if (deg[e][t] <= 0) continue;
+        const int q = P.nb(end_p(t, 1 - e)), l = link(t, 1 - e);
+        way[l & 1][l >> 1] = way_in(Q.nb(end_q(seg_q(q), fwd_at(Q, q) ? 1 : 0)), l >> 1, l & 1);
+      }
+    g.sync();
+    bool never = false;
+    for (int f = g.rank(); f < nFP; f += g.size()) {
+      const int s = P.ls(f);
+      if (!cross_at(P, s)) continue;
+      const int t = seg_p(s), e = fwd_at(P, s) ? 0 : 1;
+      const bool passed = s == end_p(t, e) ? deg[0][t] > 0 || deg[1][t] > 0 : deg[e][t] > 0 && way[e][t] >= way_in(s, t, e);
+      if (!passed) never = true;
+    }
+    never = g.any(never);
+    for (int s = g.rank(); s < mP; s += g.size()) P.nx(s) = s + 1 < mP ? s + 1 : 0;
+    g.sync();
+    if (!never) return 1;
     if (g.rank() == 0) fail(c, DEV_TRACE);
     return -1;
   }
@@ -3302,9 +3453,25 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
     }
     g.sync();
   };
-  if (!grp_links_one_to_one(g, c.R[0], c.R[1])) { sequential(1); return; }
-  grp_step1<EX>(g, c);
-  if (!grp_step2(g, c)) { sequential(2); return; }
+  const bool oneToOne = grp_links_one_to_one(g, c.R[0], c.R[1]);
+  if constexpr (G::kSolo) {
+    if (!oneToOne) { sequential(1); return; }
+    grp_step1<EX>(g, c);
+    if (!grp_step2(g, c)) { sequential(2); return; }
+  } else {
+    // Links that are not one-to-one and malformed chains leave only the chains' resolution
+    // (over the listed chain starts) and, for the former, the trace to one member.
+    if (oneToOne) grp_step1<EX>(g, c);
+    else grp_step1_shared<EX>(g, c);
+    if (!oneToOne || !grp_step2(g, c)) {
+      Ring& P = c.R[0];
+      const int n = g.list(P.m, [&](int s) { return P.it(s) && (P.lb(s) == L_LEFT_ON || P.lb(s) == L_RIGHT_ON); },
+                           [&](int s, bool hit, int before) { if (hit) P.ls(before) = s; });
+      g.sync();
+      if (lead) seq_step2(c, n);
+      g.sync();
+    }
+  }
   grp_step35<EX>(g, c);
   int tempAfter[2], tempSlot[2];
   if (!grp_step4<EX>(g, c, tempAfter, tempSlot)) return;
@@ -3326,10 +3493,10 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
   grp_step6(g, c);
   bool added = c.R[0].used != c.R[0].m || c.R[1].used != c.R[1].m;
   if constexpr (!G::kSolo) {
-    if (added) added = !grp_linearize(g, c);
+    if (added && oneToOne) added = !grp_linearize(g, c);
   }
-  if (added) {
-    // vertices were added to a ring: trace through the next/prev links on one member
+  if (added || !oneToOne) {
+    // trace through the next/prev links on one member
     if constexpr (G::kGrid) { sequential(3); return; }
     int ok = 1;
     if (lead) ok = seq_trace(c) ? 1 : 0;
@@ -4031,9 +4198,10 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    unsigned long long* nHeavy = A.take_n<unsigned long long>(2);
+    unsigned long long* nHeavy = A.take_n<unsigned long long>(4);     // [heavy, mid] of P, of Q
     if (!nHeavy) return ST_OUT_OF_MEMORY;
-    cudaMemsetAsync(nHeavy, 0, 2 * sizeof(unsigned long long), s);
+    cudaMemsetAsync(nHeavy, 0, 4 * sizeof(unsigned long long), s);
+    const unsigned midBlocks = 8 * (unsigned)nsm;
     cudaStream_t sq = s;
     cudaEvent_t fork = nullptr, join = nullptr;
     if (aux && cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
@@ -4058,16 +4226,20 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
         { ring_fill_kernel<0><<<blocks_for(nEP), kThreads, 0, ss>>>(Lb, Lo, D, R, eoffP, nEP, edgePair, vposP, regP, mP,
                                                                   SP, slotP, insBaseP, curP, insListP, heavy,
                                                                   nHeavy); note_launch(); }
+        { mid_fill_kernel<0><<<midBlocks, kMidThreads, 0, ss>>>(Lb, Lo, D, R, eoffP, edgePair, vposP, regP, mP, SP, slotP,
+                                                              insBaseP, curP, insListP, heavy, nHeavy + 1); note_launch(); }
         { heavy_fill_kernel<0><<<2 * nsm, kHeavyThreads, smem, ss>>>(Lb, Lo, D, R, eoffP, edgePair, vposP, regP, mP, SP,
-                                                                     slotP, insBaseP, curP, insListP, heavy, nHeavy,
+                                                                     slotP, insBaseP, curP, insListP, heavy, nEP, nHeavy,
                                                                      gkey, gtie, gidx); note_launch(); }
       } else {
         { range_owner_kernel<<<blocks_for_warps(K), kThreads, 0, ss>>>(eoffQ, D.nQ, K, edgePair); note_launch(); }
         { ring_fill_kernel<1><<<blocks_for(nEQ), kThreads, 0, ss>>>(Lb, Lo, D, R, eoffQ, nEQ, edgePair, vposQ, regQ, mQ,
                                                                   SQ, slotQ, insBaseQ, curQ, insListQ, heavy,
-                                                                  nHeavy + 1); note_launch(); }
+                                                                  nHeavy + 2); note_launch(); }
+        { mid_fill_kernel<1><<<midBlocks, kMidThreads, 0, ss>>>(Lb, Lo, D, R, eoffQ, edgePair, vposQ, regQ, mQ, SQ, slotQ,
+                                                              insBaseQ, curQ, insListQ, heavy, nHeavy + 2 + 1); note_launch(); }
         { heavy_fill_kernel<1><<<2 * nsm, kHeavyThreads, smem, ss>>>(Lb, Lo, D, R, eoffQ, edgePair, vposQ, regQ, mQ, SQ,
-                                                                     slotQ, insBaseQ, curQ, insListQ, heavy, nHeavy + 1,
+                                                                     slotQ, insBaseQ, curQ, insListQ, heavy, nEQ, nHeavy + 2,
                                                                      gkey, gtie, gidx); note_launch(); }
       }
     }
