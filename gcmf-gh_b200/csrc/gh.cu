@@ -2742,6 +2742,17 @@ struct LoopsShared {                                     // 12 bytes per segment
   __device__ __forceinline__ int w(int t, int e) const { return e ? (int)(raw(t) & ~kNoCrossing) : (int)p[n + t]; }
 };
 
+// The loops' nodes (long loops of the grid path): every kNodeEvery-th segment and the segments
+// that the bounded search left open, in this order; link and w lead from node to node.
+constexpr int kNodeEvery = 256;
+struct LoopsNodes {
+  const int32_t *l0, *l1, *w0, *w1;
+  int open;                                              // the first of the open segments
+  __device__ __forceinline__ int link(int i, int e) const { return (e ? l1 : l0)[i]; }
+  __device__ __forceinline__ unsigned raw(int i) const { return i < open ? kNoCrossing : 0u; }
+  __device__ __forceinline__ int w(int i, int e) const { return (e ? w1 : w0)[i]; }
+};
+
 // The size of t's loop when t is its smallest segment with a crossing, else 0 (-1: the walk
 // did not close within guard steps).  The walk goes both ways at once and stops at the
 // first smaller segment: over a loop of L segments the searches take O(L log L) steps in
@@ -2966,9 +2977,20 @@ __device__ int grp_trace_loops(const G& g, PairCtx& c) {
     return r;
   };
   // ---- the loops' smallest segments and sizes
+  // The grid bounds the search: a loop of 50,000 segments would keep one thread walking for
+  // 18 ms, twice.  Segments that are smallest within kNodeEvery steps both ways stay open and
+  // are nodes, with every kNodeEvery-th segment; all nodes walk to their neighbours, and
+  // the open ones are decided over the nodes.
+  int nOpen = 0;
+  const int nEvery = (n + kNodeEvery - 1) / kNodeEvery;
+  int32_t* node = &Q.to(0);                              // segment -> its node, -1 none (the slot map is done with)
+  int32_t* nodeT = &Q.nx(0);
+  int32_t* nodeOff = &Q.pv(0);
+  const LoopsNodes nodes{&P.nx(0), &P.nx(mP >> 1), &P.pv(0), &P.pv(mP >> 1), nEvery};
+  const bool bounded = G::kGrid && !odd;
   for (int t = g.rank(); t < n; t += g.size()) {
-    int sz = shared ? loop_size(shrd, t, n + 2) : loop_size(glob, t, n + 2);
-    if (sz < 0) { bad = true; sz = 0; }
+    int sz = shared ? loop_size(shrd, t, n + 2) : loop_size(glob, t, bounded ? 2 * kNodeEvery : n + 2);
+    if (sz < 0 && !bounded) { bad = true; sz = 0; }
     if (odd && sz > 0) {                                 // the pieces depend on the direction: walk them
       const int in0 = start_end(t), I = end_p(t, in0);
       int u = t, in = in0, v = I;
@@ -2987,6 +3009,45 @@ __device__ int grp_trace_loops(const G& g, PairCtx& c) {
   }
   g.sync();
   if (g.any(bad)) return 1;
+  if constexpr (G::kGrid) {
+    if (bounded) {
+      nOpen = g.list(n, [&](int t) { return off[t] < 0; },
+                     [&](int t, bool hit, int before) {
+                       node[t] = hit ? nEvery + before : (t % kNodeEvery == 0 ? t / kNodeEvery : -1);
+                       if (hit) { nodeT[nEvery + before] = t; off[t] = 0; }
+                     });
+      g.sync();
+    }
+    if (nOpen > 0) {
+      for (int i = g.rank(); i < nEvery + nOpen; i += g.size()) {
+        const int t = i < nEvery ? i * kNodeEvery : nodeT[i];
+        if (i < nEvery) nodeT[i] = t;
+        nodeOff[i] = INT_MIN;
+        if (node[t] != i) continue;                      // an open one
+        for (int e = 0; e < 2; ++e) {
+          int u = t, out = e, l, to, sum = 0, left = n + 1;
+          do {
+            sum += glob.w(u, out);
+            l = glob.link(u, out);
+            u = l >> 1;
+            out = 1 - (l & 1);
+            to = node[u];
+          } while (to < 0 && --left > 0);
+          if (to < 0) { bad = true; to = i; }
+          const_cast<int32_t*>(e ? nodes.l1 : nodes.l0)[i] = 2 * to + (l & 1);
+          const_cast<int32_t*>(e ? nodes.w1 : nodes.w0)[i] = sum;
+        }
+      }
+      g.sync();
+      for (int i = nEvery + g.rank(); i < nEvery + nOpen; i += g.size()) {
+        const int sz = loop_size(nodes, i, nEvery + nOpen + 2);
+        if (sz < 0) bad = true;
+        off[nodeT[i]] = sz;
+      }
+      g.sync();
+    }
+    if (g.any(bad)) { if (g.rank() == 0) fail(c, DEV_TRACE); return -1; }
+  }
   OutRegion& O = c.O;
   int32_t* csz = O.csz + O.nc;
   const int room = O.ccap - O.nc;
@@ -3028,11 +3089,31 @@ __device__ int grp_trace_loops(const G& g, PairCtx& c) {
       } while (u != t0);
     } else if (shared) {
       loop_offsets(shrd, t0, in0, base, csz[k], off);
+    } else if (nOpen > 0 && node[t0] >= nEvery) {
+      loop_offsets(nodes, node[t0], in0, base, csz[k], nodeOff);
     } else {
       loop_offsets(glob, t0, in0, base, csz[k], off);
     }
   }
   g.sync();
+  if constexpr (G::kGrid) {
+    if (nOpen > 0) {                                     // from each node on to the next one
+      for (int i = g.rank(); i < nEvery + nOpen; i += g.size()) {
+        int o = nodeOff[i];
+        if (o == INT_MIN) continue;
+        int in = o < 0 ? 1 : 0, u = nodeT[i];
+        if (in) o = ~o;
+        do {
+          off[u] = in ? ~o : o;
+          o += glob.w(u, 1 - in);
+          const int l = glob.link(u, 1 - in);
+          u = l >> 1;
+          in = l & 1;
+        } while (node[u] < 0);
+      }
+      g.sync();
+    }
+  }
   // ---- copy the pieces
   double2* out = reinterpret_cast<double2*>(O.xy) + O.nv;
   for (int b = 0; b < n; b += g.size()) {
