@@ -164,7 +164,7 @@ GCMFGH_DEV void two_prod(double a, double b, double& p, double& e) {
 }
 
 GCMFGH_DEV int exact_sign_slow(double a1, double a0, double b1, double b0, double c1, double c0,
-                                            double d1, double d0, int sub) {
+                                           double d1, double d0, int sub) {
   double ah, al, bh, bl, ch, cl, dh, dl;
   two_sum(a1, -a0, ah, al);
   two_sum(b1, -b0, bh, bl);
@@ -297,7 +297,7 @@ GCMFGH_DEV int classify_exact(double p1x, double p1y, double p2x, double p2y,
 
 // classify_exact from both sides, out of line: for the edge pairs that classify_exact_both's
 // filter leaves open.
-__device__ __noinline__ int classify_exact_open(double2 P1, double2 P2, double2 Q1, double2 Q2, double2* ab, bool* qhit);
+__device__ int classify_exact_open(double2 P1, double2 P2, double2 Q1, double2 Q2, double2* ab, bool* qhit);
 
 // classify_exact of (P, Q) and whether classify_exact of (Q, P) finds an intersection.  When
 // the four areas' FP64 values decide their signs (the bound of exact_sign) and none is zero,

@@ -383,7 +383,7 @@ struct FusedRecords {
 };
 
 template <int kExact, int kWarpAppend>
-__global__ void __launch_bounds__(kThreads, kExact ? 2 : 4)
+__global__ void __launch_bounds__(kThreads, kExact ? 3 : 4)   // (the open cases' function takes 80 registers)
 intersect_fused_kernel(LayerDev Lb, LayerDev Lo, PairDev D, const int64_t* __restrict__ chunkOff, int64_t nChunks,
                        const int32_t* __restrict__ cP, const int32_t* __restrict__ cQ,
                        const int64_t* __restrict__ offP, const int64_t* __restrict__ offQ,
@@ -433,9 +433,9 @@ intersect_fused_kernel(LayerDev Lb, LayerDev Lo, PairDev D, const int64_t* __res
             tp = classify_edges_both(P1.x, P1.y, P2.x, P2.y, Q1.x, Q1.y, Q2.x, Q2.y, eps, alpha, beta, qhit);
             tq = qhit ? 1 : 0;
           } else {
-            double a2, b2;
-            tp = classify_mode(kExact, P1.x, P1.y, P2.x, P2.y, Q1.x, Q1.y, Q2.x, Q2.y, eps, alpha, beta);
-            tq = classify_mode(kExact, Q1.x, Q1.y, Q2.x, Q2.y, P1.x, P1.y, P2.x, P2.y, eps, a2, b2);
+            bool qhit;
+            tp = classify_exact_both(P1, P2, Q1, Q2, alpha, beta, qhit);
+            tq = qhit ? 1 : 0;
           }
         }
       }

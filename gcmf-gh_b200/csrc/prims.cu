@@ -218,6 +218,111 @@ radix_scatter_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restri
   }
 }
 
+// A pass in one kernel (for up to kSweepTiles tiles): every tile ranks its keys, publishes its
+// 256 digit counts and adds up those of the tiles before it by decoupled look-back, a thread
+// per digit with kSweepAhead predecessors in flight; the digits' totals of all passes come
+// from one histogram kernel in front.  Against histogram, scan and scatter kernels with a
+// clear in between: 29 -> 13 us per pass at 20,000 keys, 38 -> 26 us at 700,000.
+constexpr int64_t kSweepTiles = 512;
+constexpr int kSweepAhead = 16;
+constexpr int kSweepMaxPasses = 8;
+
+__global__ void __launch_bounds__(kRadixThreads)
+radix_hist_all_kernel(const uint64_t* __restrict__ keys, int64_t n, int passes, unsigned long long* __restrict__ hist) {
+  __shared__ unsigned cnt[kSweepMaxPasses * 256];
+  for (int i = threadIdx.x; i < passes * 256; i += kRadixThreads) cnt[i] = 0;
+  __syncthreads();
+  for (int64_t i = (int64_t)blockIdx.x * kRadixThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kRadixThreads) {
+    const uint64_t k = keys[i];
+    for (int p = 0; p < passes; ++p) atomicAdd(&cnt[p * 256 + (int)((k >> (8 * p)) & 0xff)], 1u);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < passes * 256; i += kRadixThreads)
+    if (cnt[i]) atomicAdd(&hist[i], (unsigned long long)cnt[i]);
+}
+
+__global__ void __launch_bounds__(kRadixThreads)
+radix_sweep_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals,
+                   uint64_t* __restrict__ okeys, uint32_t* __restrict__ ovals, int64_t n, int shift,
+                   const unsigned long long* __restrict__ hist, unsigned long long* __restrict__ status,
+                   unsigned* __restrict__ ticket, int* err) {
+  __shared__ int wcnt[kRadixWarps][256];
+  __shared__ int64_t offs[256];
+  __shared__ int64_t wtot[kRadixWarps];
+  __shared__ unsigned tile_s;
+  if (threadIdx.x == 0) tile_s = atomicAdd(ticket, 1u);
+  for (int k = threadIdx.x; k < kRadixWarps * 256; k += kRadixThreads) (&wcnt[0][0])[k] = 0;
+  __syncthreads();
+  const int64_t tile = tile_s;
+  const int w = threadIdx.x >> 5;
+  const unsigned lane = lane_id();
+  const int64_t wbase = tile * kRadixTile + (int64_t)w * 32 * kRadixRounds;
+  uint64_t key[kRadixRounds];
+  uint32_t val[kRadixRounds];
+  int rank[kRadixRounds], dig[kRadixRounds];
+#pragma unroll
+  for (int r = 0; r < kRadixRounds; ++r) {
+    const int64_t i = wbase + r * 32 + lane;
+    key[r] = i < n ? keys[i] : 0;
+    val[r] = i < n ? vals[i] : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < kRadixRounds; ++r) {
+    const bool ok = wbase + r * 32 + lane < n;
+    const int d = ok ? (int)((key[r] >> shift) & 0xff) : 256 + (int)lane;   // invalid lanes: unique
+    dig[r] = d;
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const int before = __popc(peers & lanemask_lt());
+    const int b = ok ? wcnt[w][d] : 0;
+    __syncwarp();
+    if (ok && before == 0) wcnt[w][d] = b + __popc(peers);
+    __syncwarp();
+    rank[r] = b + before;
+  }
+  __syncthreads();
+  {
+    const int d = threadIdx.x;
+    int run = 0;
+    for (int ww = 0; ww < kRadixWarps; ++ww) { const int t = wcnt[ww][d]; wcnt[ww][d] = run; run += t; }
+    atomicExch(&status[tile * 256 + d], (tile == 0 ? kFlagPrefix : kFlagAgg) | (unsigned long long)run);
+    // the digit's place among all keys
+    const int64_t total = (int64_t)hist[d], incl = warp_incl_scan(total);
+    if (lane == 31) wtot[w] = incl;
+    __syncthreads();
+    int64_t at = incl - total;
+    for (int ww = 0; ww < w; ++ww) at += wtot[ww];
+    // and among those of the tiles before
+    int64_t excl = 0;
+    long long spins = 0;
+    for (int64_t t = tile - 1; t >= 0;) {
+      unsigned long long word[kSweepAhead];
+#pragma unroll
+      for (int j = 0; j < kSweepAhead; ++j)
+        word[j] = t - j >= 0 ? *((volatile unsigned long long*)&status[(t - j) * 256 + d]) : kFlagPrefix;
+      bool done = false;
+#pragma unroll
+      for (int j = 0; j < kSweepAhead; ++j) {
+        if (done || t < 0) continue;
+        if ((word[j] >> 62) == 0) { done = true; continue; }               // not published yet: read again from here
+        excl += (int64_t)(word[j] & kValueMask);
+        if ((word[j] >> 62) == 2) t = -1;
+        else --t;
+      }
+      if (done && ++spins > kSpinLimit) { raise_error(err, DEV_TIMEOUT); break; }
+    }
+    if (tile > 0) atomicExch(&status[tile * 256 + d], kFlagPrefix | (unsigned long long)(excl + run));
+    offs[d] = at + excl;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kRadixRounds; ++r) {
+    if (wbase + r * 32 + lane < n) {
+      const int64_t pos = offs[dig[r]] + wcnt[w][dig[r]] + rank[r];
+      if (pos < n) { okeys[pos] = key[r]; ovals[pos] = val[r]; }           // (beyond it only after a wait gave up)
+    }
+  }
+}
+
 // Up to kSmallSort pairs in one block: a bitonic network over (key's low bits, place), which
 // makes the order that of a stable sort; then keys and values are written in that order.
 // Five launches per 8-bit pass otherwise: 85 us for the 24-bit pair keys of a join of 2,000 x
@@ -290,7 +395,9 @@ void exclusive_scan_u8(const uint8_t* in, int64_t* out, int64_t n, int64_t* tota
 size_t radix_temp_bytes(int64_t n) {
   int64_t nb = (n + kRadixTile - 1) / kRadixTile;
   int64_t h = 256 * nb;
-  return 2 * (size_t)h * sizeof(int64_t) + scan_temp_bytes(h) + 256;
+  const size_t three = 2 * (size_t)h * sizeof(int64_t) + scan_temp_bytes(h) + 256;
+  const size_t sweep = nb <= kSweepTiles ? sizeof(unsigned long long) * (kSweepMaxPasses * 257 + (size_t)kSweepMaxPasses * h) : 0;
+  return three > sweep ? three : sweep;
 }
 
 void radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt,
@@ -307,15 +414,31 @@ void radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32
   }
   int64_t nb = (n + kRadixTile - 1) / kRadixTile;
   int64_t h = 256 * nb;
-  int64_t* hist = reinterpret_cast<int64_t*>(tmp);
-  int64_t* offs = hist + h;
-  void* stmp = reinterpret_cast<char*>(offs + h);
   uint64_t* ka = keys;
   uint32_t* va = vals;
   uint64_t* kb = keys_alt;
   uint32_t* vb = vals_alt;
   int passes = (key_bits + 7) / 8;
-  for (int p = 0; p < passes; ++p) {
+  const bool sweep = nb <= kSweepTiles;
+  if (sweep) {
+    // [digit totals of every pass | tickets | status words of every pass], cleared at once
+    unsigned long long* totals = reinterpret_cast<unsigned long long*>(tmp);
+    unsigned* tickets = reinterpret_cast<unsigned*>(totals + kSweepMaxPasses * 256);
+    unsigned long long* status = totals + kSweepMaxPasses * 256 + kSweepMaxPasses;
+    cudaMemsetAsync(tmp, 0, sizeof(unsigned long long) * (kSweepMaxPasses * 257 + (size_t)passes * h), s);
+    const unsigned hb = (unsigned)(nb < 2 * 148 ? nb : 2 * 148);
+    { radix_hist_all_kernel<<<hb, kRadixThreads, 0, s>>>(keys, n, passes, totals); note_launch(); }
+    for (int p = 0; p < passes; ++p) {
+      { radix_sweep_kernel<<<(unsigned)nb, kRadixThreads, 0, s>>>(ka, va, kb, vb, n, 8 * p, totals + 256 * p, status + p * h,
+                                                                  tickets + p, err); note_launch(); }
+      uint64_t* tk = ka; ka = kb; kb = tk;
+      uint32_t* tv = va; va = vb; vb = tv;
+    }
+  }
+  int64_t* hist = reinterpret_cast<int64_t*>(tmp);
+  int64_t* offs = hist + h;
+  void* stmp = reinterpret_cast<char*>(offs + h);
+  for (int p = 0; p < passes && !sweep; ++p) {
     int shift = 8 * p;
     { radix_hist_kernel<<<(unsigned)nb, kRadixThreads, 0, s>>>(ka, n, shift, nb, hist); note_launch(); }
     exclusive_scan_i64(hist, offs, h, nullptr, stmp, err, s);
