@@ -648,6 +648,57 @@ __global__ void __launch_bounds__(32) multi_clip_batch_kernel(MultiArgs b, const
   multi_clip_pair(a);
 }
 
+// ---- the batch's layers.  A warp per ring: its vertices with the closing one, at `first`
+// plus one closing vertex per ring before it.
+__global__ void multi_ring_kernel(const double2* __restrict__ open, const int32_t* __restrict__ size,
+                                  const int64_t* __restrict__ first, int64_t nr, double2* __restrict__ xy,
+                                  int32_t* __restrict__ vnum, int64_t* __restrict__ vps, int64_t* __restrict__ start) {
+  const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= nr) return;
+  const int m = size[c];
+  const double2* from = open + first[c];
+  const int64_t at = first[c] + c;
+  for (int i = lane_id(); i <= m; i += 32) xy[at + i] = from[i < m ? i : 0];
+  if (lane_id() == 0) { vnum[c] = m + 1; vps[c] = at + m + 1; start[c] = at; }
+}
+
+// a warp per pair: its rings' first edges and their total, rings + 1 entries
+__global__ void multi_edge_kernel(const int32_t* __restrict__ size, const int64_t* __restrict__ first,
+                                  const int64_t* __restrict__ c0, const int32_t* __restrict__ rings, int64_t n,
+                                  int64_t* __restrict__ edge) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= n) return;
+  const int64_t c = c0[i], e = first[c];
+  const int k = rings[i];
+  for (int j = lane_id(); j < k; j += 32) edge[c + i + j] = first[c + j] - e;
+  if (lane_id() == 0) edge[c + i + k] = first[c + k - 1] + size[c + k - 1] - e;
+}
+
+// a warp per pair: the ids of its ring pairs
+__global__ void multi_ids_kernel(const int64_t* __restrict__ k0, const int64_t* __restrict__ cP,
+                                 const int64_t* __restrict__ cQ, const int32_t* __restrict__ ringsQ, int64_t n,
+                                 int32_t* __restrict__ pid, int32_t* __restrict__ qid) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= n) return;
+  const int64_t a = k0[i], b = k0[i + 1];
+  const int kq = ringsQ[i];
+  for (int64_t k = a + lane_id(); k < b; k += 32) {
+    pid[k] = (int32_t)(cP[i] + (k - a) / kq);
+    qid[k] = (int32_t)(cQ[i] + (k - a) % kq);
+  }
+}
+
+// a warp per pair: the records of its ring pairs
+__global__ void multi_count_kernel(const int64_t* __restrict__ count1, const int64_t* __restrict__ k0, int64_t n,
+                                   int64_t* __restrict__ count) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= n) return;
+  int64_t c = 0;
+  for (int64_t k = k0[i] + lane_id(); k < k0[i + 1]; k += 32) c += count1[k];
+  c = warp_sum(c);
+  if (lane_id() == 0) count[i] = c;
+}
+
 // per-pair result regions -> one contiguous result (a warp per pair)
 __global__ void multi_compact_kernel(const MultiPairDesc* __restrict__ desc, int64_t n,
                                      const int32_t* __restrict__ ocs, const double* __restrict__ oxy,
@@ -670,18 +721,17 @@ int run_clip_multi_batch(int64_t n, const double* hP, const int32_t* sizesP, con
   if (n <= 0 || !hP || !hQ || !sizesP || !sizesQ || !ringsP || !ringsQ) return ST_INVALID_ARGUMENT;
   auto sync = [&]() { return cudaStreamSynchronize(s) == cudaSuccess; };
   // ---- every ring of every pair as two layers (closing vertex stored); ring pairs of
-  // pair i are (P ring c, Q ring d) for its c, d, numbered i's k0 + c * kQ + d
+  // pair i are (P ring c, Q ring d) for its c, d, numbered i's k0 + c * kQ + d.  The host walks the
+  // sizes once; the caller's vertices and sizes go up as they are and the layers, edge
+  // offsets and ring pair ids are laid out on the device.
   const int32_t* rings[2] = {ringsP, ringsQ};
   const int32_t* sz[2] = {sizesP, sizesQ};
   const double* src[2] = {hP, hQ};
-  std::vector<int64_t> c0[2], e0[2], ne[2];
-  std::vector<double> hxy[2];
-  std::vector<int32_t> hvn[2];
-  std::vector<int64_t> hvp[2], hstart[2], hedge[2];
-  int64_t nring[2] = {0, 0};
+  std::vector<int64_t> c0[2], e0[2], ne[2], k0(n + 1);
+  int64_t nring[2] = {0, 0}, nvert[2] = {0, 0};
   for (int sd = 0; sd < 2; ++sd) {
     c0[sd].resize(n); e0[sd].resize(n); ne[sd].resize(n);
-    int64_t ring = 0, o = 0, v = 0, e = 0;
+    int64_t ring = 0, e = 0;
     for (int64_t i = 0; i < n; ++i) {
       if (rings[sd][i] < 1) return ST_INVALID_ARGUMENT;
       c0[sd][i] = ring;
@@ -690,60 +740,54 @@ int run_clip_multi_batch(int64_t n, const double* hP, const int32_t* sizesP, con
       for (int c = 0; c < rings[sd][i]; ++c, ++ring) {
         const int m = sz[sd][ring];
         if (m < 3) return ST_INVALID_ARGUMENT;
-        hstart[sd].push_back(v);
-        hedge[sd].push_back(le);
-        hxy[sd].insert(hxy[sd].end(), src[sd] + 2 * o, src[sd] + 2 * (o + m));
-        hxy[sd].push_back(src[sd][2 * o]);
-        hxy[sd].push_back(src[sd][2 * o + 1]);
-        o += m;
-        v += m + 1;
         le += m;
-        hvn[sd].push_back(m + 1);
-        hvp[sd].push_back(v);
       }
-      hedge[sd].push_back(le);            // pair i's local edge offsets: rings + 1 entries
       ne[sd][i] = le;
       e += le;
     }
     nring[sd] = ring;
+    nvert[sd] = e;
     if (ring > INT32_MAX) return ST_INVALID_ARGUMENT;
   }
-  std::vector<int64_t> k0(n + 1);
   k0[0] = 0;
   for (int64_t i = 0; i < n; ++i) k0[i + 1] = k0[i] + (int64_t)ringsP[i] * ringsQ[i];
   const int64_t K = k0[n];
-  std::vector<int32_t> hpid(K), hqid(K);
-  for (int64_t i = 0; i < n; ++i)
-    for (int64_t k = 0; k < k0[i + 1] - k0[i]; ++k) {
-      hpid[k0[i] + k] = (int32_t)(c0[0][i] + k / ringsQ[i]);
-      hqid[k0[i] + k] = (int32_t)(c0[1][i] + k % ringsQ[i]);
-    }
   double* dxy[2];
   int32_t* dvn[2];
-  int64_t *dvp[2], *dstart[2], *dedge[2];
-  int32_t* dsz[2];
+  int64_t *dvp[2], *dstart[2], *dedge[2], *dc0[2];
+  int32_t *dsz[2], *drings[2];
+  int64_t* dk0 = A.take_n<int64_t>(n + 1);
+  int32_t* dpid = A.take_n<int32_t>(K);
+  int32_t* dqid = A.take_n<int32_t>(K);
+  if (!dk0 || !dpid || !dqid) return ST_OUT_OF_MEMORY;
+  cudaMemcpyAsync(dk0, k0.data(), (n + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, s);
   for (int sd = 0; sd < 2; ++sd) {
     const int64_t nr = nring[sd];
-    dxy[sd] = A.take_n<double>(hxy[sd].size());
+    dxy[sd] = A.take_n<double>(2 * (nvert[sd] + nr));
     dvn[sd] = A.take_n<int32_t>(nr);
     dvp[sd] = A.take_n<int64_t>(nr);
     dstart[sd] = A.take_n<int64_t>(nr);
     dedge[sd] = A.take_n<int64_t>(nr + n);
     dsz[sd] = A.take_n<int32_t>(nr);
-    if (!dxy[sd] || !dvn[sd] || !dvp[sd] || !dstart[sd] || !dedge[sd] || !dsz[sd]) return ST_OUT_OF_MEMORY;
-    cudaMemcpyAsync(dxy[sd], hxy[sd].data(), hxy[sd].size() * sizeof(double), cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(dvn[sd], hvn[sd].data(), nr * sizeof(int32_t), cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(dvp[sd], hvp[sd].data(), nr * sizeof(int64_t), cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(dstart[sd], hstart[sd].data(), nr * sizeof(int64_t), cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(dedge[sd], hedge[sd].data(), (nr + n) * sizeof(int64_t), cudaMemcpyHostToDevice, s);
+    dc0[sd] = A.take_n<int64_t>(n);
+    drings[sd] = A.take_n<int32_t>(n);
+    double* open = A.take_n<double>(2 * nvert[sd]);
+    int64_t* first = A.take_n<int64_t>(nr);                  // first vertex of each open ring
+    void* st = A.take(scan_temp_bytes(nr));
+    if (!dxy[sd] || !dvn[sd] || !dvp[sd] || !dstart[sd] || !dedge[sd] || !dsz[sd] || !dc0[sd] || !drings[sd] || !open ||
+        !first || !st)
+      return ST_OUT_OF_MEMORY;
     cudaMemcpyAsync(dsz[sd], sz[sd], nr * sizeof(int32_t), cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(dc0[sd], c0[sd].data(), n * sizeof(int64_t), cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(drings[sd], rings[sd], n * sizeof(int32_t), cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(open, src[sd], 2 * nvert[sd] * sizeof(double), cudaMemcpyHostToDevice, s);
+    exclusive_scan_i32(dsz[sd], first, nr, nullptr, st, d_err, s);
+    { multi_ring_kernel<<<(unsigned)((32 * nr + 127) / 128), 128, 0, s>>>(
+          reinterpret_cast<const double2*>(open), dsz[sd], first, nr, reinterpret_cast<double2*>(dxy[sd]), dvn[sd],
+          dvp[sd], dstart[sd]); note_launch(); }
+    { multi_edge_kernel<<<(unsigned)((32 * n + 127) / 128), 128, 0, s>>>(dsz[sd], first, dc0[sd], drings[sd], n, dedge[sd]); note_launch(); }
   }
-  int32_t* dpid = A.take_n<int32_t>(K);
-  int32_t* dqid = A.take_n<int32_t>(K);
-  if (!dpid || !dqid) return ST_OUT_OF_MEMORY;
-  cudaMemcpyAsync(dpid, hpid.data(), K * sizeof(int32_t), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(dqid, hqid.data(), K * sizeof(int32_t), cudaMemcpyHostToDevice, s);
-  if (!sync()) return ST_CUDA_ERROR;                         // host staging vectors end here
+  { multi_ids_kernel<<<(unsigned)((32 * n + 127) / 128), 128, 0, s>>>(dk0, dc0[0], dc0[1], drings[1], n, dpid, dqid); note_launch(); }
   const LayerDev LP{dxy[0], dvn[0], dvp[0], nring[0]}, LQ{dxy[1], dvn[1], dvp[1], nring[1]};
   // ---- intersection records of every ring pair (stages G0-G3), in ring-pair order
   ClipParams p2 = prm;
@@ -754,17 +798,19 @@ int run_clip_multi_batch(int64_t n, const double* hP, const int32_t* sizesP, con
   int st = run_clip(LP, LQ, dpid, dqid, K, p2, A, CR, d_err, hs, s, nullptr, nullptr, &ex);
   if (st != ST_OK) return st;
   const int64_t nRall = ex.n_records;
-  std::vector<int64_t> c1(K);
-  cudaMemcpyAsync(c1.data(), CR.count1, K * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  // records per pair
+  int64_t* dcount = A.take_n<int64_t>(n);
+  if (!dcount) return ST_OUT_OF_MEMORY;
+  { multi_count_kernel<<<(unsigned)((32 * n + 127) / 128), 128, 0, s>>>(CR.count1, dk0, n, dcount); note_launch(); }
+  std::vector<int64_t> hcount1(n);
+  cudaMemcpyAsync(hcount1.data(), dcount, n * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
   if (!sync()) return ST_CUDA_ERROR;
   // ---- each pair's place in the work arrays and result regions
   std::vector<MultiPairDesc> hd(n);
-  std::vector<int64_t> hcount1(n);
   int64_t r = 0, sP = 0, sQ = 0, vo = 0, co = 0;
   for (int64_t i = 0; i < n; ++i) {
     MultiPairDesc& d = hd[i];
-    int64_t nR = 0;
-    for (int64_t k = k0[i]; k < k0[i + 1]; ++k) nR += c1[k];
+    const int64_t nR = hcount1[i];
     const int64_t capP = ne[0][i] + 2 * nR + ringsP[i] + 8, capQ = ne[1][i] + 2 * nR + ringsQ[i] + 8;
     if (capP > INT32_MAX || capQ > INT32_MAX) return ST_OUT_OF_MEMORY;
     d.kP = ringsP[i]; d.kQ = ringsQ[i];
@@ -775,7 +821,6 @@ int run_clip_multi_batch(int64_t n, const double* hP, const int32_t* sizesP, con
     d.sP0 = sP; d.sQ0 = sQ; d.capP = (int32_t)capP; d.capQ = (int32_t)capQ;
     d.v0 = vo; d.vcap = 2 * (capP + capQ) + 16;
     d.c0 = co; d.ccap = (int32_t)std::min<int64_t>(2 * nR + ringsP[i] + ringsQ[i] + 16, INT32_MAX); d.pad = 0;
-    hcount1[i] = nR;
     r += nR; sP += capP; sQ += capQ; vo += d.vcap; co += d.ccap;
   }
   if (r != nRall) return ST_CUDA_ERROR;                    // records are in ring-pair order
@@ -824,7 +869,7 @@ int run_clip_multi_batch(int64_t n, const double* hP, const int32_t* sizesP, con
   a.status = C.status; a.outNC = C.ncomp; a.outNV = nvOut;
   a.epsClean = prm.eps_clean; a.uni = prm.union_mode; a.exact = prm.exact; a.err = d_err;
   cudaMemsetAsync(C.swapped, 0, n * sizeof(int32_t), s);
-  cudaMemcpyAsync(C.count1, hcount1.data(), n * sizeof(int64_t), cudaMemcpyHostToDevice, s);
+  cudaMemcpyAsync(C.count1, dcount, n * sizeof(int64_t), cudaMemcpyDeviceToDevice, s);
   cudaMemcpyAsync(dd, hd.data(), n * sizeof(MultiPairDesc), cudaMemcpyHostToDevice, s);
   // Pairs per warp: one while the batch leaves warps to spare (its pairs then do not wait for
   // one another's branches), up to 32 for large ones.
