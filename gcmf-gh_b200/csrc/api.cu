@@ -166,6 +166,15 @@ gcmfgh_status finish(gcmfgh_ctx* c, int st) {
   return GCMFGH_OK;
 }
 
+// The clip's status counts, queued behind it: they come with finish()'s one wait.
+void queue_clip_stats(gcmfgh_ctx* c, int st) {
+  if (st != ST_OK || c->clip.n_pairs <= 0) return;
+  cudaMemsetAsync(c->d_stats, 0, 3 * sizeof(unsigned long long), c->stream);
+  { clip_stats_kernel<<<(unsigned)((c->clip.n_pairs + kThreads - 1) / kThreads), kThreads, 0, c->stream>>>(
+      c->clip.status, c->clip.n_pairs, c->d_stats); note_launch(); }
+  cudaMemcpyAsync(c->h_scratch + 56, c->d_stats, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream);
+}
+
 gcmfgh_status clip_info(gcmfgh_ctx* c, gcmfgh_clip_info* info) {
   if (!info) return GCMFGH_OK;
   info->n_pairs = c->clip.n_pairs;
@@ -175,14 +184,9 @@ gcmfgh_status clip_info(gcmfgh_ctx* c, gcmfgh_clip_info* info) {
   info->n_ring_vertices = c->clip.n_ring_vertices;
   info->n_invalid = info->n_disjoint = info->n_error = 0;
   if (c->clip.n_pairs > 0) {
-    cudaMemsetAsync(c->d_stats, 0, 3 * sizeof(unsigned long long), c->stream);
-    { clip_stats_kernel<<<(unsigned)((c->clip.n_pairs + kThreads - 1) / kThreads), kThreads, 0, c->stream>>>(
-        c->clip.status, c->clip.n_pairs, c->d_stats); note_launch(); }
-    cudaMemcpyAsync(c->h_scratch, c->d_stats, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream);
-    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return GCMFGH_CUDA_ERROR;
-    info->n_invalid = c->h_scratch[0];
-    info->n_disjoint = c->h_scratch[1];
-    info->n_error = c->h_scratch[2];
+    info->n_invalid = c->h_scratch[56];
+    info->n_disjoint = c->h_scratch[57];
+    info->n_error = c->h_scratch[58];
   }
   return GCMFGH_OK;
 }
@@ -242,6 +246,7 @@ gcmfgh_status run_clip_ctx(gcmfgh_ctx* c, const gcmfgh_layer* b, const gcmfgh_la
   const ClipParams prm = force ? *force : clip_params(c, b, o, n);
   int st = run_clip(to_dev(b), to_dev(o), pid, qid, n, prm, c->clip_arena, c->clip, c->d_err,
                     c->h_scratch, c->stream, &c->marks[1], c->aux, nullptr, c->aux2, mbrB, mbrO, je);
+  queue_clip_stats(c, st);
   gcmfgh_status r = finish(c, st);
   if (r != GCMFGH_OK) return r;
   c->have_clip = true;
@@ -810,6 +815,7 @@ gcmfgh_status gh_clip_multi(gcmfgh_ctx* c, const double* P, const int32_t* p_siz
   cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
   int st = run_clip_multi(P, p_sizes, p_rings, Q, q_sizes, q_rings, c->prm, c->clip_arena, c->clip, c->d_err,
                           c->h_scratch, c->stream);
+  queue_clip_stats(c, st);
   gcmfgh_status r = finish(c, st);
   if (r != GCMFGH_OK) return r;
   c->have_clip = true;
@@ -827,6 +833,7 @@ gcmfgh_status gh_clip_multi_batch(gcmfgh_ctx* c, int64_t n, const double* P, con
   cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
   int st = run_clip_multi_batch(n, P, p_sizes, p_rings, Q, q_sizes, q_rings, c->prm, c->clip_arena, c->clip,
                                 c->d_err, c->h_scratch, c->stream);
+  queue_clip_stats(c, st);
   gcmfgh_status r = finish(c, st);
   if (r != GCMFGH_OK) return r;
   c->have_clip = true;

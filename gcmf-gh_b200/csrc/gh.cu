@@ -920,9 +920,12 @@ __global__ void record_count_kernel(Records R, int64_t nR, const int64_t* __rest
 
 // slot of each edge's source vertex in the concatenated merged rings: the exclusive scan
 // of (1 + insertions) over the edges, i.e. the edge index plus the scan of the insertions
-__global__ void edge_slots_kernel(const int64_t* __restrict__ insBase, int64_t nE, int64_t* __restrict__ vpos) {
+// (both sides in one launch, as in pair_ring_kernel: blockIdx.y)
+__global__ void edge_slots_kernel(const int64_t* __restrict__ insP, int64_t nEP, int64_t* __restrict__ vposP,
+                                  const int64_t* __restrict__ insQ, int64_t nEQ, int64_t* __restrict__ vposQ) {
   int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (e < nE) vpos[e] = e + insBase[e];
+  if (blockIdx.y == 0) { if (e < nEP) vposP[e] = e + insP[e]; }
+  else if (e < nEQ) vposQ[e] = e + insQ[e];
 }
 
 // The merged rings of one side live in one buffer of n slots, column by column:
@@ -982,12 +985,23 @@ struct RingSet {
 };
 
 // per pair: ring size, region offset (ring + room for added vertices)
-__global__ void pair_ring_kernel(const int64_t* __restrict__ eoff, const int64_t* __restrict__ vpos,
-                                 const int32_t* __restrict__ n, const int32_t* __restrict__ nrec,
-                                 const int32_t* __restrict__ status, int64_t K, int64_t nE,
-                                 const int64_t* __restrict__ insTot,
-                                 int32_t* __restrict__ m, int64_t* __restrict__ regSize,
+struct RingSide {
+  const int64_t* eoff; const int64_t* vpos; const int32_t* n;
+  int64_t nE;
+  const int64_t* insTot;
+  int32_t* m; int64_t* regSize;
+};
+__global__ void pair_ring_kernel(RingSide sideP, RingSide sideQ, const int32_t* __restrict__ nrec,
+                                 const int32_t* __restrict__ status, int64_t K,
                                  unsigned long long* __restrict__ ringTot) {
+  const RingSide& S = blockIdx.y == 0 ? sideP : sideQ;
+  const int64_t* eoff = S.eoff;
+  const int64_t* vpos = S.vpos;
+  const int32_t* n = S.n;
+  const int64_t nE = S.nE;
+  const int64_t* insTot = S.insTot;
+  int32_t* m = S.m;
+  int64_t* regSize = S.regSize;
   int64_t k = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   unsigned long long mm = 0;
   if (k < K) {
@@ -3869,11 +3883,14 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   int64_t* chunkOff = A.take_n<int64_t>(K);
   int64_t* eoffP = A.take_n<int64_t>(K);
   int64_t* eoffQ = A.take_n<int64_t>(K);
-  int64_t* tot = A.take_n<int64_t>(16);
+  // totals and counters, cleared at once: 0-15 totals, 16 binned pairs, 20-27 labelling
+  // classes, 28-31 heavy and mid edges, 32 long pairs of the edge filter
+  int64_t* tot = A.take_n<int64_t>(40);
   void* stK = A.take(scan_temp_bytes(K));
   if (!D.pS || !D.qS || !D.nP || !D.nQ || !D.pSide || !D.cmbr || !D.status || !C.swapped || !C.count1 ||
       !cP || !cQ || !offP || !offQ || !nchunk || !chunkOff || !eoffP || !eoffQ || !tot || !stK)
     return ST_OUT_OF_MEMORY;
+  cudaMemsetAsync(tot, 0, 40 * sizeof(int64_t), s);
   { setup_kernel<<<blocks_for(K), kThreads, 0, s>>>(Lb, Lo, d_pid, d_qid, K, mb, mo, D, C.swapped, prm.no_swap); note_launch(); }
   // The narrow-tile and whole-warp passes of the edge filter take disjoint pairs (by size):
   // with an auxiliary stream the warp pass runs beside the tile pass.
@@ -3893,9 +3910,8 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   LongPairs lpF;
   if (longPairs) {
     lpF.ids = A.take_n<int32_t>(K);
-    lpF.n = A.take_n<unsigned>(1);
-    if (!lpF.ids || !lpF.n) return ST_OUT_OF_MEMORY;
-    cudaMemsetAsync(lpF.n, 0, sizeof(unsigned), s);
+    lpF.n = reinterpret_cast<unsigned*>(tot + 32);
+    if (!lpF.ids) return ST_OUT_OF_MEMORY;
   }
   auto edge_filter = [&](auto mode, int32_t* lp, int32_t* lq) {
     constexpr int kMode = decltype(mode)::value;
@@ -3921,9 +3937,8 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   exclusive_scan_i32(D.nP, eoffP, K, tot + 2, stK, d_err, s);
   exclusive_scan_i32(D.nQ, eoffQ, K, tot + 3, stK, d_err, s);
   int64_t* bigList = A.take_n<int64_t>(K);
-  unsigned long long* nBig = A.take_n<unsigned long long>(1);
-  if (!bigList || !nBig) return ST_OUT_OF_MEMORY;
-  cudaMemsetAsync(nBig, 0, sizeof(unsigned long long), s);
+  unsigned long long* nBig = reinterpret_cast<unsigned long long*>(tot + 16);
+  if (!bigList) return ST_OUT_OF_MEMORY;
   { chunk_count_kernel<<<blocks_for(K), kThreads, 0, s>>>(cP, cQ, K, nchunk, bigList, nBig, prm.bin_grid); note_launch(); }
   exclusive_scan_i64(nchunk, chunkOff, K, tot + 4, stK, d_err, s);
   mk->mark("clip:setup+filter", s);
@@ -3946,9 +3961,6 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   int32_t* pairRec = nullptr;
   int32_t* pairQ = nullptr;
   if (fused) {
-    pairRec = A.take_n<int32_t>(K);
-    pairQ = A.take_n<int32_t>(K);
-    if (!pairRec || !pairQ) return ST_OUT_OF_MEMORY;
   } else {
     chunkRec = A.take_n<int32_t>(nCh);
     chunkQ = A.take_n<int32_t>(nCh);
@@ -3957,12 +3969,16 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     stC = A.take(scan_temp_bytes(std::max<int64_t>(nCh, 1)));
     if (!chunkRec || !chunkQ || !recScan || !qScan || !stC) return ST_OUT_OF_MEMORY;
   }
-  int64_t* binRec = A.take_n<int64_t>(K);
-  int64_t* binQ = A.take_n<int64_t>(K);
-  if (!LP || !LQ || !chunkPair || !binRec || !binQ) return ST_OUT_OF_MEMORY;
+  // per-pair counts, cleared at once: binned records and Q hits, and the fused pass's
+  int64_t* binRec = A.take_n<int64_t>(3 * K);
+  if (!LP || !LQ || !chunkPair || !binRec) return ST_OUT_OF_MEMORY;
+  int64_t* binQ = binRec + K;
+  if (fused) {
+    pairRec = reinterpret_cast<int32_t*>(binRec + 2 * K);
+    pairQ = pairRec + K;
+  }
   if (nCh > 0) { chunk_pair_kernel<<<blocks_for_warps(K), kThreads, 0, s>>>(chunkOff, nchunk, K, chunkPair); note_launch(); }
-  cudaMemsetAsync(binRec, 0, K * sizeof(int64_t), s);
-  cudaMemsetAsync(binQ, 0, K * sizeof(int64_t), s);
+  cudaMemsetAsync(binRec, 0, 3 * K * sizeof(int64_t), s);
   edge_filter(std::integral_constant<int, 1>{}, LP, LQ);
   // The binned pairs (below) go to the auxiliary stream when there is one: fork here, before
   // the chunked count is queued on s, so that the two run side by side.
@@ -4002,13 +4018,6 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     recCap = prm.rec_hint > 0 ? prm.rec_hint + prm.rec_hint / 4 + 4096 : kFirstRecordCap;
     if (nBigPairs == 0) recCap = std::min(recCap, std::max<int64_t>(nCh * kChunk, 1));
     if (!take_records(recCap)) return ST_OUT_OF_MEMORY;
-    cudaMemsetAsync(recTot, 0, sizeof(unsigned long long), s);
-    cudaMemsetAsync(pairRec, 0, K * sizeof(int32_t), s);
-    cudaMemsetAsync(pairQ, 0, K * sizeof(int32_t), s);
-    if (sb != s) {                                  // the counter is cleared before either starts
-      cudaEventRecord(bev[0], s);
-      cudaStreamWaitEvent(sb, bev[0], 0);
-    }
     launch_fused(true);
   } else if (nCh > 0) {
     { (prm.exact ? intersect_kernel<0, 1> : intersect_kernel<0, 0>)<<<blocks_for_warps(nCh), kThreads, 0, s>>>(
@@ -4161,35 +4170,29 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     return ST_OK;
   }
   // ---- G4 ring layout
-  int32_t* insP = A.take_n<int32_t>(nEP);
-  int32_t* insQ = A.take_n<int32_t>(nEQ);
-  int64_t* srcLinkP = A.take_n<int64_t>(nEP);
-  int64_t* srcLinkQ = A.take_n<int64_t>(nEQ);
+  // per edge, cleared at once: links of the source vertices, insertion counts and cursors
+  int64_t* srcLinkP = A.take_n<int64_t>(2 * (nEP + nEQ));
   int64_t* vposP = A.take_n<int64_t>(nEP);
   int64_t* vposQ = A.take_n<int64_t>(nEQ);
   int64_t* insBaseP = A.take_n<int64_t>(nEP);
   int64_t* insBaseQ = A.take_n<int64_t>(nEQ);
-  int32_t* curP = A.take_n<int32_t>(nEP);
-  int32_t* curQ = A.take_n<int32_t>(nEQ);
   int64_t* slotP = A.take_n<int64_t>(nR);
   int64_t* slotQ = A.take_n<int64_t>(nR);
   void* stE = A.take(scan_temp_bytes(std::max<int64_t>(std::max(nEP, nEQ), 1)));
-  if (!insP || !insQ || !srcLinkP || !srcLinkQ || !vposP || !vposQ || !insBaseP ||
-      !insBaseQ || !curP || !curQ || !slotP || !slotQ || !stE)
-    return ST_OUT_OF_MEMORY;
-  cudaMemsetAsync(insP, 0, nEP * sizeof(int32_t), s);
-  cudaMemsetAsync(insQ, 0, nEQ * sizeof(int32_t), s);
-  cudaMemsetAsync(srcLinkP, 0, nEP * sizeof(int64_t), s);
-  cudaMemsetAsync(srcLinkQ, 0, nEQ * sizeof(int64_t), s);
-  cudaMemsetAsync(curP, 0, nEP * sizeof(int32_t), s);
-  cudaMemsetAsync(curQ, 0, nEQ * sizeof(int32_t), s);
+  if (!srcLinkP || !vposP || !vposQ || !insBaseP || !insBaseQ || !slotP || !slotQ || !stE) return ST_OUT_OF_MEMORY;
+  int64_t* srcLinkQ = srcLinkP + nEP;
+  int32_t* insP = reinterpret_cast<int32_t*>(srcLinkQ + nEQ);
+  int32_t* insQ = insP + nEP;
+  int32_t* curP = insQ + nEQ;
+  int32_t* curQ = curP + nEP;
+  cudaMemsetAsync(srcLinkP, 0, 2 * (nEP + nEQ) * sizeof(int64_t), s);
   if (nR > 0)
     { record_count_kernel<<<blocks_for(nR), kThreads, 0, s>>>(R, nR, eoffP, eoffQ, D.status, insP, insQ,
                                                             srcLinkP, srcLinkQ); note_launch(); }
   exclusive_scan_i32(insP, insBaseP, nEP, tot + 9, stE, d_err, s);
   exclusive_scan_i32(insQ, insBaseQ, nEQ, tot + 10, stE, d_err, s);
-  { edge_slots_kernel<<<blocks_for(nEP), kThreads, 0, s>>>(insBaseP, nEP, vposP); note_launch(); }
-  { edge_slots_kernel<<<blocks_for(nEQ), kThreads, 0, s>>>(insBaseQ, nEQ, vposQ); note_launch(); }
+  { edge_slots_kernel<<<dim3(blocks_for(std::max<int64_t>(std::max(nEP, nEQ), 1)), 2), kThreads, 0, s>>>(
+        insBaseP, nEP, vposP, insBaseQ, nEQ, vposQ); note_launch(); }
   // Sizes: the record export reads the exact ones back; the clip takes bounds instead
   // and saves the two host round trips (a record inserts at most one vertex per side).
   const bool exactSizes = ex != nullptr;
@@ -4213,20 +4216,17 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     { record_scatter_kernel<<<blocks_for(nR), kThreads, 0, s>>>(R, nR, eoffP, eoffQ, D.status, insBaseP, curP,
                                                               insListP, insBaseQ, curQ, insListQ); note_launch(); }
   unsigned long long* ringTot = reinterpret_cast<unsigned long long*>(tot + 6);
-  cudaMemsetAsync(ringTot, 0, sizeof(unsigned long long), s);
-  { pair_ring_kernel<<<blocks_for(K), kThreads, 0, s>>>(eoffP, vposP, D.nP, nrec, D.status, K, nEP, tot + 9, mP,
-                                                      regSizeP, ringTot); note_launch(); }
-  { pair_ring_kernel<<<blocks_for(K), kThreads, 0, s>>>(eoffQ, vposQ, D.nQ, nrec, D.status, K, nEQ, tot + 10, mQ,
-                                                      regSizeQ, ringTot); note_launch(); }
+  { pair_ring_kernel<<<dim3(blocks_for(K), 2), kThreads, 0, s>>>(RingSide{eoffP, vposP, D.nP, nEP, tot + 9, mP, regSizeP},
+                                                              RingSide{eoffQ, vposQ, D.nQ, nEQ, tot + 10, mQ, regSizeQ},
+                                                              nrec, D.status, K, ringTot); note_launch(); }
   // The one-thread and warp labelling kernels take their pairs in size order (largest
   // first, label_order_kernel), and the ring regions are laid out in that order, so that
   // the pairs labelled side by side have neighbouring regions.  The record export keeps
   // the regions in pair order.
   const int64_t midMin = std::min(prm.mid_label_min, prm.big_label_min);
-  unsigned long long* mcnt = A.take_n<unsigned long long>(8);
+  unsigned long long* mcnt = reinterpret_cast<unsigned long long*>(tot + 20);
   uint32_t* oval = A.take_n<uint32_t>(K);
-  if (!mcnt || !oval) return ST_OUT_OF_MEMORY;
-  cudaMemsetAsync(mcnt, 0, 8 * sizeof(unsigned long long), s);
+  if (!oval) return ST_OUT_OF_MEMORY;
   if (!ex) {
     uint64_t* okey = A.take_n<uint64_t>(K);
     uint64_t* okeyAlt = A.take_n<uint64_t>(K);
@@ -4239,11 +4239,16 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     if (!okey || !okeyAlt || !ovalAlt || !otmp || !sortedP || !sortedQ || !offSP || !offSQ) return ST_OUT_OF_MEMORY;
     { label_order_kernel<<<blocks_for(K), kThreads, 0, s>>>(mP, mQ, D.status, K, std::max<int64_t>(prm.tile_label_max, 0),
                                                            midMin, prm.big_label_min, okey, oval, mcnt); note_launch(); }
+    if (K == 1) {                                     // one pair: nothing to order, its regions come first
+      cudaMemsetAsync(regP, 0, sizeof(int64_t), s);
+      cudaMemsetAsync(regQ, 0, sizeof(int64_t), s);
+    } else {
     radix_sort_pairs(okey, oval, okeyAlt, ovalAlt, K, 8, otmp, d_err, s);
     { permute_sizes_kernel<<<blocks_for(K), kThreads, 0, s>>>(oval, K, regSizeP, regSizeQ, sortedP, sortedQ); note_launch(); }
     exclusive_scan_i64(sortedP, offSP, K, tot + 11, stK, d_err, s);
     exclusive_scan_i64(sortedQ, offSQ, K, tot + 12, stK, d_err, s);
     { unpermute_offsets_kernel<<<blocks_for(K), kThreads, 0, s>>>(oval, K, offSP, offSQ, regP, regQ); note_launch(); }
+    }
   } else {
     exclusive_scan_i64(regSizeP, regP, K, tot + 11, stK, d_err, s);
     exclusive_scan_i64(regSizeQ, regQ, K, tot + 12, stK, d_err, s);
@@ -4279,9 +4284,7 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    unsigned long long* nHeavy = A.take_n<unsigned long long>(4);     // [heavy, mid] of P, of Q
-    if (!nHeavy) return ST_OUT_OF_MEMORY;
-    cudaMemsetAsync(nHeavy, 0, 4 * sizeof(unsigned long long), s);
+    unsigned long long* nHeavy = reinterpret_cast<unsigned long long*>(tot + 28);     // [heavy, mid] of P, of Q
     const unsigned midBlocks = 8 * (unsigned)nsm;
     cudaStream_t sq = s;
     cudaEvent_t fork = nullptr, join = nullptr;
