@@ -11,20 +11,21 @@
 //                   vertices is P), MBRs, common MBR (ghcuda.cpp:94-125), disjoint check
 //   G1 edge filter  warp/pair: P and Q edges whose box touches the common MBR
 //                   (gppolyclip_mDIV512.cu:382-415), compacted in edge order
-//   G2 count        warp per 256-edge-pair chunk of each pair's filtered P x Q grid: box
+//   G2/G3 records   warp per 32-edge-pair chunk of each pair's filtered P x Q grid: box
 //                   test (:345-371) and classification from both sides (:95-169);
-//                   records = P-side hits, the P/Q totals decide validity (:1461)
-//   G3 emit         same chunks; records written in (pair, P edge, Q edge) order, so no
-//                   sort is needed and results do not depend on scheduling
+//                   records = P-side hits, appended as they are found, the P/Q totals
+//                   decide validity (:1461).  Pairs with large grids: a uniform grid over
+//                   the common MBR, a warp per eight P edges.  (The record export counts
+//                   first and writes in (pair, P edge, Q edge) order.)
 //   G4 ring layout  per edge: 1 source vertex + inserted vertices; one device scan per
 //                   side gives every vertex its slot (replaces the host scans :1431-1434)
-//   G5 ring fill    thread/edge: inserted vertices ordered by exact parameter (ties: later
+//   G5 ring fill    thread, warp or block per edge by its insertions: inserted vertices ordered by exact parameter (ties: later
 //                   insertion first, as polygon.h:101-113 inserts in the loop order of
 //                   polyclip.h:202-205) instead of the reference GPU's 1e-7-quantised
 //                   radix sort (:290-305, :1034)
 //   G6 links        thread/record: neighbour links as polyclip.h:215-267 makes them; a
 //                   source vertex linked by several records keeps the last one
-//   G7 label+trace  thread/pair: initial labels, chains, special cases, entry/exit, split
+//   G7 label+trace  thread, warp, block or grid per pair by its size: initial labels, chains, special cases, entry/exit, split
 //                   pairs, crossing candidates, tracing and clean-up
 //   G8 compaction   per-pair output regions -> one contiguous result
 //
@@ -934,8 +935,7 @@ __global__ void edge_slots_kernel(const int64_t* __restrict__ insP, int64_t nEP,
 // walks a pair keeps three words per ring instead of a pointer per column, and each
 // column stays dense for the scans over one field.
 //   nx, pv, nb  next, previous, neighbour (slot on the other ring, -1 none)
-//   tn tl to ls tracing scratch: next run start (other ring), run length, output offset,
-//               and (by list index) the slots of the flagged vertices
+//   tn tl to ls scratch of the trace and the clean-up
 //   it          intersection flag (cleared when visited by the trace)
 //   lb, ee      IntersectionLabel, EntryExitLabel
 //   fl          bit0 split candidate, bit1 crossing candidate
