@@ -19,14 +19,15 @@
 //                   first and writes in (pair, P edge, Q edge) order.)
 //   G4 ring layout  per edge: 1 source vertex + inserted vertices; one device scan per
 //                   side gives every vertex its slot (replaces the host scans :1431-1434)
-//   G5 ring fill    thread, warp or block per edge by its insertions: inserted vertices ordered by exact parameter (ties: later
-//                   insertion first, as polygon.h:101-113 inserts in the loop order of
-//                   polyclip.h:202-205) instead of the reference GPU's 1e-7-quantised
-//                   radix sort (:290-305, :1034)
+//   G5 ring fill    thread, warp or block per edge by its insertions: inserted vertices
+//                   ordered by exact parameter (ties: later insertion first, as
+//                   polygon.h:101-113 inserts in the loop order of polyclip.h:202-205)
+//                   instead of the reference GPU's 1e-7-quantised radix sort (:290-305, :1034)
 //   G6 links        thread/record: neighbour links as polyclip.h:215-267 makes them; a
 //                   source vertex linked by several records keeps the last one
-//   G7 label+trace  thread, warp, block or grid per pair by its size: initial labels, chains, special cases, entry/exit, split
-//                   pairs, crossing candidates, tracing and clean-up
+//   G7 label+trace  thread, warp, block or grid per pair by its size: initial labels, chains,
+//                   special cases, entry/exit, split pairs, crossing candidates, tracing and
+//                   clean-up
 //   G8 compaction   per-pair output regions -> one contiguous result
 //
 // Layout in HBM: the input layers stay interleaved FP64 (16 B per vertex).  Records are
@@ -765,7 +766,7 @@ __device__ __forceinline__ bool bin_f32_rejects(float4 p, float4 q, float M) {
 // range of the global counter taken per classified group, as in intersect_fused_kernel.
 // Bound by instruction issue.  A thread per P edge enumerating its listings in FP64, once to
 // count and once to emit, took 271 ms for the 400,000 x 200,000-vertex pair (2.9e7
-// records) and 31.3 ms for the degenerate batch of 10,007 pairs (2.3e7), this 18.6 and 10.5 ms.
+// records) and 31.3 ms for the degenerate batch of 10,007 pairs (2.3e7), this 14.1 and 9.2 ms.
 // (3 blocks per SM at 80 registers: 22.4 ms against 27.2 ms for 2 at 128, cells of the mean box.)
 constexpr int kBinEdges = 8;
 
@@ -2823,7 +2824,9 @@ __device__ __forceinline__ void loop_offsets(const T& tab, int t, int in, int ba
 // from that crossing on.  So instead of walking them one after another (a chain of dependent
 // loads over all pieces of the pair, with the rest of the group waiting), every segment finds
 // out whether it is its loop's smallest, the loops' sizes are scanned, and all loops are
-// walked at once for the offsets of their segments.
+// walked at once for the offsets of their segments.  Trace of 10,007 degenerate pairs (2.3e7
+// crossings): 10.5 s of blocks' time as one walk per pair, 0.8 s so (a step costs two shared
+// loads where the loop table fits shared memory).
 // Returns 0 when done, 1 when the conditions do not hold (the caller then runs the general
 // walk), -1 on a capacity error.
 template <class G>

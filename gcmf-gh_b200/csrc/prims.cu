@@ -222,7 +222,8 @@ radix_scatter_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restri
 // 256 digit counts and adds up those of the tiles before it by decoupled look-back, a thread
 // per digit with kSweepAhead predecessors in flight; the digits' totals of all passes come
 // from one histogram kernel in front.  Against histogram, scan and scatter kernels with a
-// clear in between: 29 -> 13 us per pass at 20,000 keys, 38 -> 26 us at 700,000.
+// clear in between, all passes together: 0.115 -> 0.074 ms at 28,000 keys of 32 bits, 0.19 ->
+// 0.175 ms at 720,000 of 40.
 constexpr int64_t kSweepTiles = 512;
 constexpr int kSweepAhead = 16;
 constexpr int kSweepMaxPasses = 8;
@@ -325,8 +326,8 @@ radix_sweep_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict
 
 // Up to kSmallSort pairs in one block: a bitonic network over (key's low bits, place), which
 // makes the order that of a stable sort; then keys and values are written in that order.
-// Five launches per 8-bit pass otherwise: 85 us for the 24-bit pair keys of a join of 2,000 x
-// 2,000 polygons, 160 us for both layers' 32-bit keys.
+// Five launches per 8-bit pass otherwise.  Join of 2,000 x 2,000 polygons: MBRs and both
+// layers' sorts 0.161 -> 0.066 ms, pair sort 0.085 -> 0.049 ms.
 constexpr int kSmallSort = 4096;
 constexpr int kSmallSortThreads = 1024;
 
