@@ -701,6 +701,7 @@ def precision_measure(local, total=1_000_000, chunk=50_000, check_degenerate=120
 def run_ours(args, rank, world, local):
     import torch
     import gcmfgh
+    import pyoracle
     from gcmfgh import synth
     torch.cuda.set_device(local)
     dist = None
@@ -912,7 +913,9 @@ def run_ours(args, rank, world, local):
         if not args.no_precision and world == 1:
             line["precision"] = precision_measure(local, total=args.precision_pairs, chunk=args.precision_chunk,
                                                   check_all_degenerate=args.precision_check_all)
-        if world == 1 and not args.no_cpu_baseline:
+        if world == 1 and not args.no_cpu_baseline and not pyoracle.ref_available():
+            line["cpu_baseline"] = {"unavailable": "oracle/_ref not built (reference sources absent at build time)"}
+        elif world == 1 and not args.no_cpu_baseline:
             nb = args.sample_bases or 20000
             p, s, cores = reference_cpu_sample(base, ovl, nb, 7)
             line["cpu_baseline"] = {"value": p / s, "unit": "pairs/s", "cores": cores, "kind": "reference",
