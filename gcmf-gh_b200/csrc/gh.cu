@@ -1129,6 +1129,10 @@ __global__ void __launch_bounds__(kThreads, 4) ring_fill_kernel(LayerDev Lb, Lay
   for (int i = 0; i < cnt; ++i) write_inserted<kSide>(f, R, lst[i], i, S, slotOfRec);
 }
 
+// Sort key of an insertion's parameter: both zeros are one parameter (a crossing's parameter
+// rounds to -0.0 or +0.0 by the other edge's direction), as ring_fill_kernel compares them.
+__device__ __forceinline__ uint64_t param_key(double v) { return ordered_key(v + 0.0); }
+
 // A warp per mid edge: the records' (parameter bits, ~other edge) sorted in the warp's part of
 // shared memory, up to 32 by counting each record's predecessors with shuffles, more with
 // a bitonic network; then the vertices are written in order.  A block per edge beyond 32
@@ -1166,7 +1170,7 @@ mid_fill_kernel(LayerDev Lb, LayerDev Lo, PairDev D, Records R, const int64_t* _
       uint32_t t = ~0u;
       if (lane < cnt) {
         r = insList[l0 + lane];
-        k = ordered_key(kSide == 0 ? R.a[r] : R.b[r]);
+        k = param_key(kSide == 0 ? R.a[r] : R.b[r]);
         t = 0xffffffffu - (uint32_t)(kSide == 0 ? R.q[r] : R.p[r]);
       }
       int rank = 0;
@@ -1186,7 +1190,7 @@ mid_fill_kernel(LayerDev Lb, LayerDev Lo, PairDev D, Records R, const int64_t* _
       idx[i] = (uint16_t)i;
       if (i < cnt) {
         const int64_t r = insList[l0 + i];
-        key[i] = ordered_key(kSide == 0 ? R.a[r] : R.b[r]);
+        key[i] = param_key(kSide == 0 ? R.a[r] : R.b[r]);
         tie[i] = 0xffffffffu - (uint32_t)(kSide == 0 ? R.q[r] : R.p[r]);
       }
     }
@@ -1269,7 +1273,7 @@ heavy_fill_kernel(LayerDev Lb, LayerDev Lo, PairDev D, Records R, const int64_t*
     for (int i = threadIdx.x; i < npad; i += blockDim.x) {
       if (i < cnt) {
         int64_t r = insList[l0 + i];
-        key[i] = ordered_key(kSide == 0 ? R.a[r] : R.b[r]);
+        key[i] = param_key(kSide == 0 ? R.a[r] : R.b[r]);
         tie[i] = 0xffffffffu - (uint32_t)(kSide == 0 ? R.q[r] : R.p[r]);
         idx[i] = (uint32_t)i;
       } else {
