@@ -614,8 +614,13 @@ __global__ void bin_grid_kernel(PairDev D, BinSet S, int n) {
   } else if (h > 0) {
     gy = fmin(target, 4096.0);
   }
-  BinGrid G{c.x, c.y, w > 0 ? w / gx : 1.0, h > 0 ? h / gy : 1.0, (int)gx, (int)gy,
-            __double2float_ru(2.0 * fmax(fmax(w, h), 0.0))};
+  // The FP32 copies' range M.  What the side test's margins leave beside its error bound
+  // (2^-45 M^2, bin_f32_rejects) is above what products rounded at FP32's smallest step
+  // (2^-149) can lose for M >= 2^-50, and no product overflows up to 2^60.  Other ranges get no
+  // copies (a negative M): their edges all go to FP64.
+  const double range = 2.0 * fmax(fmax(w, h), 0.0);
+  const float M = range >= 0x1p-50 && range <= 0x1p60 ? __double2float_ru(range) : -1.f;
+  BinGrid G{c.x, c.y, w > 0 ? w / gx : 1.0, h > 0 ? h / gy : 1.0, (int)gx, (int)gy, M};
   S.grid[i] = G;
   S.ncell[i] = G.gx * G.gy;
 }
@@ -632,7 +637,7 @@ __device__ __forceinline__ int bin_class(bool firstCol, bool firstRow) {
 }
 
 // The FP32 copy of an edge relative to the grid's corner (four NaNs when it leaves the
-// range M: no FP32 test then rejects it).  Each value is within M * 2^-24 of the exact one.
+// range M, or M is negative: no FP32 test then rejects it).  Each value is within M * 2^-24 of the exact one.
 __device__ __forceinline__ float4 bin_edge_f32(double2 a, double2 b, const BinGrid& G) {
   const float4 r = make_float4(__double2float_rn(a.x - G.x0), __double2float_rn(a.y - G.y0),
                                __double2float_rn(b.x - G.x0), __double2float_rn(b.y - G.y0));
@@ -734,7 +739,8 @@ bin_pairs_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, int64_t np,
 // of the other, the sign tests having room for the copies' and the arithmetic's rounding.
 // With d = M 2^-24 the copies' error, A and B the 1-norms of the two differences that an
 // area is the cross product of (each at most 4 M), the area's error is below
-// 2 d (A + B) + 4 d min(A, B) + 8 d^2 + 4 2^-24 A B < 24 d (A + B + d); 32 is used.
+// 2 d (A + B) + 4 d min(A, B) + 8 d^2 + 4 2^-24 A B < 24 d (A + B + d); 32 is used.  The rest,
+// 8 d (A + B + d) >= 2^-45 M^2, covers underflow for the M that have copies (bin_grid_kernel).
 template <int kExact>
 __device__ __forceinline__ bool bin_f32_rejects(float4 p, float4 q, float M) {
   const float slop = M * 2.3841858e-7f;                                  // 2^-22

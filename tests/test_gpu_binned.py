@@ -54,3 +54,67 @@ def test_every_pair_binned(engine, exact, hint):
     assert np.array_equal(r.ncomp, o.ncomp)
     assert np.array_equal(r.comp_size, o.comp_size)
     assert np.array_equal(r.xy, o.xy)
+
+
+def _near_pairs(exponent):
+    """Pairs whose vertices lie close to the other ring's edges, at sizes whose products
+    underflow, overflow or just fit FP32."""
+    rng = np.random.default_rng(12)
+    pairs = []
+    for n in [3, 4, 5, 8, 17, 40] * 50:
+        P = synth._star(rng, n, 0.0, 0.0, 1.0, 0.5, 1.0)
+        Q = P * (1.0 + rng.choice([1e-1, 1e-2, 1e-8]) * rng.uniform(-1.0, 1.0, size=P.shape))
+        pairs.append((P * 2.0 ** exponent, np.roll(Q * 2.0 ** exponent, 1, 0)))
+    return pairs
+
+
+def _underflow_pairs(exponent):
+    """Pairs with an edge that ends 2^-26 beyond another: of 400,000, those that a side test on
+    FP32 copies whose margins underflow would take to be apart."""
+    rng = np.random.default_rng(1)
+    n, s = 400_000, 2.0 ** exponent
+    p1, p2 = rng.uniform(0.0, 1.0, (n, 2)), rng.uniform(0.0, 1.0, (n, 2))
+    d = p2 - p1
+    normal = np.stack([-d[:, 1], d[:, 0]], 1)
+    at = p1 + rng.uniform(0.1, 0.9, (n, 1)) * d
+    q1 = at + normal * rng.uniform(0.1, 1.2, (n, 1)) * 2.0 ** -26
+    q2 = at - normal * rng.uniform(0.3, 1.0, (n, 1))
+    f1, f2, g1, g2 = ((v * s).astype(np.float32) for v in (p1, p2, q1, q2))
+    M = np.float32(2.0 * s)
+    e, a, b = f2 - f1, g1 - f1, g2 - f1
+    norm = lambda v: np.abs(v[:, 0]) + np.abs(v[:, 1])                     # noqa: E731
+    with np.errstate(under="ignore"):
+        s1, s2 = (e[:, 0] * v[:, 1] - e[:, 1] * v[:, 0] for v in (a, b))
+        m1, m2 = (M * np.float32(2.0 ** -19) * (norm(e) + M * np.float32(2.0 ** -24) + norm(v)) for v in (a, b))
+    apart = ((s1 > m1) & (s2 > m2)) | ((s1 < -m1) & (s2 < -m2))
+    inside = (np.minimum(q1, q2) > 0.0).all(1) & (np.maximum(q1, q2) < 1.0).all(1)
+    # (the far corners make the common box the unit square)
+    return [(np.array([p1[i], p2[i], [1.0, 1.0], [0.0, 0.0]]) * s, np.array([q1[i], q2[i], [1.0, 0.0], [0.0, 1.0]]) * s)
+            for i in np.nonzero(apart & inside)[0]]
+
+
+@pytest.mark.parametrize("exponent", [-90, -68, -67, -66, -52, -51, -50, -48, 56, 58, 60, 62, 64, 100])
+def test_sizes_beyond_fp32(engine, exponent):
+    import gcmfgh
+    pairs = _near_pairs(exponent)
+    if -68 <= exponent <= -66:
+        beyond = _underflow_pairs(exponent)
+        assert len(beyond) >= 3
+        pairs += beyond
+    base, ovl = (synth.Layer.from_rings([p[i] for p in pairs]) for i in (0, 1))
+    ids = np.arange(len(pairs), dtype=np.int32)
+    try:
+        engine.set_tuning(bin_grid=0)
+        engine.set_precision(True)
+        engine.set_params(1e-7, 0.0, False)
+        engine.clip_batch(gcmfgh.DeviceLayer(base), gcmfgh.DeviceLayer(ovl), ids, ids)
+        r = engine.clip_result()
+    finally:
+        engine.set_tuning(bin_grid=1 << 16)
+        engine.set_precision(False)
+        engine.set_params(1e-7, 1e-7, False)
+    o = pyoracle.clip_batch(base, ovl, ids, ids, eps_clean=0.0, exact=True)
+    assert np.array_equal(r.status, o.status)
+    assert np.array_equal(r.count1[r.status != 2], o.count1[o.status != 2])
+    assert np.array_equal(r.comp_size, o.comp_size)
+    assert np.array_equal(r.xy, o.xy)
