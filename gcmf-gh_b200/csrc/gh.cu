@@ -1030,7 +1030,7 @@ __global__ void pair_ring_kernel(RingSide sideP, RingSide sideQ, const int32_t* 
 // more than kLightEdge insertions are listed for mid_fill_kernel (a warp each), those with more than
 // kMidEdge for heavy_fill_kernel (a block each).
 constexpr int kLightEdge = 8;
-constexpr int kMidEdge = 512;
+constexpr int kMidEdge = 256;
 
 struct EdgeFill {
   int64_t k, base;
@@ -1144,6 +1144,11 @@ __device__ __forceinline__ uint64_t param_key(double v) { return ordered_key(v +
 // a bitonic network; then the vertices are written in order.  A block per edge beyond 32
 // insertions (512 threads over 64 elements, a barrier per step) took 2.8 of the fill's 4.0 ms on
 // 2,500 degenerate pairs, and most of 16 ms on the large pair, whose edges all have 70 to 140.
+// The bound of kMidEdge is its shared memory, 14 bytes an element for every warp: with 512 (28
+// KB a block, all of an SM's at 8 blocks) four contexts on alternate steps of the batched join
+// took 5.66 ms a step, with 256 5.53, the L1 that their other kernels use being left to them;
+// 10,007 degenerate pairs 31.3 -> 29.4 ms, the large pair 48.7 -> 47.0.  With 128 the step takes 5.52,
+// the large pair 49.8 ms.
 constexpr int kMidThreads = 128;
 
 template <int kSide>

@@ -1,6 +1,6 @@
 """Crossings whose parameter rounds to zero, of either sign, on an edge with others: both
 zeros are one parameter, so the later other edge comes first whatever form orders the edge's
-insertions (a thread to 8, a warp to 512, a block beyond), against the oracle (bit for bit)."""
+insertions (a thread to 8, a warp to 256, a block beyond), against the oracle (bit for bit)."""
 from fractions import Fraction
 
 import numpy as np
@@ -72,7 +72,7 @@ def _crossings_of_first_edge(P, Q):
     return n, zeros
 
 
-COUNTS = [4, 7, 8, 9, 10, 31, 32, 33, 65, 511, 512, 513, 700]
+COUNTS = [4, 7, 8, 9, 10, 31, 32, 33, 65, 255, 256, 257, 513, 700]
 
 
 @pytest.mark.parametrize("count", COUNTS)
