@@ -546,6 +546,10 @@ gcmfgh_status gcmfgh_set_tuning(gcmfgh_ctx* c, int key, int64_t value) {
     c->hint_explicit = value > 0;
     return GCMFGH_OK;
   }
+  if (key == GCMFGH_TUNE_GRID_WAIT) {
+    c->prm.grid_wait = value;
+    return GCMFGH_OK;
+  }
   c->tuning_explicit = true;
   if (key == GCMFGH_TUNE_BIN_GRID) c->prm.bin_grid = value;
   else if (key == GCMFGH_TUNE_BIG_LABEL) c->prm.big_label_min = value;

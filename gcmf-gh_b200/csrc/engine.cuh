@@ -111,6 +111,8 @@ struct ClipParams {
   int64_t big_label_min = 1ll << 18;   // merged-ring slots above which a pair is labelled grid-wide
   int fused_emit = 1;                  // count and emit the intersection records in one pass
   int64_t rec_hint = 0;                // records expected (the last clip's count; 0 unknown)
+  int64_t grid_wait = 1ll << 26;       // polls without progress after which a barrier of the
+                                       // grid-wide labelling gives up (tens of seconds)
 };
 
 // The one-thread labelling's limit for a clip of n pairs when no threshold is set.  A thread

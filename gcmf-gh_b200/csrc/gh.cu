@@ -1667,18 +1667,24 @@ __device__ void seq_step1(PairCtx& c) {
   }
 }
 
+// What one member's long loops call as they go on: a grid's barrier counts it as progress.
+struct NoBeat { __device__ __forceinline__ void operator()(int) const {} };
+
 // step 2: intersection chains (polyclip.h:405-451).  n >= 0: the chain starts are among the n
 // slots listed in P.ls, in order
-__device__ void seq_step2(PairCtx& c, int n = -1) {
+template <class B = NoBeat>
+__device__ void seq_step2(PairCtx& c, int n = -1, B beat = B()) {
   Ring& P = c.R[0];
   Ring& Q = c.R[1];
   const int count = n < 0 ? P.m : n;
   for (int i = 0; i < count; ++i) {
     const int s = n < 0 ? i : P.ls(i);
+    beat(i);
     if (!P.it(s) || (P.lb(s) != L_LEFT_ON && P.lb(s) != L_RIGHT_ON)) continue;
     int x = P.lb(s) == L_LEFT_ON ? R_LEFT : R_RIGHT;
     int X = s, I = s, guard = P.m + 1;
     do {
+      beat(guard);
       P.lb(I) = L_NONE;
       if (P.nb(I) >= 0) Q.lb(P.nb(I)) = L_NONE;
       I = P.nx(I);
@@ -1773,13 +1779,14 @@ __device__ bool seq_step4(PairCtx& c) {
 
 // step 5: split vertex pairs (polyclip.h:661-714).  n >= 0: the candidates of P are the n
 // slots listed in P.ls, in order
-template <int EX>
-__device__ bool seq_step5(PairCtx& c, int n = -1) {
+template <int EX, class B = NoBeat>
+__device__ bool seq_step5(PairCtx& c, int n = -1, B beat = B()) {
   Ring& P = c.R[0];
   Ring& Q = c.R[1];
   const int pm0 = n < 0 ? P.used : n;
   for (int i = 0; i < pm0; ++i) {
     const int ip = n < 0 ? i : P.ls(i);
+    beat(i);
     if (!(P.fl(ip) & 1)) continue;
     int iq = P.nb(ip);
     if (iq < 0 || !(Q.fl(iq) & 1)) continue;
@@ -1980,6 +1987,7 @@ __device__ __forceinline__ unsigned warp_flow_scan(unsigned x) {   // inclusive
 // (BlockGroup) or the whole grid (GridGroup) per pair; every member executes every group
 // call (uniform control flow).  kItems: ring slots a member takes between two scans.
 struct WarpGroup {
+  __device__ __forceinline__ void beat(int) const {}
   static constexpr bool kBlock = false;
   static constexpr bool kGrid = false;
   static constexpr bool kSolo = false;
@@ -2025,6 +2033,7 @@ struct WarpGroup {
 
 // One thread per pair: every collective is the identity, nothing synchronises.
 struct SoloGroup {
+  __device__ __forceinline__ void beat(int) const {}
   static constexpr bool kGrid = false;
   static constexpr bool kSolo = true;
   static constexpr int kItems = 1;
@@ -2051,6 +2060,7 @@ constexpr int kBlockLoopTableBytes = 96 * 1024;
 constexpr int kBlockListRounds = 8;   // elements per thread between two barriers of list()
 constexpr int kBlockScratch = kBlockLabelWarps + 1 + (kBlockListRounds * kBlockLabelWarps + 2) / 2;
 struct BlockGroup {
+  __device__ __forceinline__ void beat(int) const {}
   static constexpr bool kBlock = true;
   static constexpr bool kGrid = false;
   static constexpr bool kSolo = false;
@@ -2166,13 +2176,16 @@ struct BlockGroup {
   }
 };
 
-// The whole grid on one pair (a cooperative launch: all blocks are resident).  The blocks
-// meet at a counting barrier; its wait is bounded, and once one wait has given up (an error
-// is raised) every later barrier falls through, so the kernel ends.
+// The whole grid on one pair (a cooperative launch: all blocks are resident).  The blocks meet
+// at a counting barrier.  Its wait is bounded by progress: it gives up only when, for
+// ClipParams::grid_wait polls, no block has arrived and no member that works alone (a chain, a
+// long loop, the split vertices) has called beat().  A wait that gave up ends the kernel: the
+// error is raised, and every block leaves at the barrier where it learns of it, before it uses what
+// it would have waited for.
 constexpr int kGridBlocksMax = 512;
-constexpr long long kGridWaitPolls = 1ll << 26;
 struct GridScratch {
   unsigned arrive;
+  unsigned beats;
   int dead;
   unsigned long long slot[3];                            // reductions, in turn
   unsigned long long blk[2][kGridBlocksMax];             // blocks' parts of a scan, in turn
@@ -2186,10 +2199,15 @@ struct GridGroup {
   BlockGroup blk;
   GridScratch* gs;
   int* err;
+  long long wait;
+  int* gone;                                             // shared: the block leaves
   mutable unsigned epoch = 0, reds = 0, scans = 0;
-  __device__ __forceinline__ GridGroup(const BlockGroup& b, GridScratch* g, int* e) : blk(b), gs(g), err(e) {}
+  __device__ __forceinline__ GridGroup(const BlockGroup& b, GridScratch* g, int* e, long long w, int* left)
+      : blk(b), gs(g), err(e), wait(w), gone(left) {}
   __device__ __forceinline__ int rank() const { return (int)(blockIdx.x * kBlockLabelThreads + threadIdx.x); }
   __device__ __forceinline__ int size() const { return (int)(gridDim.x * kBlockLabelThreads); }
+  // progress of a member's long loop, by its step count
+  __device__ __forceinline__ void beat(int step) const { if ((step & 1023) == 1023) atomicAdd(&gs->beats, 1u); }
   __device__ void sync() const {
     ++epoch;
     __syncthreads();
@@ -2198,13 +2216,19 @@ struct GridGroup {
       __threadfence();
       atomicAdd(&gs->arrive, 1u);
       volatile GridScratch* v = gs;
-      for (long long polls = 0; (int)(v->arrive - target) < 0; ++polls) {
-        if (v->dead) break;
-        if (polls > kGridWaitPolls) { v->dead = 1; raise_error(err, DEV_TIMEOUT); break; }
+      unsigned seen = v->arrive + v->beats;
+      for (long long polls = 0; (int)(v->arrive - target) < 0 && !v->dead;) {
+        if (++polls <= wait) continue;
+        const unsigned now = v->arrive + v->beats;
+        if (now == seen) { v->dead = 1; raise_error(err, DEV_TIMEOUT); break; }
+        seen = now;
+        polls = 0;
       }
       __threadfence();
+      *gone = v->dead;
     }
     __syncthreads();
+    if (*gone) asm volatile("exit;");
   }
   // combine one value per block: add(slot, value) by each block's first thread
   template <class A>
@@ -2390,7 +2414,7 @@ __device__ bool grp_step2(const G& g, PairCtx& c) {
   for (int s = g.rank(); s < m; s += g.size()) {
     if (!P.it(s) || (P.lb(s) != L_LEFT_ON && P.lb(s) != L_RIGHT_ON)) continue;
     int I = (s + 1 < m) ? s + 1 : 0, guard = m;
-    while (P.lb(I) == L_ON_ON && --guard > 0) I = (I + 1 < m) ? I + 1 : 0;
+    while (P.lb(I) == L_ON_ON && --guard > 0) { g.beat(guard); I = (I + 1 < m) ? I + 1 : 0; }
     if ((P.lb(I) != L_ON_LEFT && P.lb(I) != L_ON_RIGHT) || !P.it(I)) ok = false;
   }
   if (!g.all(ok)) return false;
@@ -2401,6 +2425,7 @@ __device__ bool grp_step2(const G& g, PairCtx& c) {
     int I = (s + 1 < m) ? s + 1 : 0;
     Q.lb(P.nb(s)) = L_NONE;
     while (P.lb(I) == L_ON_ON) {
+      g.beat(I);
       P.lb(I) = L_NONE;
       Q.lb(P.nb(I)) = L_NONE;
       I = (I + 1 < m) ? I + 1 : 0;
@@ -2787,12 +2812,13 @@ struct LoopsNodes {
 // did not close within guard steps).  The walk goes both ways at once and stops at the
 // first smaller segment: over a loop of L segments the searches take O(L log L) steps in
 // all, whatever its order, and the smallest segment's own takes L / 2.
-template <class T>
-__device__ __forceinline__ int loop_size(const T& tab, int t, int guard) {
+template <class T, class B = NoBeat>
+__device__ __forceinline__ int loop_size(const T& tab, int t, int guard, B beat = B()) {
   if (tab.raw(t) & kNoCrossing) return 0;
   int f = tab.link(t, 1), b = tab.link(t, 0);            // where the two walks arrive
   int sz = tab.w(t, 1);
   while ((f >> 1) != t) {
+    beat(guard >> 1);
     const int ft = f >> 1, bt = b >> 1, fo = 1 - (f & 1), bi = b & 1;
     if ((ft < t && !(tab.raw(ft) & kNoCrossing)) || (bt < t && !(tab.raw(bt) & kNoCrossing))) return 0;
     sz += tab.w(ft, fo);
@@ -2965,8 +2991,8 @@ __device__ int grp_trace_loops(const G& g, PairCtx& c) {
     for (int t = g.rank(); t < n; t += g.size())         // peel the tails from their first states on
       for (int e = 0; e < 2; ++e) {
         if (way[e][t] != -1) continue;
-        int l = link(t, 1 - e);
-        while (atomicSub(&deg[l & 1][l >> 1], 1) == 1) l = link(l >> 1, 1 - (l & 1));
+        int l = link(t, 1 - e), steps = 0;
+        while (atomicSub(&deg[l & 1][l >> 1], 1) == 1) { g.beat(++steps); l = link(l >> 1, 1 - (l & 1)); }
       }
     g.sync();
     auto way_in = [&](int s, int t, int e) { return e ? dist(end_p(t, 0), s, mP) : dist(s, end_p(t, 1), mP); };
@@ -3020,14 +3046,16 @@ __device__ int grp_trace_loops(const G& g, PairCtx& c) {
   int32_t* nodeOff = &Q.pv(0);
   const LoopsNodes nodes{&P.nx(0), &P.nx(mP >> 1), &P.pv(0), &P.pv(mP >> 1), nEvery};
   const bool bounded = G::kGrid && !odd;
+  auto beat = [&g](int step) { g.beat(step); };
   for (int t = g.rank(); t < n; t += g.size()) {
-    int sz = shared ? loop_size(shrd, t, n + 2) : loop_size(glob, t, bounded ? 2 * kNodeEvery : n + 2);
+    int sz = shared ? loop_size(shrd, t, n + 2) : loop_size(glob, t, bounded ? 2 * kNodeEvery : n + 2, beat);
     if (sz < 0 && !bounded) { bad = true; sz = 0; }
     if (odd && sz > 0) {                                 // the pieces depend on the direction: walk them
       const int in0 = start_end(t), I = end_p(t, in0);
-      int u = t, in = in0, v = I;
+      int u = t, in = in0, v = I, steps = 0;
       sz = 0;
       do {
+        beat(++steps);
         const Step r = step_of(u, in, v, -1);
         sz += r.lp + r.lq;
         v = Q.nb(r.left);
@@ -3059,6 +3087,7 @@ __device__ int grp_trace_loops(const G& g, PairCtx& c) {
         for (int e = 0; e < 2; ++e) {
           int u = t, out = e, l, to, sum = 0, left = n + 1;
           do {
+            beat(left);
             sum += glob.w(u, out);
             l = glob.link(u, out);
             u = l >> 1;
@@ -3108,8 +3137,9 @@ __device__ int grp_trace_loops(const G& g, PairCtx& c) {
   for (int k = g.rank(); k < nl; k += g.size()) {
     const int t0 = lead[k], base = off[t0], in0 = start_end(t0);
     if (odd) {
-      int u = t0, in = in0, v = end_p(t0, in0), o = base;
+      int u = t0, in = in0, v = end_p(t0, in0), o = base, steps = 0;
       do {
+        beat(++steps);
         const Step r = step_of(u, in, v, -1);
         off[u] = in ? ~o : o;
         eV[u] = v;
@@ -3133,9 +3163,10 @@ __device__ int grp_trace_loops(const G& g, PairCtx& c) {
       for (int i = g.rank(); i < nEvery + nOpen; i += g.size()) {
         int o = nodeOff[i];
         if (o == INT_MIN) continue;
-        int in = o < 0 ? 1 : 0, u = nodeT[i];
+        int in = o < 0 ? 1 : 0, u = nodeT[i], steps = 0;
         if (in) o = ~o;
         do {
+          beat(++steps);
           off[u] = in ? ~o : o;
           o += glob.w(u, 1 - in);
           const int l = glob.link(u, 1 - in);
@@ -3299,12 +3330,13 @@ __device__ bool grp_linearize(const G& g, PairCtx& c) {
 // wrong the part is gone over again from the vertex that was kept, until nothing changes
 // (lane 0's part is right from the start, so at most 32 times; parts agree after one
 // or two).  Returns how many vertices are kept; writes them to dst when it is given.
-__device__ int warp_cleanup_component(const double2* src, double2* dst, int n, double eps) {
+template <class G>
+__device__ int warp_cleanup_component(const G& g, const double2* src, double2* dst, int n, double eps) {
   const int lane = (int)lane_id();
   auto area_is_small = [eps](double2 a, double2 b, double2 c) { return fabs(area2(a.x, a.y, b.x, b.y, c.x, c.y)) < eps; };
   const double2 last = src[n - 1];
   int r = 0;
-  while (r < n && (r == n - 1 ? 0.0 < eps : area_is_small(last, src[r], src[r + 1]))) ++r;
+  while (r < n && (r == n - 1 ? 0.0 < eps : area_is_small(last, src[r], src[r + 1]))) g.beat(++r);
   if (r >= n) return 0;
   const int len = n - 1 - r, per = (len + 31) / 32;
   const int a = r + 1 + min(lane * per, len), b = r + 1 + min((lane + 1) * per, len);
@@ -3314,6 +3346,7 @@ __device__ int warp_cleanup_component(const double2* src, double2* dst, int n, d
     kept = 0;
     double2 k = src[prev];
     for (int j = a; j < b; ++j) {
+      g.beat(j);
       const double2 v = src[j], nx = j + 1 < n ? src[j + 1] : first;
       if (area_is_small(k, v, nx)) continue;
       if (out) out[kept] = v;
@@ -3346,8 +3379,9 @@ __device__ int warp_cleanup_component(const double2* src, double2* dst, int n, d
 // takes 32 components, short ones a lane each, long ones all lanes together -- and leave
 // the result in place when nothing is removed; else the kept vertices go, in order, to the
 // free part of the pair's output region behind the traced ones (*where: its offset there).
-template <class G>
-__device__ void grp_cleanup(const G& g, PairCtx& c, int32_t* outNC, int64_t* outNV, int64_t* where) {
+// sequential(): one member's clean-up, component after component.
+template <class G, class S>
+__device__ void grp_cleanup(const G& g, PairCtx& c, int32_t* outNC, int64_t* outNV, int64_t* where, S sequential) {
   OutRegion& O = c.O;
   if constexpr (G::kSolo) {
     double2* xy = reinterpret_cast<double2*>(O.xy);
@@ -3379,7 +3413,7 @@ __device__ void grp_cleanup(const G& g, PairCtx& c, int32_t* outNC, int64_t* out
     constexpr int kShortComp = 32;
     const int nc = O.nc, lane = (int)lane_id();
     if (nc == 0 || 2 * O.nv > O.vcap) {                  // (the region has room for twice a well-formed trace)
-      if (g.rank() == 0) seq_cleanup(c, outNC, outNV);
+      if (g.rank() == 0) sequential();
       g.sync();
       return;
     }
@@ -3433,7 +3467,7 @@ __device__ void grp_cleanup(const G& g, PairCtx& c, int32_t* outNC, int64_t* out
           }
           any = __any_sync(kFull, small) != 0;
         }
-        const int lk = any ? warp_cleanup_component(v, nullptr, ln, c.eps_clean) : ln;
+        const int lk = any ? warp_cleanup_component(g, v, nullptr, ln, c.eps_clean) : ln;
         if (lane == src) kept = lk;
       }
       if (k < nc) {
@@ -3472,7 +3506,7 @@ __device__ void grp_cleanup(const G& g, PairCtx& c, int32_t* outNC, int64_t* out
         const double2* v = xy + __shfl_sync(kFull, s0, src);
         double2* d = out + __shfl_sync(kFull, d0, src);
         if (lk == ln) for (int j = lane; j < ln; j += 32) d[j] = v[j];
-        else warp_cleanup_component(v, d, ln, c.eps_clean);
+        else warp_cleanup_component(g, v, d, ln, c.eps_clean);
       }
     }
     g.sync();
@@ -3502,7 +3536,7 @@ __device__ void prefetch_ring(const G& g, const Ring& R) {
   }
 }
 
-// What the sequential phases of a pair start from: 1 the links, 2 the labels, 3 the flags
+// What a grid leaves of a pair to one thread: 1 the trace and the clean-up, 2 the clean-up
 // (rings of m slots, `used` with the added vertices; components and vertices already out).
 struct BigSeq { int from, mP, mQ, usedP, usedQ, nc; int64_t nv; };
 
@@ -3557,20 +3591,15 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
     prefetch_ring(g, c.R[0]);
     prefetch_ring(g, c.R[1]);
   }
-  // where the sequential phases take over; a grid leaves them to a kernel of one thread
-  auto sequential = [&](int from) {
-    if constexpr (G::kGrid) {
-      if (lead) *a.seq = BigSeq{from, c.R[0].m, c.R[1].m, c.R[0].used, c.R[1].used, c.O.nc, c.O.nv};
-    } else {
-      if (lead) seq_pair_from<EX>(c, from, outNC, outNV);
-    }
-    g.sync();
+  // what a grid leaves to a kernel of one thread
+  auto leave = [&](int from) {
+    if (lead) *a.seq = BigSeq{from, c.R[0].m, c.R[1].m, c.R[0].used, c.R[1].used, c.O.nc, c.O.nv};
   };
   const bool oneToOne = grp_links_one_to_one(g, c.R[0], c.R[1]);
   if constexpr (G::kSolo) {
-    if (!oneToOne) { sequential(1); return; }
+    if (!oneToOne) { seq_pair_from<EX>(c, 1, outNC, outNV); return; }
     grp_step1<EX>(g, c);
-    if (!grp_step2(g, c)) { sequential(2); return; }
+    if (!grp_step2(g, c)) { seq_pair_from<EX>(c, 2, outNC, outNV); return; }
   } else {
     // Links that are not one-to-one and malformed chains leave only the chains' resolution
     // (over the listed chain starts) and, for the former, the trace to one member.
@@ -3581,7 +3610,7 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
       const int n = g.list(P.m, [&](int s) { return P.it(s) && (P.lb(s) == L_LEFT_ON || P.lb(s) == L_RIGHT_ON); },
                            [&](int s, bool hit, int before) { if (hit) P.ls(before) = s; });
       g.sync();
-      if (lead) seq_step2(c, n);
+      if (lead) seq_step2(c, n, [&g](int step) { g.beat(step); });
       g.sync();
     }
   }
@@ -3596,7 +3625,7 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
       n = g.list(P.used, [&](int s) { return (P.fl(s) & 1) != 0; }, [&](int s, bool hit, int before) { if (hit) P.ls(before) = s; });
       g.sync();
     }
-    if (lead) ok = seq_step5<EX>(c, n);
+    if (lead) ok = seq_step5<EX>(c, n, [&g](int step) { g.beat(step); });
     ok = g.bcast0((int)ok);
     c.R[0].used = g.bcast0(c.R[0].used);
     c.R[1].used = g.bcast0(c.R[1].used);
@@ -3610,7 +3639,7 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
   }
   if (added || !oneToOne) {
     // trace through the next/prev links on one member
-    if constexpr (G::kGrid) { sequential(3); return; }
+    if constexpr (G::kGrid) { leave(1); return; }
     int ok = 1;
     if (lead) ok = seq_trace(c) ? 1 : 0;
     ok = g.bcast0(ok);
@@ -3625,7 +3654,7 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
     else r = grp_trace_loops(g, c);
     if (r < 0) return;
     if (r > 0) {
-      if constexpr (G::kGrid) { sequential(3); return; }
+      if constexpr (G::kGrid) { leave(1); return; }
       else if (!grp_trace(g, c)) return;
     }
   }
@@ -3633,7 +3662,10 @@ __device__ void label_trace_pair(const G& g, const LabelArgs& a, int64_t k) {
     if (lead) fail(c, DEV_CAPACITY);
     return;
   }
-  grp_cleanup(g, c, outNC, outNV, a.outVOff + k);
+  grp_cleanup(g, c, outNC, outNV, a.outVOff + k, [&]() {
+    if constexpr (G::kGrid) leave(2);
+    else seq_cleanup(c, outNC, outNV);
+  });
 }
 
 // Two register budgets for the warp and one-thread kernels.  kWide (batches of at least
@@ -3759,7 +3791,8 @@ template <int EX>
 __global__ void __launch_bounds__(kBlockLabelThreads)
 label_trace_grid_kernel(LabelArgs a, const int64_t* __restrict__ list, int n, GridScratch* gs, BigSeq* seq) {
   __shared__ long long sm[kBlockScratch];
-  const GridGroup g(BlockGroup{sm, nullptr, 0}, gs, a.err);
+  __shared__ int gone;
+  const GridGroup g(BlockGroup{sm, nullptr, 0}, gs, a.err, a.prm.grid_wait, &gone);
   for (int i = 0; i < n; ++i) {
     a.seq = seq + i;
     label_trace_pair<EX>(g, a, list[i]);
@@ -3769,9 +3802,10 @@ label_trace_grid_kernel(LabelArgs a, const int64_t* __restrict__ list, int n, Gr
 
 // the pairs that the grid left to the sequential phases, a thread each
 template <int EX>
-__global__ void big_seq_kernel(LabelArgs a, const int64_t* __restrict__ list, const BigSeq* __restrict__ seq) {
+__global__ void big_seq_kernel(LabelArgs a, const int64_t* __restrict__ list, const BigSeq* __restrict__ seq,
+                               const GridScratch* __restrict__ gs) {
   const BigSeq q = seq[blockIdx.x];
-  if (q.from == 0) return;
+  if (q.from == 0 || gs->dead) return;                   // (a grid that gave up leaves rings half done)
   const int64_t k = list[blockIdx.x];
   PairCtx c;
   c.R[0] = ring_of(a.SP, a.regP[k], q.mP, (int)a.regSizeP[k]);
@@ -3786,8 +3820,7 @@ __global__ void big_seq_kernel(LabelArgs a, const int64_t* __restrict__ list, co
   c.err = a.err;
   c.status = a.D.status + k;
   c.noInter[0] = c.noInter[1] = c.ident[0] = c.ident[1] = false;
-  if (q.from < 3) seq_pair_from<EX>(c, q.from, a.outNC + k, a.outNV + k);
-  else if (seq_trace(c)) seq_cleanup(c, a.outNC + k, a.outNV + k);
+  if (q.from == 2 || seq_trace(c)) seq_cleanup(c, a.outNC + k, a.outNV + k);
 }
 
 // ---------------------------------------------------------------- G8 compaction
@@ -4514,7 +4547,7 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
                                       args, 0, s) != cudaSuccess)
         return ST_CUDA_ERROR;
       note_launch();
-      { (prm.exact ? big_seq_kernel<1> : big_seq_kernel<0>)<<<(unsigned)nGrid, 1, 0, s>>>(la, blist, seq); note_launch(); }
+      { (prm.exact ? big_seq_kernel<1> : big_seq_kernel<0>)<<<(unsigned)nGrid, 1, 0, s>>>(la, blist, seq, gs); note_launch(); }
     }
   }
   mk->mark("clip:label+trace", s);

@@ -256,7 +256,7 @@ class Engine:
 
     def set_tuning(self, bin_grid=None, big_label=None, mid_label=None, tile_label=None, wide_label=None,
                    f32_filter=None, fused_emit=None, record_hint=None, join_sweep=None,
-                   sweep_two_pass=None):
+                   sweep_two_pass=None, grid_wait=None):
         """Work-distribution thresholds, the join's FP32 prefilters, the one-pass record
         count + emit and its capacity hint (results depend on none of them)."""
         if f32_filter is not None:      # bit 0: MBR y prefilter, bit 1: edge prefilter
@@ -269,6 +269,8 @@ class Engine:
             _check(lib().gcmfgh_set_tuning(self.h, 8, 1 if join_sweep else 0))
         if sweep_two_pass is not None:  # the sweep's count and emit as two passes
             _check(lib().gcmfgh_set_tuning(self.h, 9, 1 if sweep_two_pass else 0))
+        if grid_wait is not None:       # polls without progress at a grid-wide barrier
+            _check(lib().gcmfgh_set_tuning(self.h, 10, int(grid_wait)))
         if bin_grid is not None:
             _check(lib().gcmfgh_set_tuning(self.h, 0, int(bin_grid)))
         if big_label is not None:

@@ -174,6 +174,10 @@ const char* gcmfgh_status_string(gcmfgh_status s);
  * sized from the last join's totals (again, at the counted sizes, when a join finds
  * more).  Candidates, flags, counts and edge lists are the same. */
 #define GCMFGH_TUNE_SWEEP_TWO_PASS 9
+/* GCMFGH_TUNE_GRID_WAIT: polls without any progress after which a barrier of the grid-wide
+ * labelling gives up; the call then ends with GCMFGH_DEVICE_ERROR (default 2^26, tens of
+ * seconds) */
+#define GCMFGH_TUNE_GRID_WAIT 10
 gcmfgh_status gcmfgh_set_tuning(gcmfgh_ctx* ctx, int key, int64_t value);
 
 /* ---- autotuner of the work-distribution thresholds.  No counterpart in the reference
