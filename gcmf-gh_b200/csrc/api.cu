@@ -219,8 +219,8 @@ ClipParams clip_params(const gcmfgh_ctx* c, const gcmfgh_layer* b, const gcmfgh_
   if (!c->tuning_explicit) {
     const TuneRecord* t = find_tuning(c, floor_log2((double)std::max<int64_t>(n, 1)), mean_verts_log2(b, o), p.exact);
     if (t) apply_tuning(p, *t);
-    else p.tile_label_max = default_tile_label(n);
   }
+  if (p.tile_label_max < 0) p.tile_label_max = default_tile_label(n);
   return p;
 }
 
@@ -548,6 +548,16 @@ gcmfgh_status gcmfgh_set_tuning(gcmfgh_ctx* c, int key, int64_t value) {
   }
   if (key == GCMFGH_TUNE_GRID_WAIT) {
     c->prm.grid_wait = value;
+    return GCMFGH_OK;
+  }
+  if (key == GCMFGH_TUNE_DEFAULTS) {
+    const ClipParams d;
+    c->prm.bin_grid = d.bin_grid;
+    c->prm.tile_label_max = d.tile_label_max;
+    c->prm.mid_label_min = d.mid_label_min;
+    c->prm.big_label_min = d.big_label_min;
+    c->prm.wide_label_min = d.wide_label_min;
+    c->tuning_explicit = false;
     return GCMFGH_OK;
   }
   c->tuning_explicit = true;

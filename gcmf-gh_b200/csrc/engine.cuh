@@ -104,7 +104,8 @@ struct ClipParams {
   int no_swap = 0;            // 1: clip base as P even when it has fewer vertices
   int exact = 0;              // 1: exact orientation/classification signs (eps unused there)
   int64_t bin_grid = 1ll << 16;        // edge-pair grid above which a pair's edges are binned
-  int64_t tile_label_max = 96;         // merged-ring slots up to which one thread labels a pair
+  int64_t tile_label_max = -1;         // merged-ring slots up to which one thread labels a pair
+                                       // (-1: default_tile_label of the clip's pairs)
   int64_t wide_label_min = 1 << 16;    // clip batches of at least this many pairs use the
                                        // high-occupancy labelling kernels
   int64_t mid_label_min = 1ll << 10;   // merged-ring slots above which a block labels a pair
@@ -115,7 +116,7 @@ struct ClipParams {
                                        // grid-wide labelling gives up (tens of seconds)
 };
 
-// The one-thread labelling's limit for a clip of n pairs when no threshold is set.  A thread
+// The one-thread labelling's limit for a clip of n pairs unless it is set or recorded.  A thread
 // takes as long as its pair's slots (0.35 ms at 96), which only a batch that fills the GPU
 // with threads hides; below that a warp per pair is faster.  Label + trace with limits 96 /
 // 32 / 0: 0.38 / 0.11 / 0.04 ms at 1,300 pairs, 0.63 / 0.44 / 0.33 at 20,000 (exact),

@@ -256,9 +256,11 @@ class Engine:
 
     def set_tuning(self, bin_grid=None, big_label=None, mid_label=None, tile_label=None, wide_label=None,
                    f32_filter=None, fused_emit=None, record_hint=None, join_sweep=None,
-                   sweep_two_pass=None, grid_wait=None):
+                   sweep_two_pass=None, grid_wait=None, defaults=False):
         """Work-distribution thresholds, the join's FP32 prefilters, the one-pass record
         count + emit and its capacity hint (results depend on none of them)."""
+        if defaults:                    # the five thresholds below as in a new engine
+            _check(lib().gcmfgh_set_tuning(self.h, 11, 0))
         if f32_filter is not None:      # bit 0: MBR y prefilter, bit 1: edge prefilter
             _check(lib().gcmfgh_set_tuning(self.h, 5, int(f32_filter)))
         if fused_emit is not None:

@@ -178,6 +178,10 @@ const char* gcmfgh_status_string(gcmfgh_status s);
  * labelling gives up; the call then ends with GCMFGH_DEVICE_ERROR (default 2^26, tens of
  * seconds) */
 #define GCMFGH_TUNE_GRID_WAIT 10
+/* GCMFGH_TUNE_DEFAULTS: the thresholds BIN_GRID, BIG_LABEL, MID_LABEL, TILE_LABEL and WIDE_LABEL are
+ * as in a new context again (value: 0).  Setting one of them leaves the others' defaults as
+ * they are, and puts all of them before recorded tunings. */
+#define GCMFGH_TUNE_DEFAULTS 11
 gcmfgh_status gcmfgh_set_tuning(gcmfgh_ctx* ctx, int key, int64_t value);
 
 /* ---- autotuner of the work-distribution thresholds.  No counterpart in the reference

@@ -38,6 +38,15 @@ def engine():
     eng.close()
 
 
+@pytest.fixture(autouse=True)
+def default_thresholds(request):
+    """Tests set and restore thresholds on the shared engine; those that a user's engine
+    chooses by the batch come back only this way."""
+    yield
+    if "engine" in request.fixturenames:
+        request.getfixturevalue("engine").set_tuning(defaults=True)
+
+
 def load_poly(path):
     """Reference .poly text: 'x y,' per vertex, ';' closes a component."""
     comps = []
