@@ -774,9 +774,15 @@ __device__ __forceinline__ bool bin_f32_rejects(float4 p, float4 q, float M) {
 // count and once to emit, took 271 ms for the 400,000 x 200,000-vertex pair (2.9e7
 // records) and 31.3 ms for the degenerate batch of 10,007 pairs (2.3e7), this 14.1 and 9.2 ms.
 // (3 blocks per SM at 80 registers: 22.4 ms against 27.2 ms for 2 at 128, cells of the mean box.)
+// kBoxes 0: there are no copies (kMaxBoxes), every listing is classified.
 constexpr int kBinEdges = 8;
 
-template <int kExact>
+// Listings up to which the FP32 copies are made: 16 bytes each beside the 4 of the listing, 8.6 GB
+// here.  A ring of n edges with about sqrt(n) of them as long as the ring has up to 2 n sqrt(n)
+// listings, which with copies would not fit the GPU from 3e6 edges on.
+constexpr int64_t kMaxBoxes = 1ll << 29;
+
+template <int kExact, int kBoxes>
 __global__ void __launch_bounds__(kThreads, 3)
 bin_append_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, int64_t np,
                   const int64_t* __restrict__ offP, const int32_t* __restrict__ LP,
@@ -877,7 +883,7 @@ bin_append_kernel(LayerDev Lb, LayerDev Lo, PairDev D, BinSet S, int64_t np,
         }
         const int64_t e = __shfl_sync(0xffffffffu, from, lo & 31) + t;
         bool keep = false;
-        if (t < total) keep = !bin_f32_rejects<kExact>(pf, __ldg(cellBox + e), G.M);
+        if (t < total) keep = !kBoxes || !bin_f32_rejects<kExact>(pf, __ldg(cellBox + e), G.M);
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (keep) wq[queued + __popc(m & lanemask_lt())] = make_int2(p, cellList[e]);
         queued += __popc(m);
@@ -4090,7 +4096,9 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     if (nBinP == 0) return;
     const FusedRecords F{recTot, recCap, nullptr, nullptr};
     auto u64 = [](int64_t* p) { return reinterpret_cast<unsigned long long*>(p); };
-    (prm.exact ? bin_append_kernel<1> : bin_append_kernel<0>)<<<blocks_for_warps((nBinP + kBinEdges - 1) / kBinEdges),
+    auto kern = cellBox ? (prm.exact ? bin_append_kernel<1, 1> : bin_append_kernel<0, 1>)
+                        : (prm.exact ? bin_append_kernel<1, 0> : bin_append_kernel<0, 0>);
+    kern<<<blocks_for_warps((nBinP + kBinEdges - 1) / kBinEdges),
                                                                kThreads, 0, st>>>(
         Lb, Lo, D, BS, nBinP, offP, LP, cellOff, cellList, cellBox, prm.eps, R, F, countPairs ? u64(binRec) : nullptr,
         u64(binQ));
@@ -4142,8 +4150,9 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     cudaMemsetAsync(cellCnt, 0, nCls * sizeof(int32_t), sb);        // the listing cursors
     if (!syncb()) return ST_CUDA_ERROR;
     cellList = A.take_n<int32_t>(hs[43]);
-    if (fused) cellBox = A.take_n<float4>(hs[43]);
-    if (!cellList || (fused && !cellBox)) return ST_OUT_OF_MEMORY;
+    const bool boxes = fused && hs[43] <= kMaxBoxes;
+    if (boxes) cellBox = A.take_n<float4>(hs[43]);
+    if (!cellList || (boxes && !cellBox)) return ST_OUT_OF_MEMORY;
     if (nBinQ > 0)
       { bin_cells_kernel<1><<<blocks_for(nBinQ), kThreads, 0, sb>>>(Lb, Lo, D, BS, nBinQ, offQ, LQ, nullptr, cellOff,
                                                                    cellCnt, cellList, cellBox); note_launch(); }

@@ -118,3 +118,34 @@ def test_sizes_beyond_fp32(engine, exponent):
     assert np.array_equal(r.count1[r.status != 2], o.count1[o.status != 2])
     assert np.array_equal(r.comp_size, o.comp_size)
     assert np.array_equal(r.xy, o.xy)
+
+
+def test_more_listings_than_copies(engine):
+    """Two rings of a million edges, some of one right across it: about 9e8 listings, beyond
+    what FP32 copies are made for.  Against the two passes, which make none (and which smaller
+    pairs are compared with the oracle for)."""
+    import gcmfgh
+    n, longs = 1_000_000, 1500
+    rng = np.random.default_rng(8)
+    a = np.linspace(0.0, 2.0 * np.pi, n, endpoint=False)
+    r = 1.0 + 1e-4 * rng.uniform(-1.0, 1.0, n)
+    r[np.arange(longs) * (n // longs)] = -1.0                   # a spike to the far side and back
+    Q = np.stack([r * np.cos(a), r * np.sin(a)], 1)
+    b = np.linspace(0.0, 2.0 * np.pi, n + 100, endpoint=False)
+    s = 1.0002 * (1.0 - 0.5 * np.exp(-((b - 1.0) / 0.3) ** 2))  # dented, else around the other
+    P = np.stack([s * np.cos(b), s * np.sin(b)], 1)
+    db, do = (gcmfgh.DeviceLayer(synth.Layer.from_rings([x])) for x in (P, Q))
+    ids = np.zeros(1, np.int32)
+    got = []
+    try:
+        engine.set_precision(True)
+        for fused in (1, 0):
+            engine.set_tuning(fused_emit=fused)
+            engine.clip_batch(db, do, ids, ids)
+            got.append(engine.clip_result())
+    finally:
+        engine.set_precision(False)
+        engine.set_tuning(fused_emit=1)
+    assert got[0].count1[0] > 100
+    for f in ("status", "count1", "comp_size", "xy"):
+        assert np.array_equal(getattr(got[0], f), getattr(got[1], f)), f
