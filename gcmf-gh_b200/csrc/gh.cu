@@ -3352,7 +3352,6 @@ __device__ int warp_cleanup_component(const G& g, const double2* src, double2* d
     kept = 0;
     double2 k = src[prev];
     for (int j = a; j < b; ++j) {
-      g.beat(j);
       const double2 v = src[j], nx = j + 1 < n ? src[j + 1] : first;
       if (area_is_small(k, v, nx)) continue;
       if (out) out[kept] = v;
@@ -3365,6 +3364,7 @@ __device__ int warp_cleanup_component(const G& g, const double2* src, double2* d
   int from = a - 1, kept = 0;                            // (a - 1 >= r)
   int end = pass(from, nullptr, kept);
   for (int round = 0; round < 32; ++round) {
+    if (lane == 0 && per > 1023) g.beat(1023);          // (once a round: a beat per vertex took 0.5 of the large pair's 48 ms)
     int before = __shfl_up_sync(kFull, end, 1);
     if (lane == 0) before = r;
     const bool wrong = before != from;
