@@ -2061,7 +2061,7 @@ struct SoloGroup {
 constexpr int kBlockLabelThreads = 512;
 constexpr int kBlockLabelWarps = kBlockLabelThreads / 32;
 // Dynamic shared memory of the block labelling kernel: the trace's loop table of pairs with
-// up to 8,192 segments of P, 12 bytes each (two blocks per SM).
+// up to 8,192 segments of P, 12 bytes each.  (At 122 to 128 registers one block fits an SM.)
 constexpr int kBlockLoopTableBytes = 96 * 1024;
 constexpr int kBlockListRounds = 8;   // elements per thread between two barriers of list()
 constexpr int kBlockScratch = kBlockLabelWarps + 1 + (kBlockListRounds * kBlockLabelWarps + 2) / 2;
@@ -2620,8 +2620,7 @@ __device__ void grp_step6(const G& g, PairCtx& c) {
 // rings' intersection flags; phase 3 copies the runs.  Returns 0 when done, 1 when the
 // flags do not alternate (the caller then runs the general walk), -1 on a capacity or trace
 // error.
-template <class G>
-__device__ int grp_trace_runs_slots(const G& g, PairCtx& c) {
+__device__ int grp_trace_runs_slots(const SoloGroup& g, PairCtx& c) {
   int nF[2];
   bool mismatch = false;     // a flagged vertex that is not a crossing, or the reverse
   for (int sd = 0; sd < 2; ++sd) {
@@ -3559,9 +3558,6 @@ struct LabelArgs {
   int32_t* outNC; int64_t* outNV;
   ClipParams prm;
   int* err;
-  int64_t tileLabelMax;       // rings up to: a tile of lanes per pair
-  int64_t midLabelMin;        // rings above: a block per pair
-  int64_t bigLabelMin;        // rings above: the grid path
   const unsigned long long* midCount;
   unsigned long long* midNext; // work-stealing cursor of the block kernel
   int blockLoopCap;           // segments the block kernel's shared loop table holds (0: none)
@@ -3691,7 +3687,7 @@ label_trace_kernel(LabelArgs a) {
   label_trace_pair<EX>(g, a, (int64_t)a.order[a.nTile + w]);
 }
 
-// Pairs whose merged rings have at most tileLabelMax slots: one thread per pair
+// Pairs whose merged rings have at most ClipParams::tile_label_max slots: one thread per pair
 // (SoloGroup, measured slightly faster than 2-lane tiles on the batched workload), the
 // pairs in size order so that the 32 pairs of a warp take about as long as each other.
 template <int EX, int kWide>
@@ -3757,7 +3753,7 @@ __global__ void label_order_kernel(const int32_t* __restrict__ mP, const int32_t
   val[k] = (uint32_t)k;
 }
 
-// Pairs with midLabelMin < slots <= bigLabelMin: persistent blocks take pairs from the
+// Pairs with mid_label_min < slots <= big_label_min: persistent blocks take pairs from the
 // list through an atomic cursor (work stealing), one block of kBlockLabelThreads per pair.
 template <int EX>
 __global__ void __launch_bounds__(kBlockLabelThreads)
@@ -4017,8 +4013,7 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   void* stC = nullptr;
   int32_t* pairRec = nullptr;
   int32_t* pairQ = nullptr;
-  if (fused) {
-  } else {
+  if (!fused) {
     chunkRec = A.take_n<int32_t>(nCh);
     chunkQ = A.take_n<int32_t>(nCh);
     recScan = A.take_n<int64_t>(nCh);
@@ -4303,11 +4298,11 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
       cudaMemsetAsync(regP, 0, sizeof(int64_t), s);
       cudaMemsetAsync(regQ, 0, sizeof(int64_t), s);
     } else {
-    radix_sort_pairs(okey, oval, okeyAlt, ovalAlt, K, 8, otmp, d_err, s);
-    { permute_sizes_kernel<<<blocks_for(K), kThreads, 0, s>>>(oval, K, regSizeP, regSizeQ, sortedP, sortedQ); note_launch(); }
-    exclusive_scan_i64(sortedP, offSP, K, tot + 11, stK, d_err, s);
-    exclusive_scan_i64(sortedQ, offSQ, K, tot + 12, stK, d_err, s);
-    { unpermute_offsets_kernel<<<blocks_for(K), kThreads, 0, s>>>(oval, K, offSP, offSQ, regP, regQ); note_launch(); }
+      radix_sort_pairs(okey, oval, okeyAlt, ovalAlt, K, 8, otmp, d_err, s);
+      { permute_sizes_kernel<<<blocks_for(K), kThreads, 0, s>>>(oval, K, regSizeP, regSizeQ, sortedP, sortedQ); note_launch(); }
+      exclusive_scan_i64(sortedP, offSP, K, tot + 11, stK, d_err, s);
+      exclusive_scan_i64(sortedQ, offSQ, K, tot + 12, stK, d_err, s);
+      { unpermute_offsets_kernel<<<blocks_for(K), kThreads, 0, s>>>(oval, K, offSP, offSQ, regP, regQ); note_launch(); }
     }
   } else {
     exclusive_scan_i64(regSizeP, regP, K, tot + 11, stK, d_err, s);
@@ -4485,7 +4480,7 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     LabelArgs la{D, K, mP, mQ, regP, regQ, regSizeP, regSizeQ, SP, SQ, oxy, vOff, vcap, ocsz, cOff, ccap, nc, nv,
-                 prm, d_err, prm.tile_label_max, midMin, prm.big_label_min, mcnt, mcnt + 1, 0, oval,
+                 prm, d_err, mcnt, mcnt + 1, 0, oval,
                  nTile, nWarp};
     // long pairs: a block each, on the auxiliary stream when there is one, so they start
     // first and overlap the warp-per-pair kernel instead of trailing it

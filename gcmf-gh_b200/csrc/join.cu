@@ -139,7 +139,8 @@ __device__ __forceinline__ void block_mbr(const LayerDev& L, int64_t w, float2* 
 }
 
 // Rings of more than kMbrLong stored vertices are taken by their whole block once its warps
-// are done with the others.  n_valid[8]: the layer's largest ring, if beyond kMbrNoteMin.
+// are done with the others (MBRs + sorts of clustered layers of 300,000 and 120,000 polygons:
+// 0.24 to 0.28 ms with 256, 0.25 to 0.28 with 1,024, 0.30 to 0.36 with 8,192).  n_valid[8]: the layer's largest ring, if beyond kMbrNoteMin.
 constexpr int kMbrLong = 1024;
 constexpr int kMbrNoteMin = 128;
 
@@ -954,6 +955,14 @@ int layer_mbrs(const LayerDev& L, double* mbr, cudaStream_t s) {
   return ST_OK;
 }
 
+// lanes per pair of the narrow-tile passes, and the pair size up to which they are used
+constexpr int kJoinTile = 4;
+constexpr int64_t kJoinTileMax = 64;
+// Edge grids beyond this: a block instead of a warp.  Refine on eight pairs of clustered layers:
+// 0.26 to 0.69 ms with 2^14, 0.25 to 0.43 with 2^12, 0.26 to 2.37 with 2^17 (a grid without a hit is
+// gone through whole).
+constexpr int64_t kJoinGridMax = 1 << 14;
+
 int run_join(const LayerDev& Lb0, const LayerDev& Lo0, Arena& A, JoinDev& J, int* d_err,
              int64_t* h_scratch, cudaStream_t s, Marks* mk, cudaStream_t aux, int f32, cudaEvent_t ovl_ready,
              int64_t cand_hint, int64_t list_hint_b, int64_t list_hint_o) {
@@ -1198,11 +1207,6 @@ int run_join(const LayerDev& Lb0, const LayerDev& Lo0, Arena& A, JoinDev& J, int
 // (b << obits | o) sorted ascending; J.mbr_b/J.mbr_o hold the layers' MBRs.  d_total
 // (4 entries) and d_cnt (8 entries, zeroed) are device scratch counters; maxB, maxO bound the
 // layers' stored vertices per polygon.
-// lanes per pair of the narrow-tile passes, and the pair size up to which they are used
-constexpr int kJoinTile = 4;
-constexpr int64_t kJoinTileMax = 64;
-constexpr int64_t kJoinGridMax = 1 << 14;     // edge grids beyond this: a block instead of a warp
-
 int join_from_keys(const LayerDev& Lb, const LayerDev& Lo, const uint64_t* pkeys, int64_t K, int obits,
                    Arena& A, JoinDev& J, int64_t* d_total, unsigned long long* d_cnt, int* d_err,
                    int64_t* h_scratch, cudaStream_t s, Marks* mk, cudaStream_t aux, int64_t hintB,
