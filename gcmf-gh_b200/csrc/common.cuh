@@ -13,6 +13,7 @@
 namespace gcmfgh {
 
 constexpr int kWarp = 32;
+constexpr int kSms = 148;   // of a B200: grids of blocks that share their work
 
 // ---- error word written by kernels (never __trap): first error wins
 enum DevError : int {

@@ -208,7 +208,7 @@ edge_filter_kernel(LayerDev Lb, LayerDev Lo, PairDev D, int64_t K, int32_t* __re
 // of a batch that has no more pairs than blocks.
 constexpr int kFilterLongThreads = 512;
 constexpr int kFilterLongRounds = 4;
-constexpr int kFilterLongBlocks = 2 * 148;
+constexpr int kFilterLongBlocks = 2 * kSms;
 
 template <int kMode>
 __global__ void __launch_bounds__(kFilterLongThreads)
@@ -4336,7 +4336,7 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
     const size_t smem = (size_t)kHeavySmem * (sizeof(uint64_t) + 2 * sizeof(uint32_t));
     cudaFuncSetAttribute(heavy_fill_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(heavy_fill_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int dev = 0, nsm = 148;
+    int dev = 0, nsm = kSms;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     unsigned long long* nHeavy = reinterpret_cast<unsigned long long*>(tot + 28);     // [heavy, mid] of P, of Q
@@ -4476,7 +4476,7 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   {
     cudaMemsetAsync(nc, 0, K * sizeof(int32_t), s);
     cudaMemsetAsync(nv, 0, K * sizeof(int64_t), s);
-    int dev = 0, nsm = 148;
+    int dev = 0, nsm = kSms;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     LabelArgs la{D, K, mP, mQ, regP, regQ, regSizeP, regSizeQ, SP, SQ, oxy, vOff, vcap, ocsz, cOff, ccap, nc, nv,
@@ -4583,7 +4583,7 @@ int run_clip(const LayerDev& Lb, const LayerDev& Lo, const int32_t* d_pid, const
   { out_compact_kernel<<<blocks_for_warps(K), kThreads, 0, s>>>(K, oxy2, vOff, ocsz, cOff, nc, nv, fVOff, C.comp_off, cxy2,
                                                               C.comp_size, pieces); note_launch(); }
   if (maxPieces > 0)
-    { out_compact_pieces_kernel<<<(unsigned)std::min<int64_t>(maxPieces, 8 * 148), kThreads, 0, s>>>(
+    { out_compact_pieces_kernel<<<(unsigned)std::min<int64_t>(maxPieces, 8 * kSms), kThreads, 0, s>>>(
           pieces, oxy2, vOff, ocsz, cOff, nc, nv, fVOff, C.comp_off, cxy2, C.comp_size); note_launch(); }
   C.vert_off = fVOff;
   mk->mark("clip:compact", s);

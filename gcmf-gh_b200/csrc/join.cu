@@ -26,7 +26,7 @@ constexpr int kWarpsPerBlock = kThreads / 32;
 
 constexpr int kLongThreads = 512;       // block-per-pair kernels (kLongRing)
 constexpr int kLongRounds = 4;
-constexpr int kLongBlocks = 2 * 148;    // two of them per SM, taking the listed pairs in turn
+constexpr int kLongBlocks = 2 * kSms;    // two of them per SM, taking the listed pairs in turn
 
 inline unsigned blocks_for_warps(int64_t warps) {
   return (unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
@@ -1024,7 +1024,7 @@ int run_join(const LayerDev& Lb0, const LayerDev& Lo0, Arena& A, JoinDev& J, int
   { mbr_kernel<<<blocks_for_warps((no + kMbrPerWarp - 1) / kMbrPerWarp), kThreads, 0, so>>>(Lo, J.mbr_o, J.valid_o, keyO, idO,
                                                                                         d_cnt + 1, xyfO); note_launch(); }
   // the overlay's extent and mean box size, for the grid of the MBR filter
-  constexpr int kExtentBlocks = 148;
+  constexpr int kExtentBlocks = kSms;
   double* part = A.take_n<double>(7 * kExtentBlocks);
   if (!part) return ST_OUT_OF_MEMORY;
   if (!forceSweep) { mbr_extent_kernel<<<kExtentBlocks, kExtentThreads, 0, so>>>(J.mbr_o, J.valid_o, no, part); note_launch(); }

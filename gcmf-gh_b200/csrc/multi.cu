@@ -873,7 +873,7 @@ int run_clip_multi_batch(int64_t n, const double* hP, const int32_t* sizesP, con
   cudaMemcpyAsync(dd, hd.data(), n * sizeof(MultiPairDesc), cudaMemcpyHostToDevice, s);
   // Pairs per warp: one while the batch leaves warps to spare (its pairs then do not wait for
   // one another's branches), up to 32 for large ones.
-  const int per = (int)std::min<int64_t>(32, std::max<int64_t>(1, n / (148 * 32)));
+  const int per = (int)std::min<int64_t>(32, std::max<int64_t>(1, n / (kSms * 32)));
   { multi_clip_batch_kernel<<<(unsigned)((n + per - 1) / per), per, 0, s>>>(a, dd, n); note_launch(); }
   exclusive_scan_i32(C.ncomp, C.comp_off, n, tot, stN, d_err, s);
   exclusive_scan_i64(nvOut, C.vert_off, n, tot + 1, stN, d_err, s);

@@ -428,7 +428,7 @@ void radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32
     unsigned* tickets = reinterpret_cast<unsigned*>(totals + kSweepMaxPasses * 256);
     unsigned long long* status = totals + kSweepMaxPasses * 256 + kSweepMaxPasses;
     cudaMemsetAsync(tmp, 0, sizeof(unsigned long long) * (kSweepMaxPasses * 257 + (size_t)passes * h), s);
-    const unsigned hb = (unsigned)(nb < 2 * 148 ? nb : 2 * 148);
+    const unsigned hb = (unsigned)(nb < 2 * kSms ? nb : 2 * kSms);
     { radix_hist_all_kernel<<<hb, kRadixThreads, 0, s>>>(keys, n, passes, totals); note_launch(); }
     for (int p = 0; p < passes; ++p) {
       { radix_sweep_kernel<<<(unsigned)nb, kRadixThreads, 0, s>>>(ka, va, kb, vb, n, 8 * p, totals + 256 * p, status + p * h,
